@@ -4,7 +4,8 @@
 
 Outputs `build/libdscuda_mla_bench.so` and
 `build/libdscuda_flash_attention_bench.so` at the repository root, the names the
-reference's harness loads (`benchmarks/common.py:19-20`).  nvcc cross-compiles,
+reference's harness loads (`benchmarks/common.py:19-20`), and
+`build/_dscuda_torch.so`, the extension `dscuda_b200.mla` calls them through.  nvcc cross-compiles,
 so no GPU is needed to build.
 """
 
@@ -18,8 +19,8 @@ import sys
 
 ROOT = pathlib.Path(__file__).resolve().parents[1]
 BUILD = ROOT / "build"
-# the two product libraries, then the test-only probe library (tests/csrc)
-LIBRARIES = ("libdscuda_mla_bench.so", "libdscuda_flash_attention_bench.so", "libdscuda_test_probes.so")
+# the two product libraries, the Python extension over them, then the test-only probe library (tests/csrc)
+LIBRARIES = ("libdscuda_mla_bench.so", "libdscuda_flash_attention_bench.so", "_dscuda_torch.so", "libdscuda_test_probes.so")
 
 
 def _tool(name: str) -> str:
@@ -38,7 +39,8 @@ def build(verbose: bool = False) -> list[pathlib.Path]:
     work = BUILD / "cmake"
     work.mkdir(parents=True, exist_ok=True)
     cmake = _tool("cmake")
-    configure = [cmake, "-S", str(ROOT), "-B", str(work), "-DCMAKE_BUILD_TYPE=Release", f"-DCMAKE_CUDA_COMPILER={nvcc}"]
+    configure = [cmake, "-S", str(ROOT), "-B", str(work), "-DCMAKE_BUILD_TYPE=Release", f"-DCMAKE_CUDA_COMPILER={nvcc}",
+                 f"-DDSCUDA_PYTHON={sys.executable}"]
     if shutil.which("ninja") or (pathlib.Path(sys.executable).parent / "ninja").exists():
         configure += ["-G", "Ninja", f"-DCMAKE_MAKE_PROGRAM={_tool('ninja')}"]
     sink = None if verbose else subprocess.PIPE

@@ -9,6 +9,8 @@ from __future__ import annotations
 
 import ctypes
 import functools
+import importlib.machinery
+import importlib.util
 import os
 import pathlib
 
@@ -46,23 +48,43 @@ FLASH_SYMBOLS = {
 }
 
 
-def library_path(name: str) -> pathlib.Path:
+def build_directory() -> pathlib.Path:
     """`build/` at the repository root, or the directory named by DSCUDA_BUILD_DIR."""
-    directory = pathlib.Path(os.environ["DSCUDA_BUILD_DIR"]) if os.environ.get("DSCUDA_BUILD_DIR") else ROOT / "build"
-    return directory / f"libdscuda_{name}_bench.so"
+    return pathlib.Path(os.environ["DSCUDA_BUILD_DIR"]) if os.environ.get("DSCUDA_BUILD_DIR") else ROOT / "build"
+
+
+def library_path(name: str) -> pathlib.Path:
+    return build_directory() / f"libdscuda_{name}_bench.so"
+
+
+def _built(path: pathlib.Path) -> pathlib.Path:
+    if not path.exists():
+        raise RuntimeError(f"{path} is missing: run `python -m dscuda_b200.build` (there is no fallback path)")
+    return path
 
 
 @functools.lru_cache(maxsize=None)
 def library(name: str) -> ctypes.CDLL:
     """Load `build/libdscuda_<name>_bench.so` and set every prototype."""
-    path = library_path(name)
-    if not path.exists():
-        raise RuntimeError(f"{path} is missing: run `python -m dscuda_b200.build` (there is no fallback path)")
-    lib = ctypes.CDLL(str(path))
+    lib = ctypes.CDLL(str(_built(library_path(name))))
     for symbol, (arguments, result) in (MLA_SYMBOLS if name == "mla" else FLASH_SYMBOLS).items():
         function = getattr(lib, symbol)
         function.argtypes, function.restype = arguments, result
     return lib
+
+
+@functools.lru_cache(maxsize=None)
+def extension():
+    """The Python extension over both libraries (`csrc/bindings/torch_bridge.cpp`): torch tensors in, C-ABI calls out."""
+    import torch  # noqa: F401 (its shared libraries must be loaded first)
+
+    library("mla"), library("flash_attention")
+    name = "_dscuda_torch"
+    path = str(_built(build_directory() / f"{name}.so"))
+    loader = importlib.machinery.ExtensionFileLoader(name, path)
+    module = importlib.util.module_from_spec(importlib.util.spec_from_file_location(name, path, loader=loader))
+    loader.exec_module(module)
+    return module
 
 
 def checked(lib: ctypes.CDLL, prefix: str, status: int) -> None:
