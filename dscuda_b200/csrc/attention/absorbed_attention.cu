@@ -38,7 +38,8 @@
 // leader, warps 5 and 6 load with TMA (5: Q, the tiles' own keys and L2 prefetches; 6: the two small loads
 // on the critical path, rotary chunk and refill).  The grid is persistent: one cluster per SM pair, the 128-key tiles
 // of all sequences laid end to end and cut into equal ranges; a sequence cut by a range boundary
-// yields one normalised partial per range, merged by decode_combine_kernel.  Every wait is bounded.
+// yields one normalised partial per range, merged by decode_combine_kernel; a sequence inside one range is
+// written out as it is.  Every wait is bounded.
 #include "mla.h"
 #include "cuda_common.h"
 #include "attention_internal.h"
@@ -84,7 +85,7 @@ static_assert(SMEM_BYTES <= 232448, "decode shared memory");
 __device__ int decode_status = 0;
 
 // Scratch for mla_decode_forward_static_cuda: room for STATIC_DECODE_RECORDS split partials of
-// (log-sum-exp, 1, 512 outputs).  It lives in the image of the library, so every GPU that loads the
+// 512 outputs and their header.  It lives in the image of the library, so every GPU that loads the
 // library keeps these 16.1 MiB until the process ends.  The name below is only a host-side handle
 // in host code; the device address is looked up once per device with cudaGetSymbolAddress.
 constexpr std::size_t STATIC_DECODE_RECORDS = 8192;
@@ -98,13 +99,15 @@ struct DecodeParams {
     // causal forward only: the queries as two tensors, the outputs, the sequence length
     CUtensorMap q_lat;      // [B*T*H rows][8 chunks][64], box of 8 chunks x 64 rows
     CUtensorMap q_rope;     // [B*T*H rows, 64], box 64 x 64
+    CUtensorMap out_map;    // the outputs as [B][rows of an entry][512] bf16, stored 64 columns x 32 rows at a time
+    CUtensorMap part_map;   // decode: the split partials as [B][H][splits][512] fp32, stored 32 columns x 32 rows of one slot at a time
     __nv_bfloat16* out;     // [B,T,H,512]
     float* lse;             // [B,H,T]
     int sequence;           // T
     const __nv_bfloat16* cache;     // [cache rows, 576]
     const int* block_table; // [B, pages]
     const int* lengths;     // [B]
-    float* workspace;       // [B,H,splits,2+512]
+    float2* headers;        // [B,H,splits] behind the partials: (log-sum-exp of the partial, state), see PARTIAL_*
     int batch;
     int heads;
     int page_size;
@@ -114,6 +117,12 @@ struct DecodeParams {
     float scale;
     float scale_log2;
 };
+
+// States of a split partial.  The partials of a (sequence, head) fill its slots from 0 on; the slot after the last one says END.
+// A unit that one cluster computed as a whole has no partials: its output is final and slot 0 says so.
+constexpr float PARTIAL_USED = 1.0F;
+constexpr float PARTIAL_END = 0.0F;
+constexpr float PARTIAL_FINAL = -1.0F;
 
 struct Schedule {
     int chunk;          // 128-key tiles per cluster
@@ -327,6 +336,62 @@ __device__ __forceinline__ bool next_segment(const DecodeParams& p, const Schedu
     return false;
 }
 
+__device__ __forceinline__ int decode_tiles(const DecodeParams& p, int b) {
+    return (sequence_length<false>(p, b) + TILE_KEYS - 1) / TILE_KEYS;
+}
+
+// The cut of the list of tiles and where this cluster's range starts (splits > 1), by one warp.  A lane takes every 32nd
+// sequence, so the lengths are loaded 32 at a time: one thread walking the list paid an L2 round trip per sequence (6-8 us
+// of every decode call at 74 sequences).
+__device__ __forceinline__ Schedule cut_schedule(const DecodeParams& p, int cluster, int clusters, int lane) {
+    const int head_tiles = (p.heads + PAIR_HEADS - 1) / PAIR_HEADS;
+    long long total = 0;
+    int longest = 0;
+    for (int b = lane; b < p.batch; b += 32) {
+        const int tiles = decode_tiles(p, b);
+        total += tiles;
+        longest = max(longest, tiles);
+    }
+#pragma unroll
+    for (int offset = 16; offset > 0; offset >>= 1) {
+        total += __shfl_xor_sync(0xffffffffU, total, offset);
+        longest = max(longest, __shfl_xor_sync(0xffffffffU, longest, offset));
+    }
+    total *= head_tiles;
+    long long chunk = (total + clusters - 1) / clusters;
+    chunk = max(chunk, static_cast<long long>((longest + p.splits - 2) / (p.splits - 1)));
+    chunk = max(chunk, 1LL);
+    Schedule schedule;
+    schedule.chunk = static_cast<int>(min(chunk, 0x7fffffffLL));
+    schedule.total = static_cast<int>(min(total, 0x7fffffffLL));
+    schedule.first_unit = p.batch * head_tiles;
+    schedule.first_offset = schedule.total;
+    // first unit that reaches past the start of the range
+    const long long lo = static_cast<long long>(cluster) * schedule.chunk;
+    long long start = 0;                        // global tile index of sequence `base`
+    for (int base = 0; base < p.batch; base += 32) {
+        const int tiles = base + lane < p.batch ? decode_tiles(p, base + lane) : 0;
+        long long end = static_cast<long long>(tiles) * head_tiles;
+#pragma unroll
+        for (int offset = 1; offset < 32; offset <<= 1) {
+            const long long before = __shfl_up_sync(0xffffffffU, end, offset);
+            end += lane >= offset ? before : 0;
+        }
+        const unsigned past = __ballot_sync(0xffffffffU, start + end > lo);
+        if (past != 0U) {
+            const int which = __ffs(static_cast<int>(past)) - 1;
+            const int tiles_there = __shfl_sync(0xffffffffU, tiles, which);
+            const long long begin = start + __shfl_sync(0xffffffffU, end, which) - static_cast<long long>(tiles_there) * head_tiles;
+            const int head_tile = static_cast<int>((lo - begin) / tiles_there);
+            schedule.first_unit = (base + which) * head_tiles + head_tile;
+            schedule.first_offset = static_cast<int>(begin + static_cast<long long>(head_tile) * tiles_there);
+            break;
+        }
+        start += __shfl_sync(0xffffffffU, end, 31);
+    }
+    return schedule;
+}
+
 template <bool CAUSAL>
 __device__ __forceinline__ void absorbed_pair_body(const DecodeParams& p) {
     extern __shared__ uint8_t smem_raw[];
@@ -357,7 +422,7 @@ __device__ __forceinline__ void absorbed_pair_body(const DecodeParams& p) {
         return;
     }
 
-    if (threadIdx.x == 0) {
+    if (warp == REFILL_WARP && lane == 0) {
         mbar_init(smem_u32(&sh->q_full), 1);
         mbar_init(smem_u32(&sh->full_r), 1);
         mbar_init(smem_u32(&sh->peer_q_full), 1);
@@ -380,38 +445,12 @@ __device__ __forceinline__ void absorbed_pair_body(const DecodeParams& p) {
         mbar_init(smem_u32(&sh->sum_ready), 4);
         sh->abort_flag = 0;
         mbar_init_fence();
-        // ---- schedule of this cluster (splits > 1) ----------------------------------
-        Schedule schedule = {1, 0, 0, 0};
-        if (!CAUSAL && p.splits > 1) {
-            const int head_tiles = (p.heads + PAIR_HEADS - 1) / PAIR_HEADS;
-            long long total = 0;
-            int longest = 0;
-            for (int b = 0; b < p.batch; ++b) {
-                const int tiles = (sequence_length<false>(p, b) + TILE_KEYS - 1) / TILE_KEYS;
-                total += static_cast<long long>(tiles) * head_tiles;
-                longest = max(longest, tiles);
-            }
-            long long chunk = (total + clusters - 1) / clusters;
-            chunk = max(chunk, static_cast<long long>((longest + p.splits - 2) / (p.splits - 1)));
-            chunk = max(chunk, 1LL);
-            schedule.chunk = static_cast<int>(min(chunk, 0x7fffffffLL));
-            schedule.total = static_cast<int>(min(total, 0x7fffffffLL));
-            const long long lo = static_cast<long long>(cluster) * schedule.chunk;
-            int unit = 0;
-            long long offset = 0;
-            const int units = p.batch * head_tiles;
-            while (unit < units) {
-                const int tiles = unit_tiles<false>(p, unit, head_tiles);
-                if (offset + tiles > lo) {
-                    break;
-                }
-                offset += tiles;
-                ++unit;
-            }
-            schedule.first_unit = unit;
-            schedule.first_offset = static_cast<int>(offset);
+    }
+    if (warp == 0) {
+        const Schedule schedule = CAUSAL || p.splits == 1 ? Schedule{1, 0, 0, 0} : cut_schedule(p, cluster, clusters, lane);
+        if (lane == 0) {
+            sh->schedule = schedule;
         }
-        sh->schedule = schedule;
     }
     if (warp == MMA_WARP) {
         tmem_alloc_pair(smem_u32(&sh->tmem_base), TMEM_COLUMNS);        // the same warp of both CTAs, together
@@ -775,6 +814,27 @@ __device__ __forceinline__ void absorbed_pair_body(const DecodeParams& p) {
         const uint32_t p_full_bar = rank == 0 ? smem_u32(&sh->p_full) : map_to_cta(smem_u32(&sh->p_full), 0);
         bool alive = true;
 
+        // A sequence without cached tokens belongs to no cluster's range: its output is NaN and its LSE -inf, what the softmax
+        // of an empty row gives in the reference (reference/python/mla.py:36-38).
+        if (!CAUSAL) {
+            for (int b = cluster; b < p.batch; b += clusters) {
+                if (p.lengths[b] > 0) {
+                    continue;
+                }
+                const uint32_t nan2 = 0x7fc07fc0U;
+                uint4* rows = reinterpret_cast<uint4*>(p.out + static_cast<size_t>(b) * p.heads * RANK);
+                for (int i = static_cast<int>(rank) * 128 + r; i < p.heads * (RANK / 8); i += 256) {
+                    rows[i] = make_uint4(nan2, nan2, nan2, nan2);
+                }
+                for (int head = static_cast<int>(rank) * 128 + r; head < p.heads; head += 256) {
+                    p.lse[static_cast<size_t>(b) * p.heads + head] = -INFINITY;
+                    if (p.splits > 1) {
+                        p.headers[(static_cast<size_t>(b) * p.heads + head) * p.splits] = make_float2(-INFINITY, PARTIAL_FINAL);
+                    }
+                }
+            }
+        }
+
         while (alive && next_segment<CAUSAL>(p, schedule, walker, seg, cluster, clusters)) {
             const int tile_count = seg.tile_end - seg.tile_begin;
             // decode: row = head of the sequence's one query token.  Causal forward: row = (token, head) pair of the batch entry.
@@ -941,62 +1001,113 @@ __device__ __forceinline__ void absorbed_pair_body(const DecodeParams& p) {
             }
             const float l_total = l_sum + sh->sums[r ^ 64];
             const float inverse = 1.0F / l_total;
-            if (CAUSAL) {
-                // the finished rows: bf16 output [B,T,H,512] and the natural-log LSE [B,H,T]
-                __nv_bfloat16* out_row = p.out + ((static_cast<size_t>(seg.b) * p.sequence + (valid ? token : 0)) * p.heads + head) * RANK;
-                if (valid && key_half == 0) {
-                    p.lse[(static_cast<size_t>(seg.b) * p.heads + head) * p.sequence + token] = m_ref * p.scale + logf(l_total);
+            const float row_lse = m_ref * p.scale + logf(l_total);
+            // A segment that is a whole unit gives the finished rows (bf16), any other a normalised fp32 partial that
+            // decode_combine_kernel weights by exp(lse - max lse).
+            const bool final_rows = CAUSAL || (seg.tile_begin == 0 && seg.last_of_unit);
+            if (valid && key_half == 0) {
+                const size_t lse_index = CAUSAL ? (static_cast<size_t>(seg.b) * p.heads + head) * p.sequence + token : static_cast<size_t>(seg.b) * p.heads + head;
+                if (final_rows) {
+                    p.lse[lse_index] = row_lse;
                 }
-#pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    uint32_t o[32];
-                    tmem_ld_x32(tmem_base + lane_base + TMEM_O + c * 32, o);
-                    tmem_wait_ld();
-                    if (valid) {
-                        uint4* dst = reinterpret_cast<uint4*>(out_row + (c >> 2) * 256 + key_half * 128 + (c & 3) * 32);
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            dst[e] = make_uint4(pack_bf16x2(__uint_as_float(o[8 * e]) * inverse, __uint_as_float(o[8 * e + 1]) * inverse),
-                                                pack_bf16x2(__uint_as_float(o[8 * e + 2]) * inverse, __uint_as_float(o[8 * e + 3]) * inverse),
-                                                pack_bf16x2(__uint_as_float(o[8 * e + 4]) * inverse, __uint_as_float(o[8 * e + 5]) * inverse),
-                                                pack_bf16x2(__uint_as_float(o[8 * e + 6]) * inverse, __uint_as_float(o[8 * e + 7]) * inverse));
-                        }
-                    }
-                }
-            } else {
-                float* records = p.workspace + (static_cast<size_t>(seg.b) * p.heads + (valid ? head : 0)) * p.splits * (RANK + 2);
-                float* record = records + static_cast<size_t>(seg.slot) * (RANK + 2);
-                // A record is (log-sum-exp of the partial, 1, normalised output): decode_combine_kernel weights the
-                // partials of a (sequence, head) by exp(lse - max lse).
-                if (valid && key_half == 0) {
-                    record[0] = m_ref * p.scale + logf(l_total);
-                    record[1] = 1.0F;
-                    if (seg.last_of_unit && seg.slot + 1 < p.splits) {
-                        // a sequence fills slots 0..slot in order; the first unused one ends the list (its row sum is 0)
-                        records[static_cast<size_t>(seg.slot + 1) * (RANK + 2)] = -INFINITY;
-                        records[static_cast<size_t>(seg.slot + 1) * (RANK + 2) + 1] = 0.0F;
-                    }
-                }
-#pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    uint32_t o[32];
-                    tmem_ld_x32(tmem_base + lane_base + TMEM_O + c * 32, o);
-                    tmem_wait_ld();
-                    if (valid) {
-                        // accumulator a = c / 4, lanes 64.. hold its columns 128..255
-                        float2* dst = reinterpret_cast<float2*>(record + 2 + (c >> 2) * 256 + key_half * 128 + (c & 3) * 32);
-#pragma unroll
-                        for (int e = 0; e < 32; e += 2) {
-                            dst[e / 2] = make_float2(__uint_as_float(o[e]) * inverse, __uint_as_float(o[e + 1]) * inverse);
-                        }
+                if (!CAUSAL && p.splits > 1) {
+                    float2* headers = p.headers + lse_index * p.splits;
+                    headers[seg.slot] = make_float2(row_lse, final_rows ? PARTIAL_FINAL : PARTIAL_USED);
+                    if (!final_rows && seg.last_of_unit && seg.slot + 1 < p.splits) {
+                        headers[seg.slot + 1] = make_float2(-INFINITY, PARTIAL_END);
                     }
                 }
             }
+            // Each warp moves its 32 rows x 256 columns through 4 KB slabs (32 rows x 128 bytes, swizzled) that TMA stores
+            // write out as whole lines.  Storing a thread's own row straight from registers touched 32 lines per
+            // instruction, 8 of 32 bytes each: 11 us for the 64 rows of a CTA.  Slab 0 is the warp's own part of P (read by no
+            // MMA any more); behind the last segment Q is idle too and gives four more, so that nothing waits for a slab.
+            Walker ahead = walker;
+            Segment after;
+            const bool more = next_segment<CAUSAL>(p, schedule, ahead, after, cluster, clusters);
+            const int slabs = more ? 1 : 5;
+            int slab_count = 0;
+            const int store_row = seg.row_tile * PAIR_HEADS + static_cast<int>(rank) * CTA_HEADS + (warp & 1) * 32;
+            const bool any_row = store_row < (CAUSAL ? p.sequence * p.heads : p.heads);
+            auto slab_offset = [&](int index) { return index == 0 ? Q_BYTES + warp * 4096 : (warp * 4 + index - 1) * 4096; };
+            auto acquire_slab = [&]() -> uint32_t {
+                if (slab_count == slabs) {
+                    if (lane == 0) {
+                        tma_store_wait_read();
+                    }
+                    __syncwarp();
+                    slab_count = 0;
+                }
+                return static_cast<uint32_t>(slab_offset(slab_count++));
+            };
+            auto store_slab = [&](uint32_t offset, int column) {
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0 && any_row) {
+                    if (final_rows) {
+                        tma_store_3d(&p.out_map, smem_base + offset, column, store_row, seg.b);
+                    } else {
+                        tma_store_4d(&p.part_map, smem_base + offset, column, seg.slot, store_row, seg.b);
+                    }
+                    tma_store_commit();
+                }
+            };
+            uint32_t o[2][32];
+            tmem_ld_x32(tmem_base + lane_base + TMEM_O, o[0]);
+            uint32_t offset = 0;
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                // accumulator a = c / 4, lanes 64.. hold its columns 128..255
+                const int column = (c >> 2) * 256 + key_half * 128 + (c & 3) * 32;
+                tmem_wait_ld();
+                if (c + 1 < 8) {
+                    tmem_ld_x32(tmem_base + lane_base + TMEM_O + (c + 1) * 32, o[(c + 1) & 1]);
+                }
+                const uint32_t* values = o[c & 1];
+                if (final_rows) {
+                    if ((c & 1) == 0) {
+                        offset = acquire_slab();
+                    }
+                    uint8_t* row_ptr = smem_raw + offset + lane * 128;
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const uint32_t* x = values + 8 * u;
+                        *reinterpret_cast<uint4*>(row_ptr + ((((c & 1) * 4 + u) ^ (lane & 7)) * 16)) =
+                            make_uint4(pack_bf16x2(__uint_as_float(x[0]) * inverse, __uint_as_float(x[1]) * inverse),
+                                       pack_bf16x2(__uint_as_float(x[2]) * inverse, __uint_as_float(x[3]) * inverse),
+                                       pack_bf16x2(__uint_as_float(x[4]) * inverse, __uint_as_float(x[5]) * inverse),
+                                       pack_bf16x2(__uint_as_float(x[6]) * inverse, __uint_as_float(x[7]) * inverse));
+                    }
+                    if ((c & 1) == 1) {
+                        store_slab(offset, column - 32);
+                    }
+                } else {
+                    offset = acquire_slab();
+                    uint8_t* row_ptr = smem_raw + offset + lane * 128;
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) {
+                        float4 x;
+                        x.x = __uint_as_float(values[4 * u]) * inverse;
+                        x.y = __uint_as_float(values[4 * u + 1]) * inverse;
+                        x.z = __uint_as_float(values[4 * u + 2]) * inverse;
+                        x.w = __uint_as_float(values[4 * u + 3]) * inverse;
+                        *reinterpret_cast<float4*>(row_ptr + ((u ^ (lane & 7)) * 16)) = x;
+                    }
+                    store_slab(offset, column);
+                }
+            }
+            if (lane == 0) {
+                tma_store_wait_read();          // the slabs are P and Q of the next segment
+            }
+            __syncwarp();
             // O may be overwritten by the next segment only after every lane has been read out: the next
             // segment's first P V waits for the P arrivals of every softmax thread, which come after this point.
             tc_fence_before_sync();
             tile_index += tile_count;
             segment_index += 1;
+        }
+        if (lane == 0) {
+            tma_store_wait_all();       // the last stores have been written before the CTA exits
         }
     }
 
@@ -1025,53 +1136,73 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) absorbed
     absorbed_pair_body<true>(p);
 }
 
-// Merges the split partials of one (sequence, head).  A record is (log-sum-exp of the
-// partial, 1, normalised output); the partials are weighted by exp(lse_s - max lse).
-// Writes bf16 output and the natural-log LSE.  A sequence without cached tokens has no
-// partial at all: its output is NaN and its LSE -inf, what the softmax of an empty row
-// gives in the reference (reference/python/mla.py:36-38).
-__global__ void __launch_bounds__(128) decode_combine_kernel(__nv_bfloat16* output, float* logsumexp, const float* workspace,
-                                                             const int* lengths, int heads, int splits) {
-    const int row = blockIdx.y * heads + blockIdx.x;
-    if (lengths[blockIdx.y] <= 0) {
-        const uint32_t nan2 = 0x7fc07fc0U;
-        *reinterpret_cast<uint2*>(output + static_cast<size_t>(row) * RANK + threadIdx.x * 4) = make_uint2(nan2, nan2);
-        if (threadIdx.x == 0) {
-            logsumexp[row] = -INFINITY;
-        }
+// Merges the split partials of each (sequence, head) and writes the bf16 output and the natural-log LSE; rows whose
+// slot 0 says FINAL are done.  One warp per row, a lane owns 16 columns (four 16-byte units): the headers of 32 slots are
+// read at once, then the partials two at a time, so a row costs two or three memory latencies instead of two per slot
+// (7-14 us before, 128 threads per row walking the slots one after the other).
+constexpr int COMBINE_THREADS = 128;
+
+__global__ void __launch_bounds__(COMBINE_THREADS) decode_combine_kernel(__nv_bfloat16* output, float* logsumexp, const float* partials,
+                                                                         const float2* headers, int rows, int splits) {
+    const int lane = threadIdx.x % 32;
+    const int row = blockIdx.x * (COMBINE_THREADS / 32) + threadIdx.x / 32;
+    if (row >= rows) {
         return;
     }
-    const float* records = workspace + static_cast<size_t>(row) * splits * (RANK + 2);
-    // Slots are filled in order from 0; the first one with a zero row sum ends the list.
+    const float2* header = headers + static_cast<size_t>(row) * splits;
+    const float4* records = reinterpret_cast<const float4*>(partials) + static_cast<size_t>(row) * splits * (RANK / 4) + lane;
+    // running maximum over groups of 32 slots; nearly always there is one group
     float maximum = -INFINITY;
-    int used = 0;
-    for (; used < splits; ++used) {
-        const float l = records[static_cast<size_t>(used) * (RANK + 2) + 1];
-        if (!(l > 0.0F)) {
-            break;
-        }
-        maximum = fmaxf(maximum, records[static_cast<size_t>(used) * (RANK + 2)]);
-    }
     float normalizer = 0.0F;
-    float acc[4] = {0.0F, 0.0F, 0.0F, 0.0F};
-    const int column = threadIdx.x * 4;
-    for (int s = 0; s < used; ++s) {
-        const float* record = records + static_cast<size_t>(s) * (RANK + 2);
-        const float weight = __expf(record[0] - maximum);
-        normalizer += weight * record[1];
-        const float2 lo = *reinterpret_cast<const float2*>(record + 2 + column);
-        const float2 hi = *reinterpret_cast<const float2*>(record + 4 + column);
-        acc[0] += weight * lo.x;
-        acc[1] += weight * lo.y;
-        acc[2] += weight * hi.x;
-        acc[3] += weight * hi.y;
+    float4 acc[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        acc[u] = make_float4(0.0F, 0.0F, 0.0F, 0.0F);
+    }
+    bool listed = true;
+    for (int base = 0; base < splits && listed; base += 32) {
+        const float2 mine = base + lane < splits ? header[base + lane] : make_float2(-INFINITY, PARTIAL_END);
+        const unsigned ends = __ballot_sync(0xffffffffU, !(mine.y > 0.0F));
+        if (base == 0 && __shfl_sync(0xffffffffU, mine.y, 0) < 0.0F) {
+            return;                             // PARTIAL_FINAL
+        }
+        const int used = ends == 0U ? 32 : __ffs(static_cast<int>(ends)) - 1;
+        listed = ends == 0U;
+        float group_max = lane < used ? mine.x : -INFINITY;
+#pragma unroll
+        for (int offset = 16; offset > 0; offset >>= 1) {
+            group_max = fmaxf(group_max, __shfl_xor_sync(0xffffffffU, group_max, offset));
+        }
+        const float new_max = fmaxf(maximum, group_max);
+        const float rescale = maximum > -INFINITY ? __expf(maximum - new_max) : 0.0F;
+        maximum = new_max;
+        normalizer *= rescale;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            acc[u] = make_float4(acc[u].x * rescale, acc[u].y * rescale, acc[u].z * rescale, acc[u].w * rescale);
+        }
+        const float my_weight = lane < used ? __expf(mine.x - maximum) : 0.0F;
+#pragma unroll 2
+        for (int s = 0; s < used; ++s) {
+            const float weight = __shfl_sync(0xffffffffU, my_weight, s);
+            normalizer += weight;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const float4 x = __ldcs(records + static_cast<size_t>(base + s) * (RANK / 4) + u * 32);
+                acc[u].x += weight * x.x;
+                acc[u].y += weight * x.y;
+                acc[u].z += weight * x.z;
+                acc[u].w += weight * x.w;
+            }
+        }
     }
     const float inverse = 1.0F / normalizer;
-    uint2 packed;
-    packed.x = pack_bf16x2(acc[0] * inverse, acc[1] * inverse);
-    packed.y = pack_bf16x2(acc[2] * inverse, acc[3] * inverse);
-    *reinterpret_cast<uint2*>(output + static_cast<size_t>(row) * RANK + column) = packed;
-    if (threadIdx.x == 0) {
+    uint2* out = reinterpret_cast<uint2*>(output + static_cast<size_t>(row) * RANK) + lane;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        out[u * 32] = make_uint2(pack_bf16x2(acc[u].x * inverse, acc[u].y * inverse), pack_bf16x2(acc[u].z * inverse, acc[u].w * inverse));
+    }
+    if (lane == 0) {
         logsumexp[row] = maximum + logf(normalizer);
     }
 }
@@ -1152,7 +1283,13 @@ void launch_decode(__nv_bfloat16* output, float* logsumexp, const __nv_bfloat16*
     params.cache = paged_kv_cache;
     params.block_table = block_table;
     params.lengths = cache_lengths;
-    params.workspace = workspace;
+    // partials first (16-byte aligned records of 512 floats), then their headers: B*H*splits*(512 + 2) floats in all
+    const std::size_t records = static_cast<std::size_t>(batch_size) * heads * splits;
+    params.headers = reinterpret_cast<float2*>(workspace + records * RANK);
+    params.out_map = make_bf16_batched_rows_map(output, batch_size, heads, RANK, 32);
+    params.part_map = make_f32_records_map(workspace, batch_size, heads, splits, RANK, 32);
+    params.out = output;
+    params.lse = logsumexp;
     params.batch = batch_size;
     params.heads = heads;
     params.page_size = page_size;
@@ -1166,8 +1303,11 @@ void launch_decode(__nv_bfloat16* output, float* logsumexp, const __nv_bfloat16*
     const int clusters = std::max(1, multiprocessor_count() / 2);
     absorbed_decode_kernel<<<dim3(2 * clusters, 1, 1), THREADS, SMEM_BYTES, stream>>>(params);
     CUDA_CHECK(cudaGetLastError());
-    decode_combine_kernel<<<dim3(heads, batch_size), 128, 0, stream>>>(output, logsumexp, workspace, cache_lengths, heads, splits);
-    CUDA_CHECK(cudaGetLastError());
+if (splits > 1) {
+        decode_combine_kernel<<<(batch_size * heads + COMBINE_THREADS / 32 - 1) / (COMBINE_THREADS / 32), COMBINE_THREADS, 0, stream>>>(
+            output, logsumexp, workspace, params.headers, batch_size * heads, splits);
+        CUDA_CHECK(cudaGetLastError());
+    }
 }
 
 }  // namespace
@@ -1224,6 +1364,8 @@ void mla_compressed_attention_forward_cuda(__nv_bfloat16* output, float* logsume
     params.k_lat8 = make_bf16_chunked_map(kv_latent, k_rows, LATENT_CHUNKS, RANK, HALF_KEYS, LATENT_CHUNKS);
     params.k_lat2 = make_bf16_chunked_map(kv_latent, k_rows, LATENT_CHUNKS, RANK, HALF_KEYS, 2);
     params.k_rope = make_bf16_tile_map(key_rope, k_rows, ROPE, ROPE, HALF_KEYS);
+    params.out_map = make_bf16_batched_rows_map(output, batch_size, static_cast<std::uint64_t>(sequence_length) * heads, RANK, 32);
+    params.part_map = params.out_map;
     params.out = output;
     params.lse = logsumexp;
     params.sequence = sequence_length;

@@ -174,6 +174,17 @@ __device__ __forceinline__ void tma_store_2d(const void* tensor_map, uint32_t sm
     asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(tensor_map), "r"(smem_src), "r"(x), "r"(y) : "memory");
 }
 
+__device__ __forceinline__ void tma_store_3d(const void* tensor_map, uint32_t smem_src, int x, int y, int z) {
+    asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(tensor_map), "r"(smem_src), "r"(x), "r"(y), "r"(z)
+                 : "memory");
+}
+
+__device__ __forceinline__ void tma_store_4d(const void* tensor_map, uint32_t smem_src, int x, int y, int z, int w) {
+    asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];" ::"l"(tensor_map), "r"(smem_src), "r"(x), "r"(y),
+                 "r"(z), "r"(w)
+                 : "memory");
+}
+
 // A cache policy for data that is written or read once: first in line for eviction from L2.
 __device__ __forceinline__ uint64_t l2_evict_first_policy() {
     uint64_t policy;

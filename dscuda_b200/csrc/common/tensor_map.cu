@@ -97,4 +97,34 @@ CUtensorMap make_u64_rows_map(const void* base, std::uint64_t rows, std::uint32_
     return map;
 }
 
+CUtensorMap make_bf16_batched_rows_map(void* base, std::uint64_t batch, std::uint64_t rows, std::uint32_t cols, std::uint32_t box_rows) {
+    CUtensorMap map;
+    const cuuint64_t dims[3] = {cols, rows, batch};
+    const cuuint64_t strides[2] = {cols * 2ULL, rows * cols * 2ULL};
+    const cuuint32_t box[3] = {64, box_rows, 1};
+    const cuuint32_t element_strides[3] = {1, 1, 1};
+    const CUresult result = encode_entry_point()(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, base, dims, strides, box, element_strides,
+                                                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                                                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (result != CUDA_SUCCESS) {
+        throw std::runtime_error("cuTensorMapEncodeTiled (batched rows) failed with code " + std::to_string(static_cast<int>(result)));
+    }
+    return map;
+}
+
+CUtensorMap make_f32_records_map(void* base, std::uint64_t batch, std::uint64_t rows, std::uint64_t slots, std::uint32_t cols, std::uint32_t box_rows) {
+    CUtensorMap map;
+    const cuuint64_t dims[4] = {cols, slots, rows, batch};
+    const cuuint64_t strides[3] = {cols * 4ULL, slots * cols * 4ULL, rows * slots * cols * 4ULL};
+    const cuuint32_t box[4] = {32, 1, box_rows, 1};
+    const cuuint32_t element_strides[4] = {1, 1, 1, 1};
+    const CUresult result = encode_entry_point()(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, dims, strides, box, element_strides,
+                                                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                                                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (result != CUDA_SUCCESS) {
+        throw std::runtime_error("cuTensorMapEncodeTiled (records) failed with code " + std::to_string(static_cast<int>(result)));
+    }
+    return map;
+}
+
 }  // namespace dscuda
