@@ -44,6 +44,7 @@
 #include "cuda_common.h"
 #include "attention_internal.h"
 #include "sm100_primitives.cuh"
+#include "../common/launch.h"
 #include "../common/tensor_map.h"
 
 #include <algorithm>
@@ -416,6 +417,7 @@ __device__ __forceinline__ void absorbed_pair_body(const DecodeParams& p) {
     volatile int* abort_flag = &sh->abort_flag;
     // Both CTAs must take the same path here: the alignment is a property of the kernel image.
     if ((smem_base & 1023U) != 0U) {
+        grid_dependency_wait();
         if (threadIdx.x == 0) {
             atomicExch(&decode_status, STATUS_SMEM_MISALIGNED);
         }
@@ -447,6 +449,7 @@ __device__ __forceinline__ void absorbed_pair_body(const DecodeParams& p) {
         mbar_init_fence();
     }
     if (warp == 0) {
+        grid_dependency_wait();         // the lengths may come from the kernel in front
         const Schedule schedule = CAUSAL || p.splits == 1 ? Schedule{1, 0, 0, 0} : cut_schedule(p, cluster, clusters, lane);
         if (lane == 0) {
             sh->schedule = schedule;
@@ -466,6 +469,7 @@ __device__ __forceinline__ void absorbed_pair_body(const DecodeParams& p) {
     __syncthreads();
     cluster_sync_all();                 // the other CTA's barriers exist before anything arrives on them
     tc_fence_after_sync();
+    grid_dependency_wait();
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&sh->tmem_base);
     const Schedule schedule = sh->schedule;
 
@@ -1146,6 +1150,7 @@ __global__ void __launch_bounds__(COMBINE_THREADS) decode_combine_kernel(__nv_bf
                                                                          const float2* headers, int rows, int splits) {
     const int lane = threadIdx.x % 32;
     const int row = blockIdx.x * (COMBINE_THREADS / 32) + threadIdx.x / 32;
+    grid_dependency_wait();
     if (row >= rows) {
         return;
     }
@@ -1301,12 +1306,11 @@ void launch_decode(__nv_bfloat16* output, float* logsumexp, const __nv_bfloat16*
     configure_kernel();
     // one cluster of two CTAs per SM pair
     const int clusters = std::max(1, multiprocessor_count() / 2);
-    absorbed_decode_kernel<<<dim3(2 * clusters, 1, 1), THREADS, SMEM_BYTES, stream>>>(params);
-    CUDA_CHECK(cudaGetLastError());
-if (splits > 1) {
-        decode_combine_kernel<<<(batch_size * heads + COMBINE_THREADS / 32 - 1) / (COMBINE_THREADS / 32), COMBINE_THREADS, 0, stream>>>(
-            output, logsumexp, workspace, params.headers, batch_size * heads, splits);
-        CUDA_CHECK(cudaGetLastError());
+    launch_chained(absorbed_decode_kernel, dim3(2 * clusters), dim3(THREADS), SMEM_BYTES, stream, params);
+    if (splits > 1) {
+        const int rows = batch_size * heads;
+        launch_chained(decode_combine_kernel, dim3((rows + COMBINE_THREADS / 32 - 1) / (COMBINE_THREADS / 32)), dim3(COMBINE_THREADS), 0, stream, output,
+                       logsumexp, static_cast<const float*>(workspace), static_cast<const float2*>(params.headers), rows, splits);
     }
 }
 
@@ -1377,8 +1381,7 @@ void mla_compressed_attention_forward_cuda(__nv_bfloat16* output, float* logsume
     configure_kernel();
     const long long row_tiles = (static_cast<long long>(sequence_length) * heads + PAIR_HEADS - 1) / PAIR_HEADS * batch_size;
     const int clusters = static_cast<int>(std::max(1LL, std::min<long long>(multiprocessor_count() / 2, row_tiles)));
-    absorbed_attention_kernel<<<dim3(2 * clusters, 1, 1), THREADS, SMEM_BYTES, stream>>>(params);
-    CUDA_CHECK(cudaGetLastError());
+    launch_chained(absorbed_attention_kernel, dim3(2 * clusters), dim3(THREADS), SMEM_BYTES, stream, params);
 }
 
 std::size_t mla_decode_workspace_elements(int batch_size, int heads, int splits, int kv_rank) {

@@ -37,6 +37,7 @@
 #include "cuda_common.h"
 #include "attention_internal.h"
 #include "sm100_primitives.cuh"
+#include "../common/launch.h"
 #include "../common/tensor_map.h"
 
 #include <algorithm>
@@ -206,6 +207,7 @@ __global__ void __launch_bounds__(256) absorbed_delta_kernel(__nv_bfloat16* dq_r
                                                              size_t rows) {
     const int lane = threadIdx.x % 32;
     const size_t warp_stride = static_cast<size_t>(gridDim.x) * (blockDim.x / 32);
+    grid_dependency_wait();
     for (size_t row = static_cast<size_t>(blockIdx.x) * (blockDim.x / 32) + threadIdx.x / 32; row < rows; row += warp_stride) {
         float sum = 0.0F;
 #pragma unroll
@@ -273,6 +275,7 @@ __global__ void __launch_bounds__(THREADS, 1) absorbed_backward_key_kernel(const
     using namespace ks;
     extern __shared__ uint8_t smem_raw[];
     if (*reinterpret_cast<volatile int*>(&absorbed_backward_status) == STATUS_WAIT_TIMEOUT) {
+        grid_dependency_wait();
         return;
     }
     const int warp = threadIdx.x / 32;
@@ -329,6 +332,7 @@ __global__ void __launch_bounds__(THREADS, 1) absorbed_backward_key_kernel(const
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
+    grid_dependency_wait();
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&sh->tmem_base);
 
     if (warp == LOAD_WARP) {
@@ -559,6 +563,7 @@ __global__ void __launch_bounds__(144) absorbed_backward_reduce_kernel(const __g
     const int parts = key_tile_parts(p, key / KEYS);
     const float* scratch = reinterpret_cast<const float*>(p.dq_lat);
     const int column = threadIdx.x * 4;
+    grid_dependency_wait();
     float4 sum = make_float4(0.0F, 0.0F, 0.0F, 0.0F);
     for (int part = 0; part < parts; ++part) {
         const float4 v = *reinterpret_cast<const float4*>(scratch + ((static_cast<size_t>(part) * p.batch + b) * p.sequence + key) * (RANK + ROPE) + column);
@@ -621,6 +626,7 @@ __global__ void __launch_bounds__(THREADS, 1) absorbed_backward_query_kernel(con
     using namespace qs;
     extern __shared__ uint8_t smem_raw[];
     if (*reinterpret_cast<volatile int*>(&absorbed_backward_status) == STATUS_WAIT_TIMEOUT) {
+        grid_dependency_wait();
         return;
     }
     const int warp = threadIdx.x / 32;
@@ -669,6 +675,7 @@ __global__ void __launch_bounds__(THREADS, 1) absorbed_backward_query_kernel(con
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
+    grid_dependency_wait();
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&sh->tmem_base);
 
     if (warp == LOAD_WARP) {
@@ -957,8 +964,7 @@ void mla_compressed_attention_backward_cuda(__nv_bfloat16* dquery_latent, __nv_b
 
     const std::size_t rows = static_cast<std::size_t>(q_rows);
     const unsigned delta_blocks = static_cast<unsigned>(rows / 8 + 1 < 148 * 16 ? rows / 8 + 1 : 148 * 16);
-    absorbed_delta_kernel<<<delta_blocks, 256, 0, stream>>>(dquery_rope, output_gradient, output, rows);
-    CUDA_CHECK(cudaGetLastError());
+    launch_chained(absorbed_delta_kernel, dim3(delta_blocks), dim3(256), 0, stream, dquery_rope, output_gradient, output, rows);
     // Key side split (see key_tile_parts): about four waves of CTAs of equal length, never more
     // parts per key tile than fp32 partial rows fit into the dquery_latent buffer.
     const int key_tiles = (sequence_length + KEYS - 1) / KEYS;
@@ -979,15 +985,12 @@ void mla_compressed_attention_backward_cuda(__nv_bfloat16* dquery_latent, __nv_b
     params.key_chunk = static_cast<int>(std::min<long long>(chunk, 0x7fffffffLL));
     params.key_direct = part_count == key_tiles ? 1 : 0;
     const dim3 key_grid(static_cast<unsigned>(part_count), 2, batch_size);
-    absorbed_backward_key_kernel<<<key_grid, THREADS, ks::SMEM_BYTES, stream>>>(params);
-    CUDA_CHECK(cudaGetLastError());
+    launch_chained(absorbed_backward_key_kernel, key_grid, dim3(THREADS), ks::SMEM_BYTES, stream, params);
     if (params.key_direct == 0) {
-        absorbed_backward_reduce_kernel<<<dim3(sequence_length, batch_size), 144, 0, stream>>>(params);
-        CUDA_CHECK(cudaGetLastError());
+        launch_chained(absorbed_backward_reduce_kernel, dim3(sequence_length, batch_size), dim3(144), 0, stream, params);
     }
     const dim3 query_grid(static_cast<unsigned>((rows_per_sequence + ROWS - 1) / ROWS), 1, batch_size);
-    absorbed_backward_query_kernel<<<query_grid, THREADS, qs::SMEM_BYTES, stream>>>(params);
-    CUDA_CHECK(cudaGetLastError());
+    launch_chained(absorbed_backward_query_kernel, query_grid, dim3(THREADS), qs::SMEM_BYTES, stream, params);
 }
 
 }  // namespace dscuda

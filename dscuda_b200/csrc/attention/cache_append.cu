@@ -16,6 +16,7 @@
 #include "cuda_common.h"
 #include "attention_internal.h"
 #include "sm100_primitives.cuh"
+#include "../common/launch.h"
 
 #include <cuda_fp8.h>
 
@@ -38,6 +39,7 @@ __global__ void __launch_bounds__(APPEND_THREADS) cache_append_kernel(uint4* cac
     const int lane = threadIdx.x % 32;
     const long long warps = static_cast<long long>(gridDim.x) * (APPEND_THREADS / 32);
     const long long total = static_cast<long long>(batch) * tokens;
+    sm100::grid_dependency_wait();
     for (long long item = static_cast<long long>(blockIdx.x) * (APPEND_THREADS / 32) + threadIdx.x / 32; item < total; item += warps) {
         const int b = static_cast<int>(item / tokens);
         const int t = static_cast<int>(item % tokens);
@@ -100,6 +102,7 @@ __global__ void __launch_bounds__(APPEND_THREADS) cache_append_fp8_kernel(uint8_
     const int lane = threadIdx.x % 32;
     const long long warps = static_cast<long long>(gridDim.x) * (APPEND_THREADS / 32);
     const long long total = static_cast<long long>(batch) * tokens;
+    sm100::grid_dependency_wait();
     for (long long item = static_cast<long long>(blockIdx.x) * (APPEND_THREADS / 32) + threadIdx.x / 32; item < total; item += warps) {
         const int b = static_cast<int>(item / tokens);
         const int t = static_cast<int>(item % tokens);
@@ -159,6 +162,7 @@ __global__ void __launch_bounds__(APPEND_THREADS) cache_append_fp8_kernel(uint8_
 __global__ void __launch_bounds__(APPEND_THREADS) cache_dequantize_fp8_kernel(uint4* bf16_cache, const uint8_t* fp8_cache, long long rows) {
     const int lane = threadIdx.x % 32;
     const long long warps = static_cast<long long>(gridDim.x) * (APPEND_THREADS / 32);
+    sm100::grid_dependency_wait();
     for (long long row = static_cast<long long>(blockIdx.x) * (APPEND_THREADS / 32) + threadIdx.x / 32; row < rows; row += warps) {
         const uint8_t* src = fp8_cache + row * FP8_ROW_BYTES;
         uint4* dst = bf16_cache + row * ROW_UNITS;
@@ -223,10 +227,9 @@ void mla_cache_append_cuda(__nv_bfloat16* paged_kv_cache, const __nv_bfloat16* k
     const long long total = static_cast<long long>(batch_size) * tokens;
     const long long wanted = (total + APPEND_THREADS / 32 - 1) / (APPEND_THREADS / 32);
     const unsigned blocks = static_cast<unsigned>(wanted < 148LL * 8 ? wanted : 148LL * 8);      // 8 resident CTAs on each of 148 SMs
-    cache_append_kernel<<<blocks, APPEND_THREADS, 0, stream>>>(reinterpret_cast<uint4*>(paged_kv_cache), reinterpret_cast<const uint4*>(kv_latent),
+    launch_chained(cache_append_kernel, dim3(blocks), dim3(APPEND_THREADS), 0, stream, reinterpret_cast<uint4*>(paged_kv_cache), reinterpret_cast<const uint4*>(kv_latent),
                                                                reinterpret_cast<const uint4*>(key_rope), block_table, start_positions, token_counts,
                                                                batch_size, tokens, page_size, pages_per_sequence, cache_blocks);
-    CUDA_CHECK(cudaGetLastError());
 }
 
 void mla_cache_append_fp8_cuda(void* paged_fp8_cache, const __nv_bfloat16* kv_latent, const __nv_bfloat16* key_rope, const int* block_table,
@@ -249,10 +252,9 @@ void mla_cache_append_fp8_cuda(void* paged_fp8_cache, const __nv_bfloat16* kv_la
     const long long total = static_cast<long long>(batch_size) * tokens;
     const long long wanted = (total + APPEND_THREADS / 32 - 1) / (APPEND_THREADS / 32);
     const unsigned blocks = static_cast<unsigned>(wanted < 148LL * 8 ? wanted : 148LL * 8);
-    cache_append_fp8_kernel<<<blocks, APPEND_THREADS, 0, stream>>>(static_cast<uint8_t*>(paged_fp8_cache), reinterpret_cast<const uint4*>(kv_latent),
+    launch_chained(cache_append_fp8_kernel, dim3(blocks), dim3(APPEND_THREADS), 0, stream, static_cast<uint8_t*>(paged_fp8_cache), reinterpret_cast<const uint4*>(kv_latent),
                                                                    reinterpret_cast<const uint4*>(key_rope), block_table, start_positions,
                                                                    token_counts, batch_size, tokens, page_size, pages_per_sequence, cache_blocks);
-    CUDA_CHECK(cudaGetLastError());
 }
 
 void mla_cache_dequantize_fp8_cuda(__nv_bfloat16* paged_kv_cache, const void* paged_fp8_cache, long long first_row, long long rows,
@@ -267,9 +269,8 @@ void mla_cache_dequantize_fp8_cuda(__nv_bfloat16* paged_kv_cache, const void* pa
     }
     const long long wanted = (rows + APPEND_THREADS / 32 - 1) / (APPEND_THREADS / 32);
     const unsigned blocks = static_cast<unsigned>(wanted < 148LL * 8 ? wanted : 148LL * 8);
-    cache_dequantize_fp8_kernel<<<blocks, APPEND_THREADS, 0, stream>>>(reinterpret_cast<uint4*>(paged_kv_cache) + first_row * ROW_UNITS,
+    launch_chained(cache_dequantize_fp8_kernel, dim3(blocks), dim3(APPEND_THREADS), 0, stream, reinterpret_cast<uint4*>(paged_kv_cache) + first_row * ROW_UNITS,
                                                                        static_cast<const uint8_t*>(paged_fp8_cache) + first_row * FP8_ROW_BYTES, rows);
-    CUDA_CHECK(cudaGetLastError());
 }
 
 }  // namespace dscuda

@@ -31,6 +31,7 @@
 #include "cuda_common.h"
 #include "attention_internal.h"
 #include "sm100_primitives.cuh"
+#include "../common/launch.h"
 #include "../common/tensor_map.h"
 
 #include <atomic>
@@ -123,6 +124,7 @@ __device__ __forceinline__ bool locate_block(const BackwardParams& p, int rows_p
         lse_offset = (static_cast<size_t>(b) * p.heads + head) * p.max_seq;
         return block < blocks_in_sequence;
     }
+    grid_dependency_wait();
     for (int sequence = 0; sequence < p.batch; ++sequence) {
         const int begin = p.cu_seqlens[sequence];
         const int tokens = p.cu_seqlens[sequence + 1] - begin;
@@ -210,6 +212,7 @@ __global__ void __launch_bounds__(256) delta_kernel(float* delta, const __nv_bfl
     // half a warp per (row, head): 16 lanes x 16 bytes cover the 128 values of dO and of O
     const int half = lane / 16;
     const int part = lane % 16;
+    grid_dependency_wait();
     for (size_t base = (static_cast<size_t>(blockIdx.x) * (blockDim.x / 32) + threadIdx.x / 32) * 2; base < pairs; base += warp_stride * 2) {
         const size_t pair = base + half;
         float sum = 0.0F;
@@ -250,6 +253,7 @@ __global__ void __launch_bounds__(256) sum_dk_pe_kernel(__nv_bfloat16* dk_pe, fl
     // 16 threads per key row, four columns each; the heads are added in index order, so the sum
     // does not depend on how the CTAs of the key-side kernel were scheduled
     const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
+    grid_dependency_wait();
     for (size_t index = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; index < rows * 16; index += stride) {
         const float4* src = parts + (index / 16) * static_cast<size_t>(heads) * 16 + index % 16;
         float4 total = make_float4(0.0F, 0.0F, 0.0F, 0.0F);
@@ -320,6 +324,7 @@ __global__ void __launch_bounds__(THREADS, 1) backward_dq_kernel(const __grid_co
     using namespace dqk;
     extern __shared__ uint8_t smem_raw[];
     if (*reinterpret_cast<volatile int*>(&backward_status) != 0) {
+        grid_dependency_wait();
         return;
     }
     const int head = blockIdx.y;
@@ -337,6 +342,7 @@ __global__ void __launch_bounds__(THREADS, 1) backward_dq_kernel(const __grid_co
     // dynamic region starts 1024-byte aligned when the kernel has no static shared memory.
     const uint32_t smem_base = smem_u32(smem_raw);
     if ((smem_base & 1023U) != 0U) {
+        grid_dependency_wait();
         if (threadIdx.x == 0) {
             atomicExch(&backward_status, STATUS_SMEM_MISALIGNED);
         }
@@ -374,6 +380,7 @@ __global__ void __launch_bounds__(THREADS, 1) backward_dq_kernel(const __grid_co
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
+    grid_dependency_wait();
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&bars->tmem_base);
 
     if (warp == LOAD_WARP) {
@@ -629,6 +636,7 @@ __global__ void __launch_bounds__(THREADS, 1) backward_dq_kernel(const __grid_co
 __global__ void __launch_bounds__(THREADS, 1) backward_dkdv_kernel(const __grid_constant__ BackwardParams p) {
     extern __shared__ uint8_t smem_raw[];
     if (*reinterpret_cast<volatile int*>(&backward_status) != 0) {
+        grid_dependency_wait();
         return;
     }
     const int head = p.head0 + blockIdx.y;
@@ -662,6 +670,7 @@ __global__ void __launch_bounds__(THREADS, 1) backward_dkdv_kernel(const __grid_
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
+    grid_dependency_wait();
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&bars->tmem_base);
     constexpr uint32_t TMEM_DV = 0;
     constexpr uint32_t TMEM_DK = 128;
@@ -993,6 +1002,7 @@ __global__ void __launch_bounds__(dqs::STREAM_THREADS, 1) backward_dq_stream_ker
         using namespace dqs;
     extern __shared__ uint8_t smem_raw[];
     if (*reinterpret_cast<volatile int*>(&backward_status) != 0) {
+        grid_dependency_wait();
         return;
     }
     const int head = p.head0 + blockIdx.y;
@@ -1034,6 +1044,7 @@ __global__ void __launch_bounds__(dqs::STREAM_THREADS, 1) backward_dq_stream_ker
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
+    grid_dependency_wait();
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&bars->tmem_base);
 
     // A stage holds keys [64 s, 64 s + 64).  The first accumulator (rows q_start..q_start+127)
@@ -1281,8 +1292,7 @@ void mla_prefill_backward_cuda(__nv_bfloat16* dq, __nv_bfloat16* dk_nope, __nv_b
 
     const std::size_t pairs = static_cast<std::size_t>(total_tokens) * heads;
     const unsigned delta_blocks = static_cast<unsigned>(pairs / 8 + 1 < 148 * 32 ? pairs / 8 + 1 : 148 * 32);
-    delta_kernel<<<delta_blocks, 256, 0, stream>>>(delta, output_gradient, output, cu_seqlens, batch_size, max_sequence_length, total_tokens, heads);
-    CUDA_CHECK(cudaGetLastError());
+    launch_chained(delta_kernel, dim3(delta_blocks), dim3(256), 0, stream, delta, output_gradient, output, cu_seqlens, batch_size, max_sequence_length, total_tokens, heads);
 
     const int group = ds_group_heads(batch_size, max_sequence_length, total_tokens, heads);
     if (group > 0) {
@@ -1304,10 +1314,8 @@ void mla_prefill_backward_cuda(__nv_bfloat16* dq, __nv_bfloat16* dk_nope, __nv_b
             params.head0 = head0;
             key_grid.y = count;
             query_grid.y = count;
-            backward_dkdv_kernel<<<key_grid, THREADS, SMEM_BYTES, stream>>>(params);
-            CUDA_CHECK(cudaGetLastError());
-            backward_dq_stream_kernel<<<query_grid, dqs::STREAM_THREADS, dqs::STREAM_SMEM_BYTES, stream>>>(params);
-            CUDA_CHECK(cudaGetLastError());
+            launch_chained(backward_dkdv_kernel, key_grid, dim3(THREADS), SMEM_BYTES, stream, params);
+            launch_chained(backward_dq_stream_kernel, query_grid, dim3(dqs::STREAM_THREADS), dqs::STREAM_SMEM_BYTES, stream, params);
         }
     } else {
         dim3 grid;
@@ -1318,15 +1326,12 @@ void mla_prefill_backward_cuda(__nv_bfloat16* dq, __nv_bfloat16* dk_nope, __nv_b
         }
         params.ds_scratch = nullptr;
         params.head0 = 0;
-        backward_dq_kernel<<<grid, THREADS, dqk::SMEM_BYTES, stream>>>(params);
-        CUDA_CHECK(cudaGetLastError());
-        backward_dkdv_kernel<<<grid, THREADS, SMEM_BYTES, stream>>>(params);
-        CUDA_CHECK(cudaGetLastError());
+        launch_chained(backward_dq_kernel, grid, dim3(THREADS), dqk::SMEM_BYTES, stream, params);
+        launch_chained(backward_dkdv_kernel, grid, dim3(THREADS), SMEM_BYTES, stream, params);
     }
     const std::size_t quads = static_cast<std::size_t>(total_tokens) * 16;
     const unsigned sum_blocks = static_cast<unsigned>(quads / 256 + 1 < 148 * 8 ? quads / 256 + 1 : 148 * 8);
-    sum_dk_pe_kernel<<<sum_blocks, 256, 0, stream>>>(dk_pe, accumulator, reinterpret_cast<const float4*>(parts), static_cast<std::size_t>(total_tokens), heads);
-    CUDA_CHECK(cudaGetLastError());
+    launch_chained(sum_dk_pe_kernel, dim3(sum_blocks), dim3(256), 0, stream, dk_pe, accumulator, reinterpret_cast<const float4*>(parts), static_cast<std::size_t>(total_tokens), heads);
 }
 
 }  // namespace dscuda

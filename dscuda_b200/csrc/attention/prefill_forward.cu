@@ -24,6 +24,7 @@
 #include "cuda_common.h"
 #include "attention_internal.h"
 #include "sm100_primitives.cuh"
+#include "../common/launch.h"
 #include "../common/tensor_map.h"
 
 #include <stdexcept>
@@ -93,6 +94,7 @@ __global__ void __launch_bounds__(FORWARD_THREADS, 1) attention_forward_kernel(c
     extern __shared__ uint8_t smem_raw[];
 
     if (*reinterpret_cast<volatile int*>(&forward_status) != 0) {
+        grid_dependency_wait();
         return;
     }
 
@@ -109,6 +111,7 @@ __global__ void __launch_bounds__(FORWARD_THREADS, 1) attention_forward_kernel(c
         qblock = static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x);
         lse_base = p.lse + (static_cast<size_t>(b) * p.heads + head) * p.max_seq;
     } else {
+        grid_dependency_wait();
         int index = blockIdx.x;
         int sequence = 0;
         int begin = 0;
@@ -178,6 +181,7 @@ __global__ void __launch_bounds__(FORWARD_THREADS, 1) attention_forward_kernel(c
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
+    grid_dependency_wait();
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&bars->tmem_base);
 
     // Registers: the CTA starts with 168 per thread (12 warps).  The softmax keeps a 128-column
@@ -557,8 +561,7 @@ void launch_prefill_forward(__nv_bfloat16* output, float* logsumexp, const __nv_
     } else {
         grid = dim3(total_tokens / 256 + batch_size, heads, 1);
     }
-    attention_forward_kernel<3><<<grid, FORWARD_THREADS, ForwardLayout<3>::SMEM_BYTES, stream>>>(params);
-    CUDA_CHECK(cudaGetLastError());
+    launch_chained(attention_forward_kernel<3>, grid, dim3(FORWARD_THREADS), ForwardLayout<3>::SMEM_BYTES, stream, params);
 }
 
 int forward_device_status(bool reset) {
@@ -623,8 +626,7 @@ void flash_attention_forward_cuda(__nv_bfloat16* output, float* logsumexp, const
     params.scale_log2 = scale * 1.4426950408889634F;
     configure_forward_kernel<2>();
     const dim3 grid((sequence_length + 255) / 256, query_heads, batch_size);
-    attention_forward_kernel<2><<<grid, FORWARD_THREADS, ForwardLayout<2>::SMEM_BYTES, stream>>>(params);
-    CUDA_CHECK(cudaGetLastError());
+    launch_chained(attention_forward_kernel<2>, grid, dim3(FORWARD_THREADS), ForwardLayout<2>::SMEM_BYTES, stream, params);
 }
 
 }  // namespace dscuda

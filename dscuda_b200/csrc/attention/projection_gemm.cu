@@ -24,6 +24,7 @@
 #include "cuda_common.h"
 #include "attention_internal.h"
 #include "sm100_primitives.cuh"
+#include "../common/launch.h"
 #include "../common/tensor_map.h"
 
 #include <algorithm>
@@ -79,6 +80,7 @@ static_assert(sizeof(Shared) <= MISC_BYTES, "barrier block too large");
 __global__ void __launch_bounds__(THREADS, 1) projection_gemm_kernel(const __grid_constant__ GemmParams p) {
     extern __shared__ uint8_t smem_raw[];
     if (*reinterpret_cast<volatile int*>(&projection_status) == STATUS_WAIT_TIMEOUT) {
+        grid_dependency_wait();
         return;
     }
     const int warp = threadIdx.x / 32;
@@ -114,6 +116,7 @@ __global__ void __launch_bounds__(THREADS, 1) projection_gemm_kernel(const __gri
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
+    grid_dependency_wait();
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&sh->tmem_base);
 
     const int tiles_m = (p.m + TILE_M - 1) / TILE_M;
@@ -337,8 +340,7 @@ void launch_gemm(__nv_bfloat16* c, const __nv_bfloat16* a, const __nv_bfloat16* 
     configure_kernel();
     const long long tiles = ((m + TILE_M - 1) / TILE_M) * (n / TILE_N) * batch;
     const unsigned grid = static_cast<unsigned>(std::min<long long>(tiles, sm_count()));
-    projection_gemm_kernel<<<grid, THREADS, SMEM_BYTES, stream>>>(params);
-    CUDA_CHECK(cudaGetLastError());
+    launch_chained(projection_gemm_kernel, dim3(grid), dim3(THREADS), SMEM_BYTES, stream, params);
 }
 
 void check_heads(long long rows, int heads) {

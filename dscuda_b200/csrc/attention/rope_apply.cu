@@ -16,6 +16,8 @@
 // once.
 #include "mla.h"
 #include "cuda_common.h"
+#include "sm100_primitives.cuh"
+#include "../common/launch.h"
 
 #include <cstdint>
 #include <stdexcept>
@@ -54,6 +56,7 @@ __global__ void __launch_bounds__(ROPE_THREADS) rope_apply_kernel(uint32_t* q_pe
     const long long warps = static_cast<long long>(gridDim.x) * (ROPE_THREADS / 32);
     const double inv0 = exp2(-log2_theta * (2.0 * (2 * slot)) / 64.0);
     const double inv1 = exp2(-log2_theta * (2.0 * (2 * slot + 1)) / 64.0);
+    sm100::grid_dependency_wait();
     for (long long row = static_cast<long long>(blockIdx.x) * (ROPE_THREADS / 32) + threadIdx.x / 32; row < rows; row += warps) {
         const int position = positions != nullptr ? positions[row] : static_cast<int>(row % sequence_length);
         double s0d, c0d, s1d, c1d;
@@ -113,9 +116,8 @@ void mla_rope_apply_cuda(__nv_bfloat16* q_pe, __nv_bfloat16* k_pe, const int* po
     }
     const long long wanted = (rows + ROPE_THREADS / 32 - 1) / (ROPE_THREADS / 32);
     const unsigned blocks = static_cast<unsigned>(wanted < 148LL * 8 ? wanted : 148LL * 8);      // 8 resident CTAs on each of 148 SMs
-    rope_apply_kernel<<<blocks, ROPE_THREADS, 0, stream>>>(reinterpret_cast<uint32_t*>(q_pe), reinterpret_cast<uint32_t*>(k_pe), positions, rows, heads,
+    launch_chained(rope_apply_kernel, dim3(blocks), dim3(ROPE_THREADS), 0, stream, reinterpret_cast<uint32_t*>(q_pe), reinterpret_cast<uint32_t*>(k_pe), positions, rows, heads,
                                                            sequence_length, log2(static_cast<double>(theta)));
-    CUDA_CHECK(cudaGetLastError());
 }
 
 }  // namespace dscuda

@@ -37,6 +37,14 @@ __device__ __forceinline__ uint32_t lane_id() {
 }
 
 // ---------------------------------------------------------------------------
+// Dependent launches (../common/launch.h).  The wait comes before the first access to global memory; at least one
+// block of every grid has to reach it, or the grid could end before the one in front of it.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void grid_dependency_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// ---------------------------------------------------------------------------
 // mbarrier
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
