@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(APPEND_THREADS) cache_append_kernel(uint4* cac
 //   cache_append_fp8_kernel      quantises and writes new tokens' rows (same addressing as above);
 //   cache_dequantize_fp8_kernel  rewrites a range of physical rows in the bf16 layout the decode
 //                                kernel reads.
-// One warp per token in both: a lane owns 16 latent columns (one 16-byte unit of e4m3), eight lanes
+// One warp per token in the first: a lane owns 16 latent columns (one 16-byte unit of e4m3), eight lanes
 // own a scale group.
 // ---------------------------------------------------------------------------
 constexpr int FP8_ROW_BYTES = MLA_FP8_CACHE_ROW_BYTES;                  // 656
@@ -159,30 +159,49 @@ __global__ void __launch_bounds__(APPEND_THREADS) cache_append_fp8_kernel(uint8_
     }
 }
 
+// Two rows per pass, all loads before the first store; a lane owns columns 8 lane .. 8 lane + 7 and the same 256 further
+// on, so that each store instruction of a warp writes 512 consecutive bytes.  With one row per pass and 16 neighbouring
+// columns per lane (stores of 16 bytes 32 apart) 57,000 rows took 23.7 us.
 __global__ void __launch_bounds__(APPEND_THREADS) cache_dequantize_fp8_kernel(uint4* bf16_cache, const uint8_t* fp8_cache, long long rows) {
+    constexpr int PASS = 2;
     const int lane = threadIdx.x % 32;
     const long long warps = static_cast<long long>(gridDim.x) * (APPEND_THREADS / 32);
     sm100::grid_dependency_wait();
-    for (long long row = static_cast<long long>(blockIdx.x) * (APPEND_THREADS / 32) + threadIdx.x / 32; row < rows; row += warps) {
-        const uint8_t* src = fp8_cache + row * FP8_ROW_BYTES;
-        uint4* dst = bf16_cache + row * ROW_UNITS;
-        const uint4 quantised = __ldg(reinterpret_cast<const uint4*>(src) + lane);
-        const float scale = __ldg(reinterpret_cast<const float*>(src + FP8_SCALES_OFFSET) + (lane >> 3));
-        const uint32_t words[4] = {quantised.x, quantised.y, quantised.z, quantised.w};
-        uint32_t out[8];
+    for (long long first = (static_cast<long long>(blockIdx.x) * (APPEND_THREADS / 32) + threadIdx.x / 32) * PASS; first < rows; first += warps * PASS) {
+        uint2 codes[PASS][2];
+        float scales[PASS][2];
+        uint4 rope[PASS];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
+        for (int i = 0; i < PASS; ++i) {
+            const uint8_t* src = fp8_cache + min(first + i, rows - 1) * FP8_ROW_BYTES;
 #pragma unroll
             for (int half = 0; half < 2; ++half) {
-                const __half2_raw h = __nv_cvt_fp8x2_to_halfraw2(static_cast<__nv_fp8x2_storage_t>((words[e] >> (16 * half)) & 0xffffU), __NV_E4M3);
-                const float2 x = __half22float2(*reinterpret_cast<const __half2*>(&h));
-                out[2 * e + half] = sm100::pack_bf16x2(x.x * scale, x.y * scale);
+                codes[i][half] = __ldg(reinterpret_cast<const uint2*>(src) + half * 32 + lane);
+                scales[i][half] = __ldg(reinterpret_cast<const float*>(src + FP8_SCALES_OFFSET) + half * 2 + (lane >> 4));
             }
+            rope[i] = lane < ROPE_UNITS ? __ldg(reinterpret_cast<const uint4*>(src + FP8_ROPE_OFFSET) + lane) : make_uint4(0, 0, 0, 0);
         }
-        dst[2 * lane] = make_uint4(out[0], out[1], out[2], out[3]);
-        dst[2 * lane + 1] = make_uint4(out[4], out[5], out[6], out[7]);
-        if (lane < ROPE_UNITS) {
-            dst[LATENT_UNITS + lane] = __ldg(reinterpret_cast<const uint4*>(src + FP8_ROPE_OFFSET) + lane);
+#pragma unroll
+        for (int i = 0; i < PASS; ++i) {
+            if (first + i >= rows) {
+                break;
+            }
+            uint4* dst = bf16_cache + (first + i) * ROW_UNITS;
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                const uint32_t words[2] = {codes[i][half].x, codes[i][half].y};
+                uint32_t out[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const __half2_raw h = __nv_cvt_fp8x2_to_halfraw2(static_cast<__nv_fp8x2_storage_t>((words[e / 2] >> (16 * (e % 2))) & 0xffffU), __NV_E4M3);
+                    const float2 x = __half22float2(*reinterpret_cast<const __half2*>(&h));
+                    out[e] = sm100::pack_bf16x2(x.x * scales[i][half], x.y * scales[i][half]);
+                }
+                dst[half * 32 + lane] = make_uint4(out[0], out[1], out[2], out[3]);
+            }
+            if (lane < ROPE_UNITS) {
+                dst[LATENT_UNITS + lane] = rope[i];
+            }
         }
     }
 }
@@ -267,7 +286,7 @@ void mla_cache_dequantize_fp8_cuda(__nv_bfloat16* paged_kv_cache, const void* pa
             throw std::invalid_argument("tensor pointers must be non-null and 16-byte aligned");
         }
     }
-    const long long wanted = (rows + APPEND_THREADS / 32 - 1) / (APPEND_THREADS / 32);
+    const long long wanted = (rows + APPEND_THREADS / 16 - 1) / (APPEND_THREADS / 16);      // two rows per warp and pass
     const unsigned blocks = static_cast<unsigned>(wanted < 148LL * 8 ? wanted : 148LL * 8);
     launch_chained(cache_dequantize_fp8_kernel, dim3(blocks), dim3(APPEND_THREADS), 0, stream, reinterpret_cast<uint4*>(paged_kv_cache) + first_row * ROW_UNITS,
                                                                        static_cast<const uint8_t*>(paged_fp8_cache) + first_row * FP8_ROW_BYTES, rows);
