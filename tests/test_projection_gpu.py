@@ -60,3 +60,22 @@ def test_absorbed_decode_equals_attention_over_up_projected_cache(gpu):
     score = (torch.einsum("bqhc,bkhc->bhqk", q_nope.float(), k_nope) + torch.einsum("bqhr,bkr->bhqk", q_pe.float(), k_pe.float())) * scale
     ref = torch.einsum("bhqk,bkhd->bqhd", score.softmax(-1), v)
     assert max_err_ratio(out.float().cpu(), ref) <= 2e-2        # two bf16 roundings (q_latent, o_latent) on the absorbed route
+
+
+@pytest.mark.parametrize("rows,heads", [(3001, 7), (25000, 1), (1153, 65)])
+def test_pair_kernel_tile_edges(gpu, rows, heads):
+    """Sizes that reach the two-CTA kernel with a remainder in every direction: rows past the last 256-row tile (the second
+    CTA of a pair without any), a last column tile of 128 of its 256 columns, one head's 128 columns alone."""
+    from dscuda_b200 import mla
+    g = torch.Generator().manual_seed(rows)
+    latent, w_uk, w_uv = draw(g, rows, 512), draw(g, heads * 128, 512, std=0.05), draw(g, heads * 128, 512, std=0.05)
+    q_nope = draw(g, rows, heads, 128)
+    k_nope, v = mla.up_project(latent.to(gpu), w_uk.to(gpu), w_uv.to(gpu), heads)
+    q_latent = mla.absorb_query(q_nope.to(gpu), w_uk.to(gpu))
+    torch.cuda.synchronize()
+    assert mla.device_status() == 0
+    ref_k = (latent.float() @ w_uk.float().T).reshape(rows, heads, 128)
+    ref_v = (latent.float() @ w_uv.float().T).reshape(rows, heads, 128)
+    ref_q = torch.einsum("rhk,hkn->rhn", q_nope.float(), w_uk.float().reshape(heads, 128, 512))
+    for got, ref in ((k_nope, ref_k), (v, ref_v), (q_latent, ref_q)):
+        assert max_err_ratio(got.float().cpu(), ref) <= 2 ** -7
