@@ -34,6 +34,7 @@
 #include "../common/launch.h"
 #include "../common/tensor_map.h"
 
+#include <algorithm>
 #include <atomic>
 #include <cstddef>
 #include <stdexcept>
@@ -65,6 +66,8 @@ struct BackwardParams {
     // 128-row boxes (stationary tiles) and 64-row boxes (streamed tiles) of the same tensors
     CUtensorMap q_main_big, q_pe_big, k_main_big, k_pe_big, v_big, do_big;
     CUtensorMap q_main_sub, q_pe_sub, k_main_sub, k_pe_sub, v_sub, do_sub;
+    // stores of 32 rows: 64 bf16 columns of the gradients, 32 fp32 columns of a head's dk_pe contributions
+    CUtensorMap dq_map, dk_map, dv_map, parts_map;
     __nv_bfloat16* dq;        // [rows, H, 192]
     __nv_bfloat16* dk_nope;   // [rows, H, 128]
     __nv_bfloat16* dv;        // [rows, H, 128]
@@ -201,6 +204,29 @@ __device__ __forceinline__ void store_bf16_row(__nv_bfloat16* dst, const uint32_
     }
 }
 
+// Result tiles leave through shared memory that is idle by then: a warp lays out 32 rows x 128 bytes at a time in a 4 KB slab
+// (128-byte swizzle), from where a TMA store writes whole lines.  A thread that stores its own row touches 32 lines per
+// instruction, which cost 2-3 us of every CTA.  Rows behind the ragged end of a sequence may be another sequence's, so a
+// warp with such rows still stores thread by thread.
+constexpr int SLAB_BYTES = 32 * 128;
+
+__device__ __forceinline__ void slab_bf16x32(uint8_t* slab, int lane, int half, const uint32_t* values) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const uint32_t* x = values + 8 * u;
+        *reinterpret_cast<uint4*>(slab + lane * 128 + (((half * 4 + u) ^ (lane & 7)) * 16)) =
+            make_uint4(pack_bf16x2(__uint_as_float(x[0]), __uint_as_float(x[1])), pack_bf16x2(__uint_as_float(x[2]), __uint_as_float(x[3])),
+                       pack_bf16x2(__uint_as_float(x[4]), __uint_as_float(x[5])), pack_bf16x2(__uint_as_float(x[6]), __uint_as_float(x[7])));
+    }
+}
+
+__device__ __forceinline__ void slab_f32x32(uint8_t* slab, int lane, const uint32_t* values) {
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+        *reinterpret_cast<uint4*>(slab + lane * 128 + ((u ^ (lane & 7)) * 16)) = make_uint4(values[4 * u], values[4 * u + 1], values[4 * u + 2], values[4 * u + 3]);
+    }
+}
+
 // ---------------------------------------------------------------------------
 // delta[q] = sum_d dO[q,d] * O[q,d]; half a warp per (row, head).
 // ---------------------------------------------------------------------------
@@ -249,24 +275,49 @@ __global__ void __launch_bounds__(256) delta_kernel(float* delta, const __nv_bfl
 // ---------------------------------------------------------------------------
 // per-head dk_pe contributions -> fp32 sums and bf16 dk_pe
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) sum_dk_pe_kernel(__nv_bfloat16* dk_pe, float* sums, const float4* parts, size_t rows, int heads) {
-    // 16 threads per key row, four columns each; the heads are added in index order, so the sum
-    // does not depend on how the CTAs of the key-side kernel were scheduled
-    const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
+// A CTA takes four key rows: 16 threads x four columns each, times four quarters of the heads.  The heads of a quarter are
+// added in index order and the quarters in order, so the sum does not depend on how the CTAs of the key-side kernel were
+// scheduled.  One thread per (row, column group) for all the heads left a short batch of 64 heads waiting eight memory
+// latencies in a row (10 us).
+constexpr int SUM_ROWS = 4;
+constexpr int SUM_QUARTERS = 4;
+
+__global__ void __launch_bounds__(SUM_ROWS * 16 * SUM_QUARTERS) sum_dk_pe_kernel(__nv_bfloat16* dk_pe, float* sums, const float4* parts, size_t rows,
+                                                                                  int heads) {
+    __shared__ float4 partial[SUM_QUARTERS][SUM_ROWS * 16];
+    const int item = threadIdx.x % (SUM_ROWS * 16);
+    const int quarter = threadIdx.x / (SUM_ROWS * 16);
+    const int head_begin = heads * quarter / SUM_QUARTERS, head_end = heads * (quarter + 1) / SUM_QUARTERS;
     grid_dependency_wait();
-    for (size_t index = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; index < rows * 16; index += stride) {
-        const float4* src = parts + (index / 16) * static_cast<size_t>(heads) * 16 + index % 16;
+    for (size_t first = static_cast<size_t>(blockIdx.x) * SUM_ROWS; first < rows; first += static_cast<size_t>(gridDim.x) * SUM_ROWS) {
+        const size_t index = first * 16 + item;
         float4 total = make_float4(0.0F, 0.0F, 0.0F, 0.0F);
+        if (index < rows * 16) {
+            const float4* src = parts + (index / 16) * static_cast<size_t>(heads) * 16 + index % 16;
 #pragma unroll 8
-        for (int h = 0; h < heads; ++h) {
-            const float4 x = __ldg(src + static_cast<size_t>(h) * 16);
-            total.x += x.x;
-            total.y += x.y;
-            total.z += x.z;
-            total.w += x.w;
+            for (int h = head_begin; h < head_end; ++h) {
+                const float4 x = __ldg(src + static_cast<size_t>(h) * 16);
+                total.x += x.x;
+                total.y += x.y;
+                total.z += x.z;
+                total.w += x.w;
+            }
         }
-        reinterpret_cast<float4*>(sums)[index] = total;
-        reinterpret_cast<uint2*>(dk_pe)[index] = make_uint2(pack_bf16x2(total.x, total.y), pack_bf16x2(total.z, total.w));
+        partial[quarter][item] = total;
+        __syncthreads();
+        if (quarter == 0 && index < rows * 16) {
+#pragma unroll
+            for (int q = 1; q < SUM_QUARTERS; ++q) {
+                const float4 x = partial[q][item];
+                total.x += x.x;
+                total.y += x.y;
+                total.z += x.z;
+                total.w += x.w;
+            }
+            reinterpret_cast<float4*>(sums)[index] = total;
+            reinterpret_cast<uint2*>(dk_pe)[index] = make_uint2(pack_bf16x2(total.x, total.y), pack_bf16x2(total.z, total.w));
+        }
+        __syncthreads();
     }
 }
 
@@ -914,25 +965,47 @@ __global__ void __launch_bounds__(THREADS, 1) backward_dkdv_kernel(const __grid_
             tc_fence_after_sync();
             const bool valid = key_pos < length;
             const size_t row = static_cast<size_t>(row0 + key_pos);
+            // every MMA has finished: the K, V and streamed tiles are idle
+            const int warp_row = key_start + (warp % 4) * 32;
+            const bool whole = warp_row + 32 <= length;
             if (group == 0) {
                 __nv_bfloat16* dv_row = p.dv + (row * p.heads + head) * 128;
+                const int slab = (warp % 4) * 2 * SLAB_BYTES;
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     uint32_t values[32];
                     tmem_ld_x32(tmem_base + lane_base + TMEM_DV + c * 32, values);
                     tmem_wait_ld();
-                    if (valid) {
+                    if (whole) {
+                        slab_bf16x32(smem_aligned + slab + (c / 2) * SLAB_BYTES, lane, c % 2, values);
+                    } else if (valid) {
                         store_bf16_row(dv_row + c * 32, values, 32, 1.0F);
+                    }
+                }
+                if (whole) {
+                    fence_proxy_async_smem();
+                    __syncwarp();
+                    if (lane == 0) {
+                        for (int c = 0; c < 2; ++c) {
+                            tma_store_2d(&p.dv_map, smem_base + slab + c * SLAB_BYTES, head * 128 + c * 64, row0 + warp_row);
+                        }
+                        tma_store_commit();
+                        tma_store_wait_read();
                     }
                 }
             } else {
                 __nv_bfloat16* dk_row = p.dk_nope + (row * p.heads + head) * 128;
+                const int slab = (8 + (warp % 4) * 4) * SLAB_BYTES;
 #pragma unroll
                 for (int c = 0; c < 6; ++c) {
                     uint32_t values[32];
                     tmem_ld_x32(tmem_base + lane_base + TMEM_DK + c * 32, values);
                     tmem_wait_ld();
-                    if (valid) {
+                    if (whole && c < 4) {
+                        slab_bf16x32(smem_aligned + slab + (c / 2) * SLAB_BYTES, lane, c % 2, values);
+                    } else if (whole) {
+                        slab_f32x32(smem_aligned + slab + (c - 2) * SLAB_BYTES, lane, values);
+                    } else if (valid) {
                         if (c < 4) {
                             store_bf16_row(dk_row + c * 32, values, 32, 1.0F);
                         } else {
@@ -942,6 +1015,18 @@ __global__ void __launch_bounds__(THREADS, 1) backward_dkdv_kernel(const __grid_
                                 part[e] = make_uint4(values[4 * e], values[4 * e + 1], values[4 * e + 2], values[4 * e + 3]);
                             }
                         }
+                    }
+                }
+                if (whole) {
+                    fence_proxy_async_smem();
+                    __syncwarp();
+                    if (lane == 0) {
+                        for (int c = 0; c < 2; ++c) {
+                            tma_store_2d(&p.dk_map, smem_base + slab + c * SLAB_BYTES, head * 128 + c * 64, row0 + warp_row);
+                            tma_store_4d(&p.parts_map, smem_base + slab + (2 + c) * SLAB_BYTES, c * 32, head, row0 + warp_row, 0);
+                        }
+                        tma_store_commit();
+                        tma_store_wait_read();
                     }
                 }
             }
@@ -1118,17 +1203,35 @@ __global__ void __launch_bounds__(dqs::STREAM_THREADS, 1) backward_dq_stream_ker
         if (alive) {
             tc_fence_after_sync();
             for (int j = 0; j < (second_used ? 2 : 1); ++j) {
-                const int q_pos = q_start + j * 128 + warp * 32 + lane;
+                const int warp_row = q_start + j * 128 + warp * 32;
+                const int q_pos = warp_row + lane;
+                const bool whole = warp_row + 32 <= length;
+                const int slab = (j * 4 + warp) * 3 * SLAB_BYTES;          // the stages are idle
                 __nv_bfloat16* dq_row = p.dq + (static_cast<size_t>(row0 + q_pos) * p.heads + head) * 192;
 #pragma unroll
                 for (int c = 0; c < 6; ++c) {
                     uint32_t values[32];
                     tmem_ld_x32(tmem_base + lane_base + j * 192 + c * 32, values);
                     tmem_wait_ld();
-                    if (q_pos < length) {
+                    if (whole) {
+                        slab_bf16x32(smem_aligned + slab + (c / 2) * SLAB_BYTES, lane, c % 2, values);
+                    } else if (q_pos < length) {
                         store_bf16_row(dq_row + c * 32, values, 32, 1.0F);
                     }
                 }
+                if (whole) {
+                    fence_proxy_async_smem();
+                    __syncwarp();
+                    if (lane == 0) {
+                        for (int c = 0; c < 3; ++c) {
+                            tma_store_2d(&p.dq_map, smem_base + slab + c * SLAB_BYTES, head * 192 + c * 64, row0 + warp_row);
+                        }
+                        tma_store_commit();
+                    }
+                }
+            }
+            if (lane == 0) {
+                tma_store_wait_read();
             }
         }
     }
@@ -1275,6 +1378,10 @@ void mla_prefill_backward_cuda(__nv_bfloat16* dq, __nv_bfloat16* dk_nope, __nv_b
     params.k_pe_sub = make_bf16_tile_map(k_pe, rows, 64, 64, SUB);
     params.v_sub = make_bf16_tile_map(v, rows, wide, wide, SUB);
     params.do_sub = make_bf16_tile_map(output_gradient, rows, wide, wide, SUB);
+    params.dq_map = make_bf16_store_map(dq, rows, static_cast<std::uint64_t>(heads) * 192, 64, 32);
+    params.dk_map = make_bf16_store_map(dk_nope, rows, wide, 64, 32);
+    params.dv_map = make_bf16_store_map(dv, rows, wide, 64, 32);
+    params.parts_map = make_f32_records_map(parts, 1, rows, heads, 64, 32);
     params.dq = dq;
     params.dk_nope = dk_nope;
     params.dv = dv;
@@ -1329,9 +1436,9 @@ void mla_prefill_backward_cuda(__nv_bfloat16* dq, __nv_bfloat16* dk_nope, __nv_b
         launch_chained(backward_dq_kernel, grid, dim3(THREADS), dqk::SMEM_BYTES, stream, params);
         launch_chained(backward_dkdv_kernel, grid, dim3(THREADS), SMEM_BYTES, stream, params);
     }
-    const std::size_t quads = static_cast<std::size_t>(total_tokens) * 16;
-    const unsigned sum_blocks = static_cast<unsigned>(quads / 256 + 1 < 148 * 8 ? quads / 256 + 1 : 148 * 8);
-    launch_chained(sum_dk_pe_kernel, dim3(sum_blocks), dim3(256), 0, stream, dk_pe, accumulator, reinterpret_cast<const float4*>(parts), static_cast<std::size_t>(total_tokens), heads);
+    const std::size_t sum_blocks = std::min<std::size_t>((static_cast<std::size_t>(total_tokens) + SUM_ROWS - 1) / SUM_ROWS, 148 * 8);
+    launch_chained(sum_dk_pe_kernel, dim3(static_cast<unsigned>(sum_blocks)), dim3(SUM_ROWS * 16 * SUM_QUARTERS), 0, stream, dk_pe, accumulator,
+                   reinterpret_cast<const float4*>(parts), static_cast<std::size_t>(total_tokens), heads);
 }
 
 }  // namespace dscuda
