@@ -58,6 +58,19 @@ const Tensor& tensor(PyObject* object) {
     return t;
 }
 
+void expect_dims(const Tensor& t, int64_t dims) {
+    if (t.dim() != dims) {
+        fail(PyExc_ValueError, "expected a tensor of " + std::to_string(dims) + " dimensions, got " + std::to_string(t.dim()));
+    }
+}
+
+// The same with a given number of dimensions.
+const Tensor& tensor(PyObject* object, int64_t dims) {
+    const Tensor& t = tensor(object);
+    expect_dims(t, dims);
+    return t;
+}
+
 // The same, or null for None.
 const Tensor* optional_tensor(PyObject* object) {
     return object == Py_None ? nullptr : &tensor(object);
@@ -102,6 +115,14 @@ long long integer(PyObject* object) {
     return value;
 }
 
+// Rows of a tensor whose last `columns` elements make one row.
+long long row_count(const Tensor& t, int64_t columns) {
+    if (columns == 0) {
+        fail(PyExc_ValueError, "tensors must not be empty");
+    }
+    return t.numel() / columns;
+}
+
 // Sizes go through the C ABI as int; what does not fit is cut like a ctypes c_int argument, and the entry points
 // refuse sizes that are not positive.
 int extent(const Tensor& t, int64_t dim) {
@@ -120,13 +141,24 @@ Tensor new_like(const Tensor& t) {
     return at::empty(t.sizes(), at::TensorOptions().device(t.device()).dtype(t.scalar_type()));
 }
 
+// The interpreter lock is released for the lifetime of this object; taken back when an exception passes too (data_ptr() of a
+// tensor without storage throws inside the call).
+struct LockReleased {
+    PyThreadState* state = PyEval_SaveThread();
+    LockReleased() = default;
+    LockReleased(const LockReleased&) = delete;
+    LockReleased& operator=(const LockReleased&) = delete;
+    ~LockReleased() { PyEval_RestoreThread(state); }
+};
+
 // Runs one C-ABI call without the interpreter lock; a non-zero status becomes a RuntimeError with the library's message.
 template <class Call>
 void checked(const char* (*last_error)(), Call&& call) {
     int status;
-    Py_BEGIN_ALLOW_THREADS
-    status = call();
-    Py_END_ALLOW_THREADS
+    {
+        const LockReleased released;
+        status = call();
+    }
     if (status != 0) {
         fail(PyExc_RuntimeError, last_error());
     }
@@ -167,7 +199,7 @@ PyObject* tuple(const Tensors&... tensors) {
 DSCUDA_FUNCTION(mla_forward) {
     return guarded([&] {
         expect_arguments(count, 5);
-        const Tensor &query = tensor(args[0]), &query_rope = tensor(args[1]), &latent = tensor(args[2]), &key_rope = tensor(args[3]);
+        const Tensor &query = tensor(args[0], 4), &query_rope = tensor(args[1]), &latent = tensor(args[2]), &key_rope = tensor(args[3]);
         const float scale = number(args[4]);
         const int b = extent(query, 0), t = extent(query, 1), h = extent(query, 2), c = extent(query, 3), r = extent(query_rope, -1);
         Tensor output = new_like(query);
@@ -185,7 +217,7 @@ DSCUDA_FUNCTION(mla_forward) {
 DSCUDA_FUNCTION(mla_backward) {
     return guarded([&] {
         expect_arguments(count, 8);
-        const Tensor &dout = tensor(args[0]), &output = tensor(args[1]), &lse = tensor(args[2]), &query = tensor(args[3]), &query_rope = tensor(args[4]),
+        const Tensor &dout = tensor(args[0]), &output = tensor(args[1]), &lse = tensor(args[2]), &query = tensor(args[3], 4), &query_rope = tensor(args[4]),
                      &latent = tensor(args[5]), &key_rope = tensor(args[6]);
         const float scale = number(args[7]);
         const int b = extent(query, 0), t = extent(query, 1), h = extent(query, 2), c = extent(query, 3), r = extent(query_rope, -1);
@@ -205,7 +237,7 @@ DSCUDA_FUNCTION(mla_backward) {
 DSCUDA_FUNCTION(mla_decode) {
     return guarded([&] {
         expect_arguments(count, 10);
-        const Tensor &query = tensor(args[0]), &cache = tensor(args[1]), &table = tensor(args[2]), &lengths = tensor(args[3]);
+        const Tensor &query = tensor(args[0], 4), &cache = tensor(args[1]), &table = tensor(args[2]), &lengths = tensor(args[3]);
         const float scale = number(args[4]);
         const int splits = static_cast<int>(integer(args[5]));
         const Tensor* workspace_given = optional_tensor(args[6]);
@@ -242,7 +274,7 @@ DSCUDA_FUNCTION(mla_decode) {
 PyObject* append(PyObject* const* args, Py_ssize_t count, bool fp8) {
     return guarded([&] {
         expect_arguments(count, 6);
-        const Tensor &cache = tensor(args[0]), &latent = tensor(args[1]), &key_rope = tensor(args[2]), &table = tensor(args[3]);
+        const Tensor &cache = tensor(args[0]), &latent = tensor(args[1], 3), &key_rope = tensor(args[2]), &table = tensor(args[3]);
         const Tensor *start = optional_tensor(args[4]), *counts = optional_tensor(args[5]);
         if (fp8 && (cache.scalar_type() != at::kByte || cache.size(-1) != FP8_ROW_BYTES)) {
             fail(PyExc_ValueError, "the FP8 cache is a uint8 tensor [blocks, page, 656]");
@@ -300,8 +332,7 @@ DSCUDA_FUNCTION(rope_apply) {
         }
         const int heads = q_pe != nullptr ? extent(*q_pe, -2) : 1;
         const int width = extent(*anchor, -1);
-        const long long columns = anchor->size(-2) * anchor->size(-1);
-        const long long rows = columns != 0 ? anchor->numel() / columns : 0;
+        const long long rows = row_count(*anchor, anchor->size(-2) * anchor->size(-1));
         if (positions == nullptr && anchor->dim() != 4) {
             fail(PyExc_ValueError, "packed tensors need explicit positions");
         }
@@ -324,7 +355,7 @@ DSCUDA_FUNCTION(up_project) {
         at::DimVector sizes(latent.sizes().begin(), latent.sizes().end() - 1);
         sizes.push_back(heads);
         sizes.push_back(128);
-        const long long rows = latent.numel() / latent.size(-1);
+        const long long rows = row_count(latent, latent.size(-1));
         Tensor k_nope = new_tensor(sizes, latent, at::kBFloat16), v = new_tensor(sizes, latent, at::kBFloat16);
         void* stream = current_stream();
         checked(dscuda_mla_last_error,
@@ -340,7 +371,7 @@ PyObject* per_head_projection(PyObject* const* args, Py_ssize_t count, int64_t c
         expect_arguments(count, 2);
         const Tensor &x = tensor(args[0]), &weight = tensor(args[1]);
         const int heads = extent(x, -2);
-        const long long rows = x.numel() / (x.size(-2) * x.size(-1));
+        const long long rows = row_count(x, x.size(-2) * x.size(-1));
         at::DimVector sizes(x.sizes().begin(), x.sizes().end() - 1);
         sizes.push_back(columns);
         Tensor output = new_tensor(sizes, x, at::kBFloat16);
@@ -365,12 +396,18 @@ struct PrefillShape {
 
 PrefillShape prefill_shape(const Tensor& q_nope, const Tensor* cu_seqlens, PyObject* max_seqlen) {
     if (cu_seqlens == nullptr) {
+        expect_dims(q_nope, 4);
         return {extent(q_nope, 0), extent(q_nope, 1), static_cast<int>(q_nope.size(0) * q_nope.size(1)), extent(q_nope, 2)};
     }
     if (max_seqlen == Py_None) {
         fail(PyExc_ValueError, "packed layout needs max_seqlen (an upper bound on the longest sequence)");
     }
-    return {static_cast<int>(cu_seqlens->numel() - 1), static_cast<int>(integer(max_seqlen)), extent(q_nope, 0), extent(q_nope, 1)};
+    THPObjectPtr longest(PyNumber_Long(max_seqlen));      // int(max_seqlen): a float or a one-element tensor will do
+    if (!longest) {
+        throw python_error();
+    }
+    expect_dims(q_nope, 3);
+    return {static_cast<int>(cu_seqlens->numel() - 1), static_cast<int>(integer(longest.get())), extent(q_nope, 0), extent(q_nope, 1)};
 }
 
 // q_nope, q_pe, k_nope, k_pe, v, scale, cu_seqlens, max_seqlen, output, lse -> output, lse
@@ -454,7 +491,7 @@ DSCUDA_FUNCTION(prefill_backward) {
 DSCUDA_FUNCTION(flash_forward) {
     return guarded([&] {
         expect_arguments(count, 4);
-        const Tensor &query = tensor(args[0]), &key = tensor(args[1]), &value = tensor(args[2]);
+        const Tensor &query = tensor(args[0], 4), &key = tensor(args[1]), &value = tensor(args[2]);
         const float scale = number(args[3]);
         const int b = extent(query, 0), t = extent(query, 1), hq = extent(query, 2), d = extent(query, 3), hkv = extent(key, 2);
         Tensor output = new_like(query);
