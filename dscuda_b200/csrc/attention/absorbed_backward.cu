@@ -6,33 +6,25 @@
 // (576 score columns, 512 value columns), so the work is split the way the
 // reference splits it (kernels/attention/mla/sm89.cu:295 query side, :356 key
 // side): one kernel owns the key-side gradients, one owns the query-side
-// gradients, and each recomputes P from the saved LSE.  Both are tcgen05 kernels
-// and share one tile shape: a score tile is S^T = K Q^T with 128 keys on the
-// tensor-memory lanes and 64 (token, head) rows on the columns, so that one
-// thread owns one key, the per-row constants (LSE, delta, token index) are read
-// from shared memory, and P^T / dS^T come out in the form the gradient products
-// want.  Wide operands stream through shared memory in 64-column chunks.
+// gradients, and each recomputes P from the saved LSE.  Both are tcgen05 kernels whose score tiles are S^T = K Q^T, keys on
+// the tensor-memory lanes and (token, head) rows on the columns, so that one thread owns one key and the per-row constants
+// (LSE, delta, token index) are read from shared memory.
 //
 // One call launches, on the caller's stream:
 //   1. absorbed_delta_kernel: delta[row] = sum_c dO[row,c] O[row,c], kept in the
 //      first four bytes of each dquery_rope row (an output the last kernel
 //      overwrites, so no scratch is needed);
-//   2. absorbed_backward_key_kernel: CTA = (128-key tile, one 256-column half of
-//      dlatent, one part of the rows).  The key tile (9 chunks, 144 KB) stays in
-//      shared memory; the 64-row tiles at or after the diagonal stream by: the 17
-//      chunks of query_latent | query_rope | dO give S^T and dP^T = latent dO^T, and
-//      the 9 chunks this half needs again stay in the ring until after the
-//      softmax, as the B operands of dlatent += dS^T query_latent + P^T dO and
-//      dkey_rope += dS^T query_rope (P^T and dS^T are bf16 A operands in tensor
-//      memory).  Single writer per output element, no atomics;
+//   2. absorbed_backward_key_kernel: cluster of two CTAs = (128-key tile, one part of the rows).  The keys stay in shared
+//      memory; the 96-row tiles at or after the diagonal stream by and stay there from the score products to the gradient
+//      products dlatent += dS^T query_latent + P^T dO and dkey_rope += dS^T query_rope.  Single writer per output element,
+//      no atomics; with several parts absorbed_backward_reduce_kernel adds them in order;
 //   3. absorbed_backward_query_kernel: CTA = 64 (token, head) rows, resident as the
 //      B operands query_latent | query_rope | dO (136 KB); every 128-key tile up
 //      to the diagonal streams by twice: for S^T / dP^T, and again as the
 //      MN-major A operand of dQ^T += K^T dS^T (output columns on the lanes, rows on
 //      the columns; dS^T goes through shared memory as the B operand).
 //
-// Warps 0-7: softmax (thread = key x 32 of the 64 rows); warp 8: MMA issue (whole
-// warp, one elected lane executes); warp 9: TMA loads.  Every wait is bounded.
+// Warps 0-7: softmax; warp 8: MMA issue (whole warp, one elected lane executes); warp 9: TMA loads.  Every wait is bounded.
 #include "mla.h"
 #include "cuda_common.h"
 #include "attention_internal.h"
@@ -73,6 +65,16 @@ struct AbsorbedBackwardParams {
     CUtensorMap d_out;      // [B*T*H, 512] box 64 x 64
     CUtensorMap k_lat;      // [B*T, 512]   box 128 x 64
     CUtensorMap k_rope;     // [B*T, 64]    box 128 x 64
+    // key side; batch entries apart, so rows and keys past the end of one read as zero
+    CUtensorMap key_lat8;   // kv_latent, box 64 keys x 8 chunks
+    CUtensorMap key_rope1;  // key_rope, box 64 keys
+    CUtensorMap row_q8;     // query_latent, box 48 rows x 8 chunks
+    CUtensorMap row_q2;     // ... x 2 chunks
+    CUtensorMap row_do8;    // dO likewise
+    CUtensorMap row_do2;
+    CUtensorMap row_rope;   // query_rope, box 48 rows
+    CUtensorMap dlatent_out;    // stores of 32 keys: 64 bf16 columns of dlatent, 32 fp32 columns of a partial sum
+    CUtensorMap partials;
     __nv_bfloat16* dq_lat;  // [B,T,H,512]
     __nv_bfloat16* dq_rope; // [B,T,H,64]; the first float of each row holds delta until the query kernel overwrites it
     __nv_bfloat16* dlatent; // [B,T,512]
@@ -81,21 +83,21 @@ struct AbsorbedBackwardParams {
     int batch;
     int sequence;
     int heads;
-    int key_chunk;          // key side: at most this many 64-row tiles per CTA
+    int key_chunk;          // key side: at most this many 96-row tiles per cluster
     int key_direct;         // key side: 1 when every key tile has a single part (results go straight to the outputs)
     float scale;
     float scale_log2;
 };
 
-// Key side work split.  Key tile kt meets the 64-row tiles from floor(kt*128*H/64) to the end of
-// the sequence; that range is cut into ceil(count / key_chunk) parts of equal size, one CTA each,
-// so that the first key tiles (which meet every row) do not set the kernel's duration.  With more
-// than one part the CTAs write fp32 partial sums, part p of key row (b, key) at
-// scratch[((p*B + b)*T + key)*576 ..], and absorbed_backward_reduce_kernel adds them in part
-// order.  The scratch is the dquery_latent output, which the query-side kernel overwrites last.
+// Key side work split.  Key tile kt meets the rows of its own first token (row kt*128*H) and all later ones, in tiles of 96;
+// they are cut into ceil(count / key_chunk) parts of equal size, one cluster each, so that the first key tiles (which meet
+// every row) do not set the kernel's duration.  With more than one part the clusters write fp32 partial sums, part p of key
+// row (b, key) at scratch[((p*B + b)*T + key)*576 ..], and absorbed_backward_reduce_kernel adds them in part order.  The
+// scratch is the dquery_latent output, which the query-side kernel overwrites last.
+constexpr int KEY_SIDE_ROWS = 96;
+
 __device__ __forceinline__ int key_tile_row_tiles(const AbsorbedBackwardParams& p, int key_tile) {
-    const int rows_per_sequence = p.sequence * p.heads;
-    return (rows_per_sequence + 63) / 64 - static_cast<int>((static_cast<long long>(key_tile) * 128 * p.heads) / 64);
+    return (p.sequence * p.heads - key_tile * KEYS * p.heads + KEY_SIDE_ROWS - 1) / KEY_SIDE_ROWS;
 }
 
 __device__ __forceinline__ int key_tile_parts(const AbsorbedBackwardParams& p, int key_tile) {
@@ -233,57 +235,103 @@ __global__ void __launch_bounds__(256) absorbed_delta_kernel(__nv_bfloat16* dq_r
 }
 
 // ---------------------------------------------------------------------------
-// Key side.  Tensor memory: dlatent half 0..255, dkey_rope 256..319, S^T 320..383 (P^T overwrites
-// it as bf16), dP^T 384..447 (dS^T likewise).  Shared memory: the key tile (9 x 16 KB), a ring of
-// five 16 KB units, constants.  A unit is one TMA transaction of one or two 8 KB row chunks.
-// Per row tile, nine units in this order: the other half's two query_latent pairs and two dO
-// pairs, then this half's two query_latent pairs, query_rope, and this half's two dO pairs.  All
-// nine feed S^T / dP^T; the last five (exactly the ring) are not released after that: they stay
-// where they are and serve as the B operands of the gradient products after the softmax, so a
-// row tile is streamed once (136 KB), and they are released in the order they were loaded.
+// Key side.  A cluster of two CTAs takes 128 keys and a part of the rows; CTA r owns keys 64r..64r+63 of the tile (the A
+// rows of every product, tcgen05.mma.cta_group::2 with M = 128) and supplies half of each B operand.  Per 96-row tile:
+//
+//   S^T = K Q^T, dP^T = latent dO^T  (N = 96, CTA r supplies its own 48 rows of the tile, all columns);
+//   dlatent += dS^T Q + P^T dO       (N = 256 twice; K = 96 rows, CTA r supplies columns 128r..128r+127 of each half);
+//   dkey_rope += dS^T Q_rope         (N = 128: both CTAs supply all 64 columns, so the result is there twice).
+//
+// The eight 64-column chunks of a CTA's own 48 rows sit in slots 0..7.  Chunks {2r, 2r+1, 4+2r, 4+2r+1} are in place as
+// columns of the gradient products; the other four slots are refilled with the other CTA's rows of those columns as soon as
+// the score MMAs have read them (the same scheme as in absorbed_attention.cu), and the rotary columns of all 96 rows are
+// loaded once more into a place of their own.  So the scores are computed once per (key, row) pair and a CTA reads 168 KB
+// from L2 for 64 x 96 pairs.
+//
+// What bounds it: shared memory.  The resident keys (72 KB), P and dS (32 KB) and one tile of rows (114 KB) fill it, so the
+// chain scores -> softmax -> gradients of a tile is overlapped only by the loads of the next one: query_latent is loaded
+// again while P^T dO runs.  96 rows and not 128 because 128 do not fit.  One CTA per (128 keys, half of dlatent), which this
+// replaces, computed the scores twice, at the N = 64 rate: 1305 us at B=4 T=2048 H=16 against
+// 592 us now, 46 against 11 us at B=2 T=33 H=32 (where a part also had at least 1024 rows).
+//
+// Tensor memory: dlatent 2 x 128 columns (lanes 0-63: columns 256a + 0..127, lanes 64-127: 256a + 128..255 of the same 64
+// keys), dkey_rope 64, S^T 48 (lanes 64-127: rows 48..95), dP^T 48.
+// Warps 0-7: softmax (thread = key x 24 rows) and results; 8: MMA issue in the leader, relay of "loaded" events in the other
+// CTA; 9: TMA loads; 10: the rows' constants.
 // ---------------------------------------------------------------------------
 namespace ks {
-constexpr int RING_SLOTS = 5;
-constexpr int SLOT_BYTES = 2 * ROW_CHUNK;
-constexpr int RESIDENT_BYTES = CHUNKS * KEY_CHUNK;
-constexpr int SMEM_BYTES = RESIDENT_BYTES + RING_SLOTS * SLOT_BYTES + MISC_BYTES + 1024;
-constexpr int UNITS_PER_TILE = 9;
-constexpr int RETAINED_FROM = 4;          // units 4..8 of a tile are kept for the gradient products
+constexpr int TILE_ROWS = KEY_SIDE_ROWS;
+constexpr int HALF_ROWS = 48;                       // rows a CTA supplies
+constexpr int SHARE_ROWS = 24;                      // rows of a softmax thread
+constexpr int CTA_KEYS = 64;
+constexpr int KEY_SLOT = CTA_KEYS * 128;            // 8 KB: [64 keys x 64 bf16]
+constexpr int ROW_SLOT = HALF_ROWS * 128;           // 6 KB: [48 rows x 64 bf16]
+constexpr int K_BYTES = CHUNKS * KEY_SLOT;
+constexpr int P_OFFSET = K_BYTES;                   // P^T, then dS^T: [64 keys x 96 rows] as two 64-row chunks
+constexpr int DS_OFFSET = P_OFFSET + 2 * KEY_SLOT;
+constexpr int Q_OFFSET = DS_OFFSET + 2 * KEY_SLOT;
+constexpr int DO_OFFSET = Q_OFFSET + LATENT_CHUNKS * ROW_SLOT;
+constexpr int ROPE_OFFSET = DO_OFFSET + LATENT_CHUNKS * ROW_SLOT;       // own rows, for the scores
+constexpr int ROPE_ALL_OFFSET = ROPE_OFFSET + ROW_SLOT;                 // all 96 rows, for dkey_rope
+constexpr int MISC_OFFSET = ROPE_ALL_OFFSET + 2 * ROW_SLOT;
+constexpr int SMEM_BYTES = MISC_OFFSET + 3072;
+constexpr int KEY_THREADS = 352;
+constexpr int CONSTANTS_WARP = 10;
+constexpr int SLAB_BYTES = 32 * 128;
 constexpr uint32_t TMEM_DLAT = 0;
 constexpr uint32_t TMEM_DROPE = 256;
-constexpr uint32_t TMEM_X0 = 320;
-constexpr uint32_t TMEM_X1 = 384;
+constexpr uint32_t TMEM_S = 320;
+constexpr uint32_t TMEM_DP = 368;
 static_assert(SMEM_BYTES <= 232448, "key-side shared memory");
+static_assert(8 * 5 * SLAB_BYTES <= MISC_OFFSET, "result slabs lie in the operands' memory");
+
+struct Rows {
+    alignas(16) float lse2[TILE_ROWS];     // LSE * log2 e
+    alignas(16) float delta[TILE_ROWS];
+    alignas(16) int token[TILE_ROWS];      // -1 for rows past the end of the sequence
+};
 
 struct Shared {
-    uint64_t resident_full;
-    uint64_t unit_full[RING_SLOTS];
-    uint64_t unit_empty[RING_SLOTS];
-    uint64_t rows_ready[2];
-    uint64_t s_ready;           // tensor core -> softmax: S^T and dP^T of the tile are complete
-    uint64_t p_ready;           // 256 softmax threads: P^T and dS^T are stored
-    uint64_t final_full;
+    Rows rows[2];
+    // completed by TMA transactions of this CTA, one phase per tile
+    uint64_t k_full;
+    uint64_t q_full;            // own rows: query_latent and the rotary chunk
+    uint64_t do_full;           // own rows: dO
+    uint64_t q_refilled;        // the other CTA's rows, and the rotary columns of all rows
+    uint64_t do_refilled;
+    // leader only: the same events of the other CTA, forwarded by its relay (one arrival)
+    uint64_t peer_k_full;
+    uint64_t peer_q_full;
+    uint64_t peer_do_full;
+    uint64_t peer_q_refilled;
+    uint64_t peer_do_refilled;
+    // completed by tcgen05.commit of the leader
+    uint64_t q_refill_free;     // S has read the four slots only it needs
+    uint64_t do_refill_free;
+    uint64_t s_full;
+    uint64_t dp_full;
+    uint64_t q_free;            // dS^T Q has read everything of query_latent and query_rope
+    uint64_t do_free;           // P^T dO too; P, dS and the accumulators are quiescent
+    // leader only: one arrival per softmax warp of either CTA, P^T and dS^T are stored
+    uint64_t p_full;
+    uint64_t rows_ready[2];     // the constants of a tile, by tile parity
+    uint64_t rows_done[2];      // eight softmax warps have read them
     uint32_t tmem_base;
     int abort_flag;
-    int masked[2];
-    RowConstants rows[2];
 };
-static_assert(sizeof(Shared) <= MISC_BYTES, "key-side barrier block too large");
+static_assert(sizeof(Shared) <= SMEM_BYTES - MISC_OFFSET, "key-side barrier block too large");
 }  // namespace ks
 
-__global__ void __launch_bounds__(THREADS, 1) absorbed_backward_key_kernel(const __grid_constant__ AbsorbedBackwardParams p) {
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ks::KEY_THREADS, 1) absorbed_backward_key_kernel(const __grid_constant__ AbsorbedBackwardParams p) {
     using namespace ks;
     extern __shared__ uint8_t smem_raw[];
-    if (*reinterpret_cast<volatile int*>(&absorbed_backward_status) == STATUS_WAIT_TIMEOUT) {
-        grid_dependency_wait();
-        return;
-    }
+    // No early exit on a status left by an earlier launch: both CTAs have to take the same path to the cluster barriers.
     const int warp = threadIdx.x / 32;
     const int lane = threadIdx.x % 32;
+    const uint32_t rank = cluster_cta_rank();
     const int b = blockIdx.z;
-    const int half = blockIdx.y;                         // which 256 columns of dlatent
-    // blockIdx.x counts (key tile, part) pairs, key tile 0 first
-    int key_tile = 0, part = static_cast<int>(blockIdx.x), parts = key_tile_parts(p, 0);
+    // blockIdx.x / 2 counts (key tile, part) pairs, key tile 0 first
+    int key_tile = 0, part = static_cast<int>(blockIdx.x >> 1), parts = key_tile_parts(p, 0);
     while (part >= parts) {
         part -= parts;
         ++key_tile;
@@ -292,252 +340,379 @@ __global__ void __launch_bounds__(THREADS, 1) absorbed_backward_key_kernel(const
     const int key_start = key_tile * KEYS;
     const int rows_per_sequence = p.sequence * p.heads;
     const int tiles_of_key_tile = key_tile_row_tiles(p, key_tile);
-    const int first_tile = (rows_per_sequence + ROWS - 1) / ROWS - tiles_of_key_tile +
-                           static_cast<int>(static_cast<long long>(part) * tiles_of_key_tile / parts);
-    const int tile_count = static_cast<int>(static_cast<long long>(part + 1) * tiles_of_key_tile / parts) -
-                           static_cast<int>(static_cast<long long>(part) * tiles_of_key_tile / parts);
+    const int first_tile = static_cast<int>(static_cast<long long>(part) * tiles_of_key_tile / parts);
+    const int tile_count = static_cast<int>(static_cast<long long>(part + 1) * tiles_of_key_tile / parts) - first_tile;
+    const int first_row = key_start * p.heads + first_tile * TILE_ROWS;        // of the batch entry
 
-    const uint32_t smem_base = (smem_u32(smem_raw) + 1023U) & ~1023U;
-    uint8_t* smem_aligned = smem_raw + (smem_base - smem_u32(smem_raw));
-    const uint32_t k_smem = smem_base;
-    const uint32_t ring = smem_base + RESIDENT_BYTES;
-    Shared* sh = reinterpret_cast<Shared*>(smem_aligned + RESIDENT_BYTES + RING_SLOTS * SLOT_BYTES);
+    const uint32_t smem_base = smem_u32(smem_raw);
+    Shared* sh = reinterpret_cast<Shared*>(smem_raw + MISC_OFFSET);
     volatile int* abort_flag = &sh->abort_flag;
+    if ((smem_base & 1023U) != 0U) {            // a property of the kernel image: the same in both CTAs
+        grid_dependency_wait();
+        if (threadIdx.x == 0) {
+            atomicExch(&absorbed_backward_status, STATUS_SMEM_MISALIGNED);
+        }
+        return;
+    }
 
     if (threadIdx.x == 0) {
-        mbar_init(smem_u32(&sh->resident_full), 1);
-        for (int i = 0; i < RING_SLOTS; ++i) {
-            mbar_init(smem_u32(&sh->unit_full[i]), 1);
-            mbar_init(smem_u32(&sh->unit_empty[i]), 1);
+        for (uint64_t* bar = &sh->k_full; bar <= &sh->do_free; ++bar) {
+            mbar_init(smem_u32(bar), 1);
         }
-        mbar_init(smem_u32(&sh->rows_ready[0]), 1);
-        mbar_init(smem_u32(&sh->rows_ready[1]), 1);
-        mbar_init(smem_u32(&sh->s_ready), 1);
-        mbar_init(smem_u32(&sh->p_ready), 256);
-        mbar_init(smem_u32(&sh->final_full), 1);
+        mbar_init(smem_u32(&sh->p_full), 16);
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(smem_u32(&sh->rows_ready[i]), 1);
+            mbar_init(smem_u32(&sh->rows_done[i]), 8);
+        }
         sh->abort_flag = 0;
         mbar_init_fence();
     }
     if (warp == MMA_WARP) {
-        tmem_alloc(smem_u32(&sh->tmem_base), TMEM_COLUMNS);
-        tmem_relinquish();
+        tmem_alloc_pair(smem_u32(&sh->tmem_base), TMEM_COLUMNS);
+        tmem_relinquish_pair();
     }
     if (warp == LOAD_WARP && lane == 0) {
-        tma_prefetch_descriptor(&p.q_lat);
-        tma_prefetch_descriptor(&p.q_rope);
-        tma_prefetch_descriptor(&p.d_out);
-        tma_prefetch_descriptor(&p.k_lat);
-        tma_prefetch_descriptor(&p.k_rope);
+        tma_prefetch_descriptor(&p.key_lat8);
+        tma_prefetch_descriptor(&p.key_rope1);
+        tma_prefetch_descriptor(&p.row_q8);
+        tma_prefetch_descriptor(&p.row_q2);
+        tma_prefetch_descriptor(&p.row_do8);
+        tma_prefetch_descriptor(&p.row_do2);
+        tma_prefetch_descriptor(&p.row_rope);
     }
     tc_fence_before_sync();
     __syncthreads();
+    cluster_sync_all();
     tc_fence_after_sync();
     grid_dependency_wait();
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&sh->tmem_base);
+    auto wait = [&](uint64_t& bar, int phase) { return mbar_wait(smem_u32(&bar), phase & 1, abort_flag, &absorbed_backward_status); };
 
     if (warp == LOAD_WARP) {
         // =================== TMA producer ===================================
         if (lane == 0) {
-            const uint32_t bar = smem_u32(&sh->resident_full);
-            mbar_arrive_expect_tx(bar, RESIDENT_BYTES);
-            const int y = b * p.sequence + key_start;
-            for (int c = 0; c < LATENT_CHUNKS; ++c) {
-                tma_load_2d(k_smem + c * KEY_CHUNK, &p.k_lat, bar, c * 64, y);
+            const int own = static_cast<int>(rank) * HALF_ROWS, other = HALF_ROWS - own;
+            const int own_chunk = 2 * static_cast<int>(rank), other_slot = 2 - own_chunk;
+            uint32_t bar = smem_u32(&sh->k_full);
+            mbar_arrive_expect_tx(bar, K_BYTES);
+            tma_load_4d(smem_base, &p.key_lat8, bar, 0, key_start + static_cast<int>(rank) * CTA_KEYS, 0, b);
+            tma_load_4d(smem_base + LATENT_CHUNKS * KEY_SLOT, &p.key_rope1, bar, 0, key_start + static_cast<int>(rank) * CTA_KEYS, 0, b);
+            for (int t = 0; t < tile_count; ++t) {
+                const int row0 = first_row + t * TILE_ROWS;
+                if (t > 0 && !wait(sh->q_free, t - 1)) {
+                    break;
+                }
+                bar = smem_u32(&sh->q_full);
+                mbar_arrive_expect_tx(bar, CHUNKS * ROW_SLOT);
+                tma_load_4d(smem_base + ROPE_OFFSET, &p.row_rope, bar, 0, row0 + own, 0, b);
+                tma_load_4d(smem_base + Q_OFFSET, &p.row_q8, bar, 0, row0 + own, 0, b);
+                if (t > 0 && !wait(sh->do_free, t - 1)) {
+                    break;
+                }
+                bar = smem_u32(&sh->do_full);
+                mbar_arrive_expect_tx(bar, LATENT_CHUNKS * ROW_SLOT);
+                tma_load_4d(smem_base + DO_OFFSET, &p.row_do8, bar, 0, row0 + own, 0, b);
+                if (!wait(sh->q_refill_free, t)) {
+                    break;
+                }
+                bar = smem_u32(&sh->q_refilled);
+                mbar_arrive_expect_tx(bar, 6 * ROW_SLOT);
+                for (int a = 0; a < 2; ++a) {
+                    tma_load_4d(smem_base + Q_OFFSET + (4 * a + other_slot) * ROW_SLOT, &p.row_q2, bar, 0, row0 + other, 4 * a + own_chunk, b);
+                    tma_load_4d(smem_base + ROPE_ALL_OFFSET + a * ROW_SLOT, &p.row_rope, bar, 0, row0 + a * HALF_ROWS, 0, b);
+                }
+                if (!wait(sh->do_refill_free, t)) {
+                    break;
+                }
+                bar = smem_u32(&sh->do_refilled);
+                mbar_arrive_expect_tx(bar, 4 * ROW_SLOT);
+                for (int a = 0; a < 2; ++a) {
+                    tma_load_4d(smem_base + DO_OFFSET + (4 * a + other_slot) * ROW_SLOT, &p.row_do2, bar, 0, row0 + other, 4 * a + own_chunk, b);
+                }
             }
-            tma_load_2d(k_smem + LATENT_CHUNKS * KEY_CHUNK, &p.k_rope, bar, 0, y);
         }
-        bool alive = true;
-        int unit = 0;                                    // units issued so far
-        for (int t = 0; t < tile_count && alive; ++t) {
-            const int row0 = (first_tile + t) * ROWS;
-            // The constants of tile t-2 (same buffer) were last read before P^T(t-2) was stored,
-            // and the ring (5 units) cannot run a whole tile (14 units) ahead of the tensor core.
-            fill_row_constants(p, sh->rows[t & 1], b, row0, lane);
-            if (lane == 0) {
-                sh->masked[t & 1] = (row0 / p.heads < key_start + KEYS - 1 || row0 + ROWS > rows_per_sequence) ? 1 : 0;
+    } else if (warp == CONSTANTS_WARP) {
+        for (int t = 0; t < tile_count; ++t) {
+            if (t >= 2 && !__all_sync(0xffffffffU, wait(sh->rows_done[t & 1], (t >> 1) - 1))) {
+                break;
+            }
+            Rows& rows = sh->rows[t & 1];
+#pragma unroll
+            for (int e = 0; e < TILE_ROWS / 32; ++e) {
+                const int n = e * 32 + lane;
+                const int row = first_row + t * TILE_ROWS + n;
+                float lse_value = 0.0F, delta_value = 0.0F;
+                int token = -1;
+                if (row < rows_per_sequence) {
+                    token = row / p.heads;
+                    const int head = row - token * p.heads;
+                    lse_value = p.lse[(static_cast<size_t>(b) * p.heads + head) * p.sequence + token] * LOG2E;
+                    delta_value = stored_delta(p, static_cast<size_t>(b) * rows_per_sequence + row);
+                }
+                rows.lse2[n] = lse_value;
+                rows.delta[n] = delta_value;
+                rows.token[n] = token;
             }
             __syncwarp();
             if (lane == 0) {
                 mbar_arrive(smem_u32(&sh->rows_ready[t & 1]));
-                const int y = b * rows_per_sequence + row0;
-                for (int u = 0; u < UNITS_PER_TILE && alive; ++u, ++unit) {
-                    const int slot = unit % RING_SLOTS;
-                    if (unit >= RING_SLOTS) {
-                        alive = mbar_wait(smem_u32(&sh->unit_empty[slot]), (unit / RING_SLOTS - 1) & 1, abort_flag, &absorbed_backward_status);
-                        if (!alive) {
-                            break;
-                        }
-                    }
-                    const uint32_t full = smem_u32(&sh->unit_full[slot]);
-                    const uint32_t dst = ring + slot * SLOT_BYTES;
-                    // which tensor and which chunk pair this unit carries
-                    const CUtensorMap* map;
-                    int chunk;                           // first chunk; -1: the single rotary chunk
-                    if (u < 2) {
-                        map = &p.q_lat, chunk = 4 * (1 - half) + 2 * u;
-                    } else if (u < 4) {
-                        map = &p.d_out, chunk = 4 * (1 - half) + 2 * (u - 2);
-                    } else if (u < 6) {
-                        map = &p.q_lat, chunk = 4 * half + 2 * (u - 4);
-                    } else if (u == 6) {
-                        map = &p.q_rope, chunk = -1;
-                    } else {
-                        map = &p.d_out, chunk = 4 * half + 2 * (u - 7);
-                    }
-                    if (chunk < 0) {
-                        mbar_arrive_expect_tx(full, ROW_CHUNK);
-                        tma_load_2d(dst, map, full, 0, y);
-                    } else {
-                        mbar_arrive_expect_tx(full, 2 * ROW_CHUNK);
-                        tma_load_2d(dst, map, full, chunk * 64, y);
-                        tma_load_2d(dst + ROW_CHUNK, map, full, (chunk + 1) * 64, y);
+            }
+        }
+    } else if (warp == MMA_WARP && rank != 0) {
+        // =================== relay: this CTA's "loaded" events -> the leader =========
+        if (lane == 0) {
+            bool alive = wait(sh->k_full, 0);
+            if (alive) {
+                mbar_arrive_remote(map_to_cta(smem_u32(&sh->peer_k_full), 0));
+            }
+            for (int t = 0; t < tile_count && alive; ++t) {
+                // in the order in which they are loaded
+                uint64_t* const mine[4] = {&sh->q_full, &sh->do_full, &sh->q_refilled, &sh->do_refilled};
+                uint64_t* const leaders[4] = {&sh->peer_q_full, &sh->peer_do_full, &sh->peer_q_refilled, &sh->peer_do_refilled};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    alive = alive && wait(*mine[i], t);
+                    if (alive) {
+                        mbar_arrive_remote(map_to_cta(smem_u32(leaders[i]), 0));
                     }
                 }
             }
-            alive = __shfl_sync(0xffffffffU, alive ? 1 : 0, 0) != 0;
-            unit = __shfl_sync(0xffffffffU, unit, 0);
         }
     } else if (warp == MMA_WARP) {
-        // =================== MMA issuer (whole warp, elected lane executes) ==
+        // =================== MMA issuer (leader CTA; whole warp, elected lane executes) ==
         const uint32_t leader = elect_one();
-        constexpr uint32_t IDESC_SCORE = make_idesc_bf16(KEYS, ROWS, false, false);
-        constexpr uint32_t IDESC_GRAD = make_idesc_bf16(KEYS, 128, false, true);      // B = two row chunks side by side, MN-major
-        constexpr uint32_t IDESC_ROPE = make_idesc_bf16(KEYS, 64, false, true);
-        bool alive = __all_sync(0xffffffffU, mbar_wait(smem_u32(&sh->resident_full), 0, abort_flag, &absorbed_backward_status));
+        constexpr uint32_t IDESC_SCORE = make_idesc_bf16(KEYS, TILE_ROWS, false, false);
+        constexpr uint32_t IDESC_GRAD = make_idesc_bf16(KEYS, 256, false, true);
+        constexpr uint32_t IDESC_ROPE = make_idesc_bf16(KEYS, 128, false, true);
+        constexpr uint32_t HI = smem_desc_hi(1024);
+        const uint32_t k_lo = smem_desc_lo(smem_base, 16);
+        const uint32_t rope_lo = smem_desc_lo(smem_base + ROPE_OFFSET, 16);
+        const uint32_t p_lo = smem_desc_lo(smem_base + P_OFFSET, 16);
+        const uint32_t ds_lo = smem_desc_lo(smem_base + DS_OFFSET, 16);
+        const uint32_t rope_all_lo = smem_desc_lo(smem_base + ROPE_ALL_OFFSET, ROW_SLOT);
+        auto both = [&](uint64_t* bar) {        // one commit for this CTA's barrier, one for the other CTA's
+            commit_pair(smem_u32(bar), leader);
+            commit_pair(map_to_cta(smem_u32(bar), 1), leader);
+        };
+        // K (chunks of all columns) times the own rows in slots at `operand`; slots {2,3,6,7} (refilled in the leader) first,
+        // then {0,1,4,5} (refilled in the other CTA)
+        auto issue_scores = [&](uint32_t acc, uint32_t operand, bool fresh, uint64_t* refill_free) {
+            const uint32_t row_lo = smem_desc_lo(operand, 16);
+#pragma unroll
+            for (int group = 0; group < 2; ++group) {
+#pragma unroll
+                for (int n = 0; n < 4; ++n) {
+                    const int c = (group == 0 ? 2 : 0) + (n & 1) + (n >> 1) * 4;
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        mma_pair_ss_split(acc, k_lo + c * (KEY_SLOT >> 4) + 2 * k, HI, row_lo + c * (ROW_SLOT >> 4) + 2 * k, HI, IDESC_SCORE,
+                                          (fresh && group == 0 && n == 0 && k == 0) ? 0U : 1U, leader);
+                    }
+                }
+                commit_pair(group == 0 ? smem_u32(refill_free) : map_to_cta(smem_u32(refill_free), 1), leader);
+            }
+        };
+        // dlatent += A (P^T or dS^T at a_lo) times the columns in slots at `operand`: rows 48g.. of half a in slots 4a + 2g, + 1
+        auto issue_gradients = [&](uint32_t a_lo, uint32_t operand, bool fresh) {
+            const uint32_t column_lo = smem_desc_lo(operand, ROW_SLOT);
+#pragma unroll
+            for (int a = 0; a < 2; ++a) {
+#pragma unroll
+                for (int kk = 0; kk < 6; ++kk) {
+                    mma_pair_ss_split(tmem_base + TMEM_DLAT + a * 128, a_lo + (kk >> 2) * (KEY_SLOT >> 4) + 2 * (kk & 3), HI,
+                                      column_lo + (4 * a + 2 * (kk / 3)) * (ROW_SLOT >> 4) + (kk % 3) * (2048 >> 4), HI, IDESC_GRAD,
+                                      (fresh && kk == 0) ? 0U : 1U, leader);
+                }
+            }
+        };
+        auto wait_both = [&](uint64_t& mine, uint64_t& others, int phase) {
+            const bool alive = __all_sync(0xffffffffU, wait(mine, phase) && wait(others, phase));
+            tc_fence_after_sync();
+            return alive;
+        };
+        bool alive = wait_both(sh->k_full, sh->peer_k_full, 0);
         for (int t = 0; t < tile_count && alive; ++t) {
-            const int base = t * UNITS_PER_TILE;         // number of the tile's first unit
-            // ---- S^T = K Q^T (9 chunks), dP^T = latent dO^T (8 chunks) ----
-            for (int u = 0; u < UNITS_PER_TILE && alive; ++u) {
-                const int slot = (base + u) % RING_SLOTS;
-                alive = __all_sync(0xffffffffU,
-                                   mbar_wait(smem_u32(&sh->unit_full[slot]), ((base + u) / RING_SLOTS) & 1, abort_flag, &absorbed_backward_status));
+            alive = wait_both(sh->q_full, sh->peer_q_full, t);
+            if (!alive) {
+                break;
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                mma_pair_ss_split(tmem_base + TMEM_S, k_lo + LATENT_CHUNKS * (KEY_SLOT >> 4) + 2 * k, HI, rope_lo + 2 * k, HI, IDESC_SCORE, k != 0 ? 1U : 0U,
+                                  leader);
+            }
+            issue_scores(tmem_base + TMEM_S, smem_base + Q_OFFSET, false, &sh->q_refill_free);
+            both(&sh->s_full);
+            alive = wait_both(sh->do_full, sh->peer_do_full, t);
+            if (!alive) {
+                break;
+            }
+            issue_scores(tmem_base + TMEM_DP, smem_base + DO_OFFSET, true, &sh->do_refill_free);
+            both(&sh->dp_full);
+            alive = __all_sync(0xffffffffU, wait(sh->p_full, t)) && wait_both(sh->q_refilled, sh->peer_q_refilled, t);
+            if (!alive) {
+                break;
+            }
+            issue_gradients(ds_lo, smem_base + Q_OFFSET, t == 0);
+#pragma unroll
+            for (int kk = 0; kk < 6; ++kk) {
+                mma_pair_ss_split(tmem_base + TMEM_DROPE, ds_lo + (kk >> 2) * (KEY_SLOT >> 4) + 2 * (kk & 3), HI,
+                                  rope_all_lo + (kk / 3) * (ROW_SLOT >> 4) + (kk % 3) * (2048 >> 4), HI, IDESC_ROPE, (t | kk) != 0 ? 1U : 0U, leader);
+            }
+            both(&sh->q_free);
+            alive = wait_both(sh->do_refilled, sh->peer_do_refilled, t);
+            if (!alive) {
+                break;
+            }
+            issue_gradients(p_lo, smem_base + DO_OFFSET, false);
+            both(&sh->do_free);
+        }
+    } else {
+        // =================== softmax: thread = (key, 24 of the 96 rows) ======
+        const int tmem_lane = (warp % 4) * 32 + lane;
+        const int key_in_cta = tmem_lane & 63;
+        const int row_half = tmem_lane >> 6;
+        const int share = warp / 4;
+        const int n0 = row_half * HALF_ROWS + share * SHARE_ROWS;           // first row of this thread
+        const uint32_t lane_base = tmem_base + (static_cast<uint32_t>((warp % 4) * 32) << 16);
+        const int key_pos = key_start + static_cast<int>(rank) * CTA_KEYS + key_in_cta;
+        const uint32_t p_full_bar = map_to_cta(smem_u32(&sh->p_full), 0);
+        bool alive = true;
+        for (int t = 0; t < tile_count; ++t) {
+            alive = __all_sync(0xffffffffU, wait(sh->rows_ready[t & 1], t >> 1) && wait(sh->s_full, t));
+            if (!alive) {
+                break;
+            }
+            tc_fence_after_sync();
+            const Rows& rows = sh->rows[t & 1];
+            const int row0 = first_row + t * TILE_ROWS;
+            const bool masked = row0 / p.heads < key_start + KEYS - 1 || row0 + TILE_ROWS > rows_per_sequence;
+            uint32_t x[SHARE_ROWS];
+            float prob[SHARE_ROWS];
+#pragma unroll
+            for (int n = 0; n < SHARE_ROWS; n += 8) {
+                tmem_ld_x8(lane_base + TMEM_S + share * SHARE_ROWS + n, x + n);
+            }
+            tmem_wait_ld();
+#pragma unroll
+            for (int n = 0; n < SHARE_ROWS; n += 4) {
+                const float4 l = *reinterpret_cast<const float4*>(rows.lse2 + n0 + n);
+                prob[n] = exp2_approx(fmaf(__uint_as_float(x[n]), p.scale_log2, -l.x));
+                prob[n + 1] = exp2_approx(fmaf(__uint_as_float(x[n + 1]), p.scale_log2, -l.y));
+                prob[n + 2] = exp2_approx(fmaf(__uint_as_float(x[n + 2]), p.scale_log2, -l.z));
+                prob[n + 3] = exp2_approx(fmaf(__uint_as_float(x[n + 3]), p.scale_log2, -l.w));
+            }
+            if (masked) {
+#pragma unroll
+                for (int n = 0; n < SHARE_ROWS; n += 4) {
+                    const int4 token = *reinterpret_cast<const int4*>(rows.token + n0 + n);
+                    prob[n] = key_pos <= token.x ? prob[n] : 0.0F;
+                    prob[n + 1] = key_pos <= token.y ? prob[n + 1] : 0.0F;
+                    prob[n + 2] = key_pos <= token.z ? prob[n + 2] : 0.0F;
+                    prob[n + 3] = key_pos <= token.w ? prob[n + 3] : 0.0F;
+                }
+            }
+            // P^T and dS^T of the previous tile have been read; this thread's three 16-byte units, swizzled by the key
+            if (t > 0) {
+                alive = __all_sync(0xffffffffU, wait(sh->do_free, t - 1));
                 if (!alive) {
                     break;
                 }
-                tc_fence_after_sync();
-                const uint32_t src = ring + slot * SLOT_BYTES;
-                const bool is_dout = (u >= 2 && u < 4) || u >= 7;
-                int first_chunk, chunks_here = 2;
-                if (u < 2) {
-                    first_chunk = 4 * (1 - half) + 2 * u;
-                } else if (u < 4) {
-                    first_chunk = 4 * (1 - half) + 2 * (u - 2);
-                } else if (u < 6) {
-                    first_chunk = 4 * half + 2 * (u - 4);
-                } else if (u == 6) {
-                    first_chunk = LATENT_CHUNKS, chunks_here = 1;
-                } else {
-                    first_chunk = 4 * half + 2 * (u - 7);
-                }
-                const uint32_t acc = tmem_base + (is_dout ? TMEM_X1 : TMEM_X0);
-                for (int cc = 0; cc < chunks_here; ++cc) {
+            }
+            auto unit_address = [&](int offset, int unit) {
+                const int u = n0 / 8 + unit;
+                return reinterpret_cast<uint4*>(smem_raw + offset + (u >> 3) * KEY_SLOT + key_in_cta * 128 + (((u & 7) ^ (key_in_cta & 7)) * 16));
+            };
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        const bool first = (u == 0 || u == 2) && cc == 0 && k == 0;
-                        mma_ss_elect(acc, make_kmajor_desc(k_smem + (first_chunk + cc) * KEY_CHUNK + k * 32),
-                                     make_kmajor_desc(src + cc * ROW_CHUNK + k * 32), IDESC_SCORE, first ? 0U : 1U, leader);
-                    }
-                }
-                if (u < RETAINED_FROM) {
-                    mma_commit_elect(smem_u32(&sh->unit_empty[slot]), leader);
-                }
+            for (int unit = 0; unit < SHARE_ROWS / 8; ++unit) {
+                const float* v = prob + 8 * unit;
+                *unit_address(P_OFFSET, unit) =
+                    make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
             }
-            if (!alive) {
-                break;
-            }
-            mma_commit_elect(smem_u32(&sh->s_ready), leader);
-            alive = __all_sync(0xffffffffU, mbar_wait(smem_u32(&sh->p_ready), t & 1, abort_flag, &absorbed_backward_status));
+            alive = __all_sync(0xffffffffU, wait(sh->dp_full, t));
             if (!alive) {
                 break;
             }
             tc_fence_after_sync();
-            // ---- gradient products on the five retained units, in the order they were loaded:
-            //      dlatent half += dS^T query_latent (2 units), dkey_rope += dS^T query_rope,
-            //      dlatent half += P^T dO (2 units) ----
-            for (int u = RETAINED_FROM; u < UNITS_PER_TILE; ++u) {
-                const int slot = (base + u) % RING_SLOTS;
-                const uint32_t src = ring + slot * SLOT_BYTES;
-                if (u == 6) {
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        mma_ts_elect(tmem_base + TMEM_DROPE, tmem_base + TMEM_X1 + (k / 2) * 32 + (k % 2) * 8, make_smem_desc(src + k * 2048, ROW_CHUNK, 1024),
-                                     IDESC_ROPE, (t | k) != 0 ? 1U : 0U, leader);
-                    }
-                } else {
-                    const bool from_dout = u >= 7;
-                    const uint32_t operand = tmem_base + (from_dout ? TMEM_X0 : TMEM_X1);     // P^T for dO, dS^T for query_latent
-                    const uint32_t acc = tmem_base + TMEM_DLAT + ((from_dout ? u - 7 : u - 4) & 1) * 128;
+            for (int n = 0; n < SHARE_ROWS; n += 8) {
+                tmem_ld_x8(lane_base + TMEM_DP + share * SHARE_ROWS + n, x + n);
+            }
+            tmem_wait_ld();
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        mma_ts_elect(acc, operand + (k / 2) * 32 + (k % 2) * 8, make_smem_desc(src + k * 2048, ROW_CHUNK, 1024), IDESC_GRAD,
-                                     (from_dout || t != 0 || k != 0) ? 1U : 0U, leader);
-                    }
-                }
-                mma_commit_elect(smem_u32(&sh->unit_empty[slot]), leader);
+            for (int unit = 0; unit < SHARE_ROWS / 8; ++unit) {
+                const float4 d0 = *reinterpret_cast<const float4*>(rows.delta + n0 + 8 * unit);
+                const float4 d1 = *reinterpret_cast<const float4*>(rows.delta + n0 + 8 * unit + 4);
+                const float* v = prob + 8 * unit;
+                const uint32_t* y = x + 8 * unit;
+                *unit_address(DS_OFFSET, unit) =
+                    make_uint4(pack_bf16x2(v[0] * (__uint_as_float(y[0]) - d0.x) * p.scale, v[1] * (__uint_as_float(y[1]) - d0.y) * p.scale),
+                               pack_bf16x2(v[2] * (__uint_as_float(y[2]) - d0.z) * p.scale, v[3] * (__uint_as_float(y[3]) - d0.w) * p.scale),
+                               pack_bf16x2(v[4] * (__uint_as_float(y[4]) - d1.x) * p.scale, v[5] * (__uint_as_float(y[5]) - d1.y) * p.scale),
+                               pack_bf16x2(v[6] * (__uint_as_float(y[6]) - d1.z) * p.scale, v[7] * (__uint_as_float(y[7]) - d1.w) * p.scale));
             }
-        }
-        if (alive) {
-            mma_commit_elect(smem_u32(&sh->final_full), leader);
-        }
-    } else {
-        // =================== softmax: thread = (key, 32 of the 64 rows) ======
-        const int group = warp / 4;
-        const int r = threadIdx.x % KEYS;
-        const uint32_t lane_base = static_cast<uint32_t>((warp % 4) * 32) << 16;
-        const int key_pos = key_start + r;
-        const uint32_t st_tmem = tmem_base + lane_base + TMEM_X0 + group * 32;
-        const uint32_t dpt_tmem = tmem_base + lane_base + TMEM_X1 + group * 32;
-        bool alive = true;
-        for (int t = 0; t < tile_count; ++t) {
-            alive = __all_sync(0xffffffffU, mbar_wait(smem_u32(&sh->rows_ready[t & 1]), (t >> 1) & 1, abort_flag, &absorbed_backward_status) &&
-                                                mbar_wait(smem_u32(&sh->s_ready), t & 1, abort_flag, &absorbed_backward_status));
-            if (!alive) {
-                break;
-            }
-            tc_fence_after_sync();
-            uint32_t p_packed[16], ds_packed[16];
-            score_tile_share(p, st_tmem, dpt_tmem, sh->rows[t & 1], group, key_pos, sh->masked[t & 1] != 0, p_packed, ds_packed);
-            tmem_st_x16(st_tmem, p_packed);
-            tmem_st_x16(dpt_tmem, ds_packed);
-            tmem_wait_st();
+            fence_proxy_async_smem();
             tc_fence_before_sync();
-            mbar_arrive(smem_u32(&sh->p_ready));
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive_remote(p_full_bar);
+                mbar_arrive(smem_u32(&sh->rows_done[t & 1]));
+            }
         }
-        if (alive) {
-            alive = __all_sync(0xffffffffU, mbar_wait(smem_u32(&sh->final_full), 0, abort_flag, &absorbed_backward_status));
-        }
+        alive = __all_sync(0xffffffffU, alive && wait(sh->do_free, tile_count - 1));
         if (alive) {
             tc_fence_after_sync();
-            const bool valid = key_pos < p.sequence;
-            const size_t key_row = static_cast<size_t>(b) * p.sequence + key_pos;
-            // group g handles dlatent columns 128g..128g+127 of this half and dkey_rope columns 32g..32g+31
-            __nv_bfloat16* dlat_row = p.dlatent + key_row * RANK + half * 256 + group * 128;
-            float* partial_row = reinterpret_cast<float*>(p.dq_lat) +
-                                 ((static_cast<size_t>(part) * p.batch + b) * p.sequence + key_pos) * (RANK + ROPE);
+            // Every MMA has finished, so the operands' memory is idle: a warp lays out 32 keys x 128 bytes at a time in a 4 KB
+            // slab (swizzled) from where a TMA store writes whole lines; keys past the end of the sequence are clipped.
+            const uint32_t slabs = static_cast<uint32_t>(warp) * 5 * SLAB_BYTES;
+            uint8_t* slab_row = smem_raw + slabs + lane * 128;
+            const int store_key = key_start + static_cast<int>(rank) * CTA_KEYS + (warp & 1) * 32;
+            const int column = share * 256 + row_half * 128;
+            const bool has_rope = row_half == 0;                // lanes 64-127 hold the same sums
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                uint32_t values[32];
-                tmem_ld_x32(tmem_base + lane_base + TMEM_DLAT + group * 128 + c * 32, values);
+            for (int c = 0; c < 5; ++c) {
+                uint32_t v[32];
+                if (c == 4 && !has_rope) {
+                    break;
+                }
+                tmem_ld_x32(lane_base + (c < 4 ? TMEM_DLAT + share * 128 + c * 32 : TMEM_DROPE + share * 32), v);
                 tmem_wait_ld();
-                if (valid && p.key_direct != 0) {
-                    store_bf16x32(dlat_row + c * 32, values);
-                } else if (valid) {
-                    store_f32x32(partial_row + half * 256 + group * 128 + c * 32, values);
+                if (p.key_direct == 0) {
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) {
+                        *reinterpret_cast<uint4*>(slab_row + c * SLAB_BYTES + ((u ^ (lane & 7)) * 16)) = make_uint4(v[4 * u], v[4 * u + 1], v[4 * u + 2], v[4 * u + 3]);
+                    }
+                } else if (c < 4) {
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const uint32_t* y = v + 8 * u;
+                        *reinterpret_cast<uint4*>(slab_row + (c / 2) * SLAB_BYTES + ((((c & 1) * 4 + u) ^ (lane & 7)) * 16)) =
+                            make_uint4(pack_bf16x2(__uint_as_float(y[0]), __uint_as_float(y[1])), pack_bf16x2(__uint_as_float(y[2]), __uint_as_float(y[3])),
+                                       pack_bf16x2(__uint_as_float(y[4]), __uint_as_float(y[5])), pack_bf16x2(__uint_as_float(y[6]), __uint_as_float(y[7])));
+                    }
+                } else if (key_pos < p.sequence) {
+                    store_bf16x32(p.dk_rope + (static_cast<size_t>(b) * p.sequence + key_pos) * ROPE + share * 32, v);
                 }
             }
-            if (half == 0) {
-                uint32_t values[32];
-                tmem_ld_x32(tmem_base + lane_base + TMEM_DROPE + group * 32, values);
-                tmem_wait_ld();
-                if (valid && p.key_direct != 0) {
-                    store_bf16x32(p.dk_rope + key_row * ROPE + group * 32, values);
-                } else if (valid) {
-                    store_f32x32(partial_row + RANK + group * 32, values);
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0 && store_key < p.sequence) {
+                if (p.key_direct == 0) {
+                    for (int c = 0; c < (has_rope ? 5 : 4); ++c) {
+                        tma_store_4d(&p.partials, smem_base + slabs + c * SLAB_BYTES, c < 4 ? column + c * 32 : RANK + share * 32, 0, store_key, part * p.batch + b);
+                    }
+                } else {
+                    for (int c = 0; c < 2; ++c) {
+                        tma_store_3d(&p.dlatent_out, smem_base + slabs + c * SLAB_BYTES, column + c * 64, store_key, b);
+                    }
                 }
+                tma_store_commit();
+                tma_store_wait_read();
             }
         }
     }
 
+    // ---- teardown -----------------------------------------------------------
     __syncwarp();
     tc_fence_before_sync();
     __syncthreads();
@@ -546,9 +721,10 @@ __global__ void __launch_bounds__(THREADS, 1) absorbed_backward_key_kernel(const
             __nanosleep(1000);
         }
     }
+    cluster_sync_all();                 // neither CTA frees tensor memory or exits while the other may still signal it
     if (warp == MMA_WARP) {
         tc_fence_after_sync();
-        tmem_dealloc(tmem_base, TMEM_COLUMNS);
+        tmem_dealloc_pair(tmem_base, TMEM_COLUMNS);
     }
 }
 
@@ -965,27 +1141,37 @@ void mla_compressed_attention_backward_cuda(__nv_bfloat16* dquery_latent, __nv_b
     const std::size_t rows = static_cast<std::size_t>(q_rows);
     const unsigned delta_blocks = static_cast<unsigned>(rows / 8 + 1 < 148 * 16 ? rows / 8 + 1 : 148 * 16);
     launch_chained(absorbed_delta_kernel, dim3(delta_blocks), dim3(256), 0, stream, dquery_rope, output_gradient, output, rows);
-    // Key side split (see key_tile_parts): about four waves of CTAs of equal length, never more
-    // parts per key tile than fp32 partial rows fit into the dquery_latent buffer.
+    // Key side split (see key_tile_parts): about four waves of clusters of equal length, parts of fewer than four tiles only
+    // while all of them run at once, never more parts per key tile than fp32 partial rows fit into the dquery_latent buffer.
     const int key_tiles = (sequence_length + KEYS - 1) / KEYS;
-    const long long row_tiles = (rows_per_sequence + ROWS - 1) / ROWS;
-    auto tiles_of = [&](int key_tile) { return row_tiles - (static_cast<long long>(key_tile) * KEYS * heads) / ROWS; };
+    auto tiles_of = [&](int key_tile) { return (rows_per_sequence - static_cast<long long>(key_tile) * KEYS * heads + KEY_SIDE_ROWS - 1) / KEY_SIDE_ROWS; };
     long long tile_units = 0;
     for (int kt = 0; kt < key_tiles; ++kt) {
         tile_units += tiles_of(kt);
     }
-    const int sms = multiprocessors();
+    tile_units *= batch_size;
+    const long long clusters = std::max(1, multiprocessors() / 2);
     const long long max_parts = std::max<long long>(1, std::min<long long>(64, static_cast<long long>(heads) * RANK * 2 / ((RANK + ROPE) * 4)));
-    long long chunk = std::max<long long>(16, (2 * batch_size * tile_units + 4LL * sms - 1) / (4LL * sms));
-    chunk = std::max(chunk, (row_tiles + max_parts - 1) / max_parts);
+    long long chunk = std::max(std::min<long long>(4, (tile_units + clusters - 1) / clusters), (tile_units + 4 * clusters - 1) / (4 * clusters));
+    chunk = std::max(chunk, (tiles_of(0) + max_parts - 1) / max_parts);
     long long part_count = 0;
     for (int kt = 0; kt < key_tiles; ++kt) {
         part_count += (tiles_of(kt) + chunk - 1) / chunk;
     }
     params.key_chunk = static_cast<int>(std::min<long long>(chunk, 0x7fffffffLL));
     params.key_direct = part_count == key_tiles ? 1 : 0;
-    const dim3 key_grid(static_cast<unsigned>(part_count), 2, batch_size);
-    launch_chained(absorbed_backward_key_kernel, key_grid, dim3(THREADS), ks::SMEM_BYTES, stream, params);
+    params.key_lat8 = make_bf16_batched_chunked_map(kv_latent, batch_size, sequence_length, LATENT_CHUNKS, ks::CTA_KEYS, LATENT_CHUNKS);
+    params.key_rope1 = make_bf16_batched_chunked_map(key_rope, batch_size, sequence_length, 1, ks::CTA_KEYS, 1);
+    params.row_q8 = make_bf16_batched_chunked_map(query_latent, batch_size, rows_per_sequence, LATENT_CHUNKS, ks::HALF_ROWS, LATENT_CHUNKS);
+    params.row_q2 = make_bf16_batched_chunked_map(query_latent, batch_size, rows_per_sequence, LATENT_CHUNKS, ks::HALF_ROWS, 2);
+    params.row_do8 = make_bf16_batched_chunked_map(output_gradient, batch_size, rows_per_sequence, LATENT_CHUNKS, ks::HALF_ROWS, LATENT_CHUNKS);
+    params.row_do2 = make_bf16_batched_chunked_map(output_gradient, batch_size, rows_per_sequence, LATENT_CHUNKS, ks::HALF_ROWS, 2);
+    params.row_rope = make_bf16_batched_chunked_map(query_rope, batch_size, rows_per_sequence, 1, ks::HALF_ROWS, 1);
+    params.dlatent_out = make_bf16_batched_rows_map(dkv_latent, batch_size, sequence_length, RANK, 32);
+    params.partials = make_f32_records_map(dquery_latent, params.key_direct != 0 ? 1 : static_cast<std::uint64_t>(max_parts) * batch_size,
+                                           params.key_direct != 0 ? 1 : sequence_length, 1, RANK + ROPE, 32);
+    const dim3 key_grid(static_cast<unsigned>(2 * part_count), 1, batch_size);
+    launch_chained(absorbed_backward_key_kernel, key_grid, dim3(ks::KEY_THREADS), ks::SMEM_BYTES, stream, params);
     if (params.key_direct == 0) {
         launch_chained(absorbed_backward_reduce_kernel, dim3(sequence_length, batch_size), dim3(144), 0, stream, params);
     }

@@ -76,6 +76,28 @@ CUtensorMap make_bf16_chunked_map(const void* base, std::uint64_t rows, std::uin
     return map;
 }
 
+CUtensorMap make_bf16_batched_chunked_map(const void* base, std::uint64_t batch, std::uint64_t rows, std::uint32_t chunks, std::uint32_t box_rows,
+                                          std::uint32_t box_chunks) {
+    if ((reinterpret_cast<std::uintptr_t>(base) & 15U) != 0) {
+        throw std::invalid_argument("tensor base must be 16-byte aligned");
+    }
+    if (batch == 0 || rows == 0 || chunks == 0 || box_rows == 0 || box_rows > 256 || box_chunks == 0 || box_chunks > chunks) {
+        throw std::invalid_argument("empty tensor or bad tile shape");
+    }
+    CUtensorMap map;
+    const cuuint64_t dims[4] = {64, rows, chunks, batch};
+    const cuuint64_t strides[3] = {chunks * 128ULL, 128, rows * chunks * 128ULL};
+    const cuuint32_t box[4] = {64, box_rows, box_chunks, 1};
+    const cuuint32_t element_strides[4] = {1, 1, 1, 1};
+    const CUresult result = encode_entry_point()(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, element_strides,
+                                                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (result != CUDA_SUCCESS) {
+        throw std::runtime_error("cuTensorMapEncodeTiled (batched chunks) failed with code " + std::to_string(static_cast<int>(result)));
+    }
+    return map;
+}
+
 CUtensorMap make_u64_rows_map(const void* base, std::uint64_t rows, std::uint32_t row_words, std::uint32_t box_words, std::uint32_t box_rows) {
     if ((reinterpret_cast<std::uintptr_t>(base) & 15U) != 0 || (row_words * 8) % 16 != 0 || (box_words * 8) % 16 != 0) {
         throw std::invalid_argument("tensor base, row length and box width must be multiples of 16 bytes");

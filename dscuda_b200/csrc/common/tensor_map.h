@@ -23,6 +23,11 @@ CUtensorMap make_bf16_tile_map(const void* base, std::uint64_t rows, std::uint64
 CUtensorMap make_bf16_chunked_map(const void* base, std::uint64_t rows, std::uint32_t chunks, std::uint64_t row_stride_elements,
                                   std::uint32_t box_rows, std::uint32_t box_chunks);
 
+// The same for a batch of `rows` rows each, everything contiguous: box {64, box_rows, box_chunks, 1} at {0, row, chunk, entry}.
+// Rows past the entry's last one read as zero, not as the next entry's.
+CUtensorMap make_bf16_batched_chunked_map(const void* base, std::uint64_t batch, std::uint64_t rows, std::uint32_t chunks, std::uint32_t box_rows,
+                                          std::uint32_t box_chunks);
+
 // A plain (unswizzled) view of `rows` rows of `row_words` 64-bit words each, rows contiguous.  One load of
 // a box {box_words, box_rows} at {word, row} lands in shared memory row after row, box_words * 8 bytes each.
 CUtensorMap make_u64_rows_map(const void* base, std::uint64_t rows, std::uint32_t row_words, std::uint32_t box_words, std::uint32_t box_rows);

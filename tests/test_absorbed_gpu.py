@@ -120,6 +120,33 @@ def test_backward_matches_oracle(gpu, b, t, h):
         torch.testing.assert_close(got.cpu().float(), ref.bfloat16().float(), atol=1e-2, rtol=1e-2)
 
 
+@pytest.mark.parametrize("b,t,h", [(1, 1, 1), (1, 95, 1), (1, 96, 1), (2, 97, 1), (1, 128, 3), (2, 129, 3), (1, 48, 2), (1, 49, 2), (3, 127, 16), (1, 256, 3),
+                                   (2, 383, 7)])
+def test_backward_tile_edges(gpu, b, t, h):
+    """Sizes around the key side's tiles of 96 rows (48 to a CTA) and 128 keys (64 to a CTA), with one part (results written directly: fewer than
+    three heads) and with several, against float64.  P, dS and the results are rounded to bfloat16 (2**-9 relative each), so three roundings of
+    independent signs stay below 1e-2 in the 2-norm."""
+    from conftest import rel_l2
+    from dscuda_b200 import mla
+    generator = torch.Generator().manual_seed(1000 * t + h)
+    shapes = ((b, t, h, 512), (b, t, h, 64), (b, t, 512), (b, t, 64))
+    inputs = [(torch.randn(s, generator=generator) * .25).bfloat16() for s in shapes]
+    dout = (torch.randn(b, t, h, 512, generator=generator) * .2).bfloat16()
+    scale = ctypes.c_float(576 ** -.5).value
+    device_inputs = [x.to(gpu) for x in inputs]
+    out, lse = mla.mla_forward(*device_inputs, scale)
+    first = mla.mla_backward(dout.to(gpu), out, lse, *device_inputs, scale)
+    again = mla.mla_backward(dout.to(gpu), out, lse, *device_inputs, scale)
+    torch.cuda.synchronize()
+    assert mla.device_status() == 0
+    reference = oracle.absorbed_backward(dout.double(), out.cpu().double(), lse.cpu().double(), *(x.double() for x in inputs), scale, oracle.causal_mask(t))
+    for name, x, y, ref in zip(("dquery", "dquery_rope", "dlatent", "dkey_rope"), first, again, reference):
+        assert torch.equal(x, y), name
+        # a single key has dS = 0 exactly: what is left of dquery and dkey_rope is the rounding of delta
+        assert t == 1 or rel_l2(x.cpu().double(), ref) <= 1e-2, name
+        torch.testing.assert_close(x.cpu().double(), ref.double(), atol=1e-2, rtol=1e-2)
+
+
 def test_decode_empty_and_overlong_lengths(gpu):
     """Length 0: NaN output and -inf LSE, as the softmax of an empty row gives in the reference
     (reference/python/mla.py:36-38), whatever an earlier call left in the workspace.  A length above
