@@ -6,9 +6,8 @@
 // (576 score columns, 512 value columns), so the work is split the way the
 // reference splits it (kernels/attention/mla/sm89.cu:295 query side, :356 key
 // side): one kernel owns the key-side gradients, one owns the query-side
-// gradients, and each recomputes P from the saved LSE.  Both are tcgen05 kernels whose score tiles are S^T = K Q^T, keys on
-// the tensor-memory lanes and (token, head) rows on the columns, so that one thread owns one key and the per-row constants
-// (LSE, delta, token index) are read from shared memory.
+// gradients, and each recomputes P from the saved LSE.  Both are tcgen05 kernels on
+// clusters of two CTAs, with the operands' roles exchanged.
 //
 // One call launches, on the caller's stream:
 //   1. absorbed_delta_kernel: delta[row] = sum_c dO[row,c] O[row,c], kept in the
@@ -18,11 +17,8 @@
 //      memory; the 96-row tiles at or after the diagonal stream by and stay there from the score products to the gradient
 //      products dlatent += dS^T query_latent + P^T dO and dkey_rope += dS^T query_rope.  Single writer per output element,
 //      no atomics; with several parts absorbed_backward_reduce_kernel adds them in order;
-//   3. absorbed_backward_query_kernel: CTA = 64 (token, head) rows, resident as the
-//      B operands query_latent | query_rope | dO (136 KB); every 128-key tile up
-//      to the diagonal streams by twice: for S^T / dP^T, and again as the
-//      MN-major A operand of dQ^T += K^T dS^T (output columns on the lanes, rows on
-//      the columns; dS^T goes through shared memory as the B operand).
+//   3. absorbed_backward_query_kernel: cluster = 128 (token, head) rows; query and dO stay in shared memory, every 96-key
+//      tile up to the diagonal streams by and stays there from S / dP to dquery += dS K.
 //
 // Warps 0-7: softmax; warp 8: MMA issue (whole warp, one elected lane executes); warp 9: TMA loads.  Every wait is bounded.
 #include "mla.h"
@@ -46,35 +42,35 @@ constexpr int RANK = MLA_KV_RANK;             // 512
 constexpr int ROPE = MLA_ROPE_SIZE;           // 64
 constexpr int CHUNKS = (RANK + ROPE) / 64;    // 9 column chunks of 64; chunk 8 is the rotary part
 constexpr int LATENT_CHUNKS = RANK / 64;      // 8
-constexpr int KEYS = 128;                     // keys per tile = MMA M = tensor-memory lanes
-constexpr int ROWS = 64;                      // (token, head) rows per tile = MMA N
-constexpr int KEY_CHUNK = KEYS * 128;         // 16 KB: [128 keys x 64 bf16]
-constexpr int ROW_CHUNK = ROWS * 128;         //  8 KB: [64 rows x 64 bf16]
+constexpr int KEYS = 128;                     // key side: keys per cluster
 constexpr int THREADS = 320;
 constexpr int MMA_WARP = 8;
 constexpr int LOAD_WARP = 9;
 constexpr int TMEM_COLUMNS = 512;
-constexpr int MISC_BYTES = 2048;
 constexpr float LOG2E = 1.4426950408889634F;
 
 __device__ int absorbed_backward_status = 0;
 
 struct AbsorbedBackwardParams {
-    CUtensorMap q_lat;      // [B*T*H, 512] box 64 x 64
-    CUtensorMap q_rope;     // [B*T*H, 64]  box 64 x 64
-    CUtensorMap d_out;      // [B*T*H, 512] box 64 x 64
-    CUtensorMap k_lat;      // [B*T, 512]   box 128 x 64
-    CUtensorMap k_rope;     // [B*T, 64]    box 128 x 64
-    // key side; batch entries apart, so rows and keys past the end of one read as zero
+    // key side; batch entries are a dimension of their own, so rows and keys past the end of one read as zero
     CUtensorMap key_lat8;   // kv_latent, box 64 keys x 8 chunks
     CUtensorMap key_rope1;  // key_rope, box 64 keys
-    CUtensorMap row_q8;     // query_latent, box 48 rows x 8 chunks
+    CUtensorMap row_q4;     // query_latent, box 48 rows x 4 chunks
     CUtensorMap row_q2;     // ... x 2 chunks
-    CUtensorMap row_do8;    // dO likewise
+    CUtensorMap row_do4;    // dO likewise
     CUtensorMap row_do2;
     CUtensorMap row_rope;   // query_rope, box 48 rows
     CUtensorMap dlatent_out;    // stores of 32 keys: 64 bf16 columns of dlatent, 32 fp32 columns of a partial sum
     CUtensorMap partials;
+    // query side, likewise
+    CUtensorMap own_q8;     // query_latent, box 64 rows x 8 chunks
+    CUtensorMap own_rope;   // query_rope, box 64 rows
+    CUtensorMap own_do8;    // dO, box 64 rows x 8 chunks
+    CUtensorMap stream_k4;  // kv_latent, box 48 keys x 4 chunks
+    CUtensorMap stream_k2;  // ... x 2 chunks
+    CUtensorMap stream_rope;    // key_rope, box 48 keys
+    CUtensorMap dq_out;     // stores of 32 rows x 64 columns
+    CUtensorMap dq_rope_out;
     __nv_bfloat16* dq_lat;  // [B,T,H,512]
     __nv_bfloat16* dq_rope; // [B,T,H,64]; the first float of each row holds delta until the query kernel overwrites it
     __nv_bfloat16* dlatent; // [B,T,512]
@@ -104,82 +100,8 @@ __device__ __forceinline__ int key_tile_parts(const AbsorbedBackwardParams& p, i
     return (key_tile_row_tiles(p, key_tile) + p.key_chunk - 1) / p.key_chunk;
 }
 
-// Per-row constants of a 64-row tile, written by the load warp, read by every softmax thread.
-struct RowConstants {
-    alignas(16) float lse2[ROWS];     // LSE * log2 e
-    alignas(16) float delta[ROWS];
-    alignas(16) int token[ROWS];      // token index of the row, -1 for rows past the end of the sequence
-};
-
 __device__ __forceinline__ float stored_delta(const AbsorbedBackwardParams& p, size_t global_row) {
     return *reinterpret_cast<const float*>(p.dq_rope + global_row * ROPE);
-}
-
-// Lanes of one warp fill the constants of rows [row0, row0 + 64) of sequence `b`.
-__device__ __forceinline__ void fill_row_constants(const AbsorbedBackwardParams& p, RowConstants& rc, int b, int row0, int lane) {
-    const int rows_per_sequence = p.sequence * p.heads;
-#pragma unroll
-    for (int e = 0; e < ROWS / 32; ++e) {
-        const int n = e * 32 + lane;
-        const int row = row0 + n;
-        float lse_value = 0.0F, delta_value = 0.0F;
-        int token = -1;
-        if (row < rows_per_sequence) {
-            token = row / p.heads;
-            const int head = row - token * p.heads;
-            lse_value = p.lse[(static_cast<size_t>(b) * p.heads + head) * p.sequence + token] * LOG2E;
-            delta_value = stored_delta(p, static_cast<size_t>(b) * rows_per_sequence + row);
-        }
-        rc.lse2[n] = lse_value;
-        rc.delta[n] = delta_value;
-        rc.token[n] = token;
-    }
-}
-
-// One thread's share of a score tile: key `key_pos` (its tensor-memory lane) against 32 of the
-// tile's 64 rows.  Reads S^T and dP^T (fp32) from tensor memory and returns P^T and
-// dS^T = P^T (dP^T - delta) scale as packed bf16 pairs.  A key is visible to a row when
-// key_pos <= token(row); rows past the end have token -1.
-__device__ __forceinline__ void score_tile_share(const AbsorbedBackwardParams& p, uint32_t st_tmem, uint32_t dpt_tmem, const RowConstants& rc,
-                                                 int group, int key_pos, bool masked, uint32_t (&p_packed)[16], uint32_t (&ds_packed)[16]) {
-    uint32_t sb[32];
-    float prob[32];
-    tmem_ld_x32(st_tmem, sb);
-    tmem_wait_ld();
-    const float4* lse4 = reinterpret_cast<const float4*>(rc.lse2 + group * 32);
-    const float4* delta4 = reinterpret_cast<const float4*>(rc.delta + group * 32);
-    const int4* token4 = reinterpret_cast<const int4*>(rc.token + group * 32);
-#pragma unroll
-    for (int n = 0; n < 32; n += 4) {
-        const float4 l = lse4[n / 4];
-        prob[n] = exp2_approx(fmaf(__uint_as_float(sb[n]), p.scale_log2, -l.x));
-        prob[n + 1] = exp2_approx(fmaf(__uint_as_float(sb[n + 1]), p.scale_log2, -l.y));
-        prob[n + 2] = exp2_approx(fmaf(__uint_as_float(sb[n + 2]), p.scale_log2, -l.z));
-        prob[n + 3] = exp2_approx(fmaf(__uint_as_float(sb[n + 3]), p.scale_log2, -l.w));
-    }
-    if (masked) {
-#pragma unroll
-        for (int n = 0; n < 32; n += 4) {
-            const int4 t = token4[n / 4];
-            prob[n] = key_pos <= t.x ? prob[n] : 0.0F;
-            prob[n + 1] = key_pos <= t.y ? prob[n + 1] : 0.0F;
-            prob[n + 2] = key_pos <= t.z ? prob[n + 2] : 0.0F;
-            prob[n + 3] = key_pos <= t.w ? prob[n + 3] : 0.0F;
-        }
-    }
-#pragma unroll
-    for (int n = 0; n < 32; n += 2) {
-        p_packed[n / 2] = pack_bf16x2(prob[n], prob[n + 1]);
-    }
-    tmem_ld_x32(dpt_tmem, sb);
-    tmem_wait_ld();
-#pragma unroll
-    for (int n = 0; n < 32; n += 4) {
-        const float4 d = delta4[n / 4];
-        ds_packed[n / 2] = pack_bf16x2(prob[n] * (__uint_as_float(sb[n]) - d.x) * p.scale, prob[n + 1] * (__uint_as_float(sb[n + 1]) - d.y) * p.scale);
-        ds_packed[n / 2 + 1] =
-            pack_bf16x2(prob[n + 2] * (__uint_as_float(sb[n + 2]) - d.z) * p.scale, prob[n + 3] * (__uint_as_float(sb[n + 3]) - d.w) * p.scale);
-    }
 }
 
 __device__ __forceinline__ void store_bf16x32(__nv_bfloat16* dst, const uint32_t* values) {
@@ -191,13 +113,6 @@ __device__ __forceinline__ void store_bf16x32(__nv_bfloat16* dst, const uint32_t
         vec.z = pack_bf16x2(__uint_as_float(values[e + 4]), __uint_as_float(values[e + 5]));
         vec.w = pack_bf16x2(__uint_as_float(values[e + 6]), __uint_as_float(values[e + 7]));
         *reinterpret_cast<uint4*>(dst + e) = vec;
-    }
-}
-
-__device__ __forceinline__ void store_f32x32(float* dst, const uint32_t* values) {
-#pragma unroll
-    for (int e = 0; e < 32; e += 4) {
-        *reinterpret_cast<uint4*>(dst + e) = make_uint4(values[e], values[e + 1], values[e + 2], values[e + 3]);
     }
 }
 
@@ -249,10 +164,10 @@ __global__ void __launch_bounds__(256) absorbed_delta_kernel(__nv_bfloat16* dq_r
 // from L2 for 64 x 96 pairs.
 //
 // What bounds it: shared memory.  The resident keys (72 KB), P and dS (32 KB) and one tile of rows (114 KB) fill it, so the
-// chain scores -> softmax -> gradients of a tile is overlapped only by the loads of the next one: query_latent is loaded
-// again while P^T dO runs.  96 rows and not 128 because 128 do not fit.  One CTA per (128 keys, half of dlatent), which this
+// chain scores -> softmax -> gradients of a tile is overlapped only by the loads of the next one: a column half of an operand
+// is loaded again as soon as its gradient product has read it.  96 rows and not 128 because 128 do not fit.  One CTA per (128 keys, half of dlatent), which this
 // replaces, computed the scores twice, at the N = 64 rate: 1305 us at B=4 T=2048 H=16 against
-// 592 us now, 46 against 11 us at B=2 T=33 H=32 (where a part also had at least 1024 rows).
+// 580 us now, 46 against 11 us at B=2 T=33 H=32 (where a part also had at least 1024 rows).
 //
 // Tensor memory: dlatent 2 x 128 columns (lanes 0-63: columns 256a + 0..127, lanes 64-127: 256a + 128..255 of the same 64
 // keys), dkey_rope 64, S^T 48 (lanes 64-127: rows 48..95), dP^T 48.
@@ -295,23 +210,21 @@ struct Shared {
     Rows rows[2];
     // completed by TMA transactions of this CTA, one phase per tile
     uint64_t k_full;
-    uint64_t q_full;            // own rows: query_latent and the rotary chunk
-    uint64_t do_full;           // own rows: dO
-    uint64_t q_refilled;        // the other CTA's rows, and the rotary columns of all rows
-    uint64_t do_refilled;
+    uint64_t q_full[2];         // own rows of query_latent, by column half; the rotary chunk with half 0
+    uint64_t do_full[2];        // own rows of dO
+    uint64_t q_refilled[2];     // the other CTA's rows; the rotary columns of all rows with half 0
+    uint64_t do_refilled[2];
     // leader only: the same events of the other CTA, forwarded by its relay (one arrival)
     uint64_t peer_k_full;
-    uint64_t peer_q_full;
-    uint64_t peer_do_full;
-    uint64_t peer_q_refilled;
-    uint64_t peer_do_refilled;
+    uint64_t peer_q_full[2];
+    uint64_t peer_do_full[2];
+    uint64_t peer_q_refilled[2];
+    uint64_t peer_do_refilled[2];
     // completed by tcgen05.commit of the leader
-    uint64_t q_refill_free;     // S has read the four slots only it needs
-    uint64_t do_refill_free;
-    uint64_t s_full;
-    uint64_t dp_full;
-    uint64_t q_free;            // dS^T Q has read everything of query_latent and query_rope
-    uint64_t do_free;           // P^T dO too; P, dS and the accumulators are quiescent
+    uint64_t q_refill_free[2];  // S has read the half; half 1: S is complete
+    uint64_t do_refill_free[2]; // dP^T likewise
+    uint64_t q_free[2];         // dS^T Q has read the half (half 0: and query_rope)
+    uint64_t do_free[2];        // P^T dO has read the half; half 1: P, dS and the accumulators are quiescent
     // leader only: one arrival per softmax warp of either CTA, P^T and dS^T are stored
     uint64_t p_full;
     uint64_t rows_ready[2];     // the constants of a tile, by tile parity
@@ -356,7 +269,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ks::KEY_THREADS, 1) 
     }
 
     if (threadIdx.x == 0) {
-        for (uint64_t* bar = &sh->k_full; bar <= &sh->do_free; ++bar) {
+        for (uint64_t* bar = &sh->k_full; bar < &sh->p_full; ++bar) {
             mbar_init(smem_u32(bar), 1);
         }
         mbar_init(smem_u32(&sh->p_full), 16);
@@ -374,9 +287,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ks::KEY_THREADS, 1) 
     if (warp == LOAD_WARP && lane == 0) {
         tma_prefetch_descriptor(&p.key_lat8);
         tma_prefetch_descriptor(&p.key_rope1);
-        tma_prefetch_descriptor(&p.row_q8);
+        tma_prefetch_descriptor(&p.row_q4);
         tma_prefetch_descriptor(&p.row_q2);
-        tma_prefetch_descriptor(&p.row_do8);
+        tma_prefetch_descriptor(&p.row_do4);
         tma_prefetch_descriptor(&p.row_do2);
         tma_prefetch_descriptor(&p.row_rope);
     }
@@ -397,37 +310,35 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ks::KEY_THREADS, 1) 
             mbar_arrive_expect_tx(bar, K_BYTES);
             tma_load_4d(smem_base, &p.key_lat8, bar, 0, key_start + static_cast<int>(rank) * CTA_KEYS, 0, b);
             tma_load_4d(smem_base + LATENT_CHUNKS * KEY_SLOT, &p.key_rope1, bar, 0, key_start + static_cast<int>(rank) * CTA_KEYS, 0, b);
-            for (int t = 0; t < tile_count; ++t) {
+            bool alive = true;
+            for (int t = 0; t < tile_count && alive; ++t) {
                 const int row0 = first_row + t * TILE_ROWS;
-                if (t > 0 && !wait(sh->q_free, t - 1)) {
-                    break;
+                // i: query_latent halves 0 and 1, dO halves 0 and 1
+                for (int i = 0; i < 4 && alive; ++i) {
+                    const int a = i & 1;
+                    alive = t == 0 || wait(i < 2 ? sh->q_free[a] : sh->do_free[a], t - 1);
+                    if (alive) {
+                        bar = smem_u32(i < 2 ? &sh->q_full[a] : &sh->do_full[a]);
+                        mbar_arrive_expect_tx(bar, (i == 0 ? 5 : 4) * ROW_SLOT);
+                        if (i == 0) {
+                            tma_load_4d(smem_base + ROPE_OFFSET, &p.row_rope, bar, 0, row0 + own, 0, b);
+                        }
+                        tma_load_4d(smem_base + (i < 2 ? Q_OFFSET : DO_OFFSET) + 4 * a * ROW_SLOT, i < 2 ? &p.row_q4 : &p.row_do4, bar, 0, row0 + own, 4 * a, b);
+                    }
                 }
-                bar = smem_u32(&sh->q_full);
-                mbar_arrive_expect_tx(bar, CHUNKS * ROW_SLOT);
-                tma_load_4d(smem_base + ROPE_OFFSET, &p.row_rope, bar, 0, row0 + own, 0, b);
-                tma_load_4d(smem_base + Q_OFFSET, &p.row_q8, bar, 0, row0 + own, 0, b);
-                if (t > 0 && !wait(sh->do_free, t - 1)) {
-                    break;
-                }
-                bar = smem_u32(&sh->do_full);
-                mbar_arrive_expect_tx(bar, LATENT_CHUNKS * ROW_SLOT);
-                tma_load_4d(smem_base + DO_OFFSET, &p.row_do8, bar, 0, row0 + own, 0, b);
-                if (!wait(sh->q_refill_free, t)) {
-                    break;
-                }
-                bar = smem_u32(&sh->q_refilled);
-                mbar_arrive_expect_tx(bar, 6 * ROW_SLOT);
-                for (int a = 0; a < 2; ++a) {
-                    tma_load_4d(smem_base + Q_OFFSET + (4 * a + other_slot) * ROW_SLOT, &p.row_q2, bar, 0, row0 + other, 4 * a + own_chunk, b);
-                    tma_load_4d(smem_base + ROPE_ALL_OFFSET + a * ROW_SLOT, &p.row_rope, bar, 0, row0 + a * HALF_ROWS, 0, b);
-                }
-                if (!wait(sh->do_refill_free, t)) {
-                    break;
-                }
-                bar = smem_u32(&sh->do_refilled);
-                mbar_arrive_expect_tx(bar, 4 * ROW_SLOT);
-                for (int a = 0; a < 2; ++a) {
-                    tma_load_4d(smem_base + DO_OFFSET + (4 * a + other_slot) * ROW_SLOT, &p.row_do2, bar, 0, row0 + other, 4 * a + own_chunk, b);
+                for (int i = 0; i < 4 && alive; ++i) {
+                    const int a = i & 1;
+                    alive = wait(i < 2 ? sh->q_refill_free[a] : sh->do_refill_free[a], t);
+                    if (alive) {
+                        bar = smem_u32(i < 2 ? &sh->q_refilled[a] : &sh->do_refilled[a]);
+                        mbar_arrive_expect_tx(bar, (i == 0 ? 4 : 2) * ROW_SLOT);
+                        tma_load_4d(smem_base + (i < 2 ? Q_OFFSET : DO_OFFSET) + (4 * a + other_slot) * ROW_SLOT, i < 2 ? &p.row_q2 : &p.row_do2, bar, 0, row0 + other,
+                                    4 * a + own_chunk, b);
+                        if (i == 0) {
+                            tma_load_4d(smem_base + ROPE_ALL_OFFSET, &p.row_rope, bar, 0, row0, 0, b);
+                            tma_load_4d(smem_base + ROPE_ALL_OFFSET + ROW_SLOT, &p.row_rope, bar, 0, row0 + HALF_ROWS, 0, b);
+                        }
+                    }
                 }
             }
         }
@@ -467,13 +378,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ks::KEY_THREADS, 1) 
             }
             for (int t = 0; t < tile_count && alive; ++t) {
                 // in the order in which they are loaded
-                uint64_t* const mine[4] = {&sh->q_full, &sh->do_full, &sh->q_refilled, &sh->do_refilled};
-                uint64_t* const leaders[4] = {&sh->peer_q_full, &sh->peer_do_full, &sh->peer_q_refilled, &sh->peer_do_refilled};
+                uint64_t* const mine[4] = {sh->q_full, sh->do_full, sh->q_refilled, sh->do_refilled};
+                uint64_t* const leaders[4] = {sh->peer_q_full, sh->peer_do_full, sh->peer_q_refilled, sh->peer_do_refilled};
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    alive = alive && wait(*mine[i], t);
+                for (int i = 0; i < 8; ++i) {
+                    alive = alive && wait(mine[i / 2][i & 1], t);
                     if (alive) {
-                        mbar_arrive_remote(map_to_cta(smem_u32(leaders[i]), 0));
+                        mbar_arrive_remote(map_to_cta(smem_u32(&leaders[i / 2][i & 1]), 0));
                     }
                 }
             }
@@ -494,35 +405,26 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ks::KEY_THREADS, 1) 
             commit_pair(smem_u32(bar), leader);
             commit_pair(map_to_cta(smem_u32(bar), 1), leader);
         };
-        // K (chunks of all columns) times the own rows in slots at `operand`; slots {2,3,6,7} (refilled in the leader) first,
-        // then {0,1,4,5} (refilled in the other CTA)
-        auto issue_scores = [&](uint32_t acc, uint32_t operand, bool fresh, uint64_t* refill_free) {
+        // K times the own rows in the four slots of column half `half` of the operand at `operand`
+        auto issue_scores = [&](uint32_t acc, uint32_t operand, int half, bool fresh) {
             const uint32_t row_lo = smem_desc_lo(operand, 16);
 #pragma unroll
-            for (int group = 0; group < 2; ++group) {
+            for (int n = 0; n < 4; ++n) {
 #pragma unroll
-                for (int n = 0; n < 4; ++n) {
-                    const int c = (group == 0 ? 2 : 0) + (n & 1) + (n >> 1) * 4;
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        mma_pair_ss_split(acc, k_lo + c * (KEY_SLOT >> 4) + 2 * k, HI, row_lo + c * (ROW_SLOT >> 4) + 2 * k, HI, IDESC_SCORE,
-                                          (fresh && group == 0 && n == 0 && k == 0) ? 0U : 1U, leader);
-                    }
+                for (int k = 0; k < 4; ++k) {
+                    mma_pair_ss_split(acc, k_lo + (4 * half + n) * (KEY_SLOT >> 4) + 2 * k, HI, row_lo + (4 * half + n) * (ROW_SLOT >> 4) + 2 * k, HI, IDESC_SCORE,
+                                      (fresh && n == 0 && k == 0) ? 0U : 1U, leader);
                 }
-                commit_pair(group == 0 ? smem_u32(refill_free) : map_to_cta(smem_u32(refill_free), 1), leader);
             }
         };
-        // dlatent += A (P^T or dS^T at a_lo) times the columns in slots at `operand`: rows 48g.. of half a in slots 4a + 2g, + 1
-        auto issue_gradients = [&](uint32_t a_lo, uint32_t operand, bool fresh) {
+        // columns of half a of dlatent += A (P^T or dS^T at a_lo) times the operand: its rows 48g.. are in slots 4a + 2g, + 1
+        auto issue_gradients = [&](uint32_t a_lo, uint32_t operand, int a, bool fresh) {
             const uint32_t column_lo = smem_desc_lo(operand, ROW_SLOT);
 #pragma unroll
-            for (int a = 0; a < 2; ++a) {
-#pragma unroll
-                for (int kk = 0; kk < 6; ++kk) {
-                    mma_pair_ss_split(tmem_base + TMEM_DLAT + a * 128, a_lo + (kk >> 2) * (KEY_SLOT >> 4) + 2 * (kk & 3), HI,
-                                      column_lo + (4 * a + 2 * (kk / 3)) * (ROW_SLOT >> 4) + (kk % 3) * (2048 >> 4), HI, IDESC_GRAD,
-                                      (fresh && kk == 0) ? 0U : 1U, leader);
-                }
+            for (int kk = 0; kk < 6; ++kk) {
+                mma_pair_ss_split(tmem_base + TMEM_DLAT + a * 128, a_lo + (kk >> 2) * (KEY_SLOT >> 4) + 2 * (kk & 3), HI,
+                                  column_lo + (4 * a + 2 * (kk / 3)) * (ROW_SLOT >> 4) + (kk % 3) * (2048 >> 4), HI, IDESC_GRAD, (fresh && kk == 0) ? 0U : 1U,
+                                  leader);
             }
         };
         auto wait_both = [&](uint64_t& mine, uint64_t& others, int phase) {
@@ -532,40 +434,53 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ks::KEY_THREADS, 1) 
         };
         bool alive = wait_both(sh->k_full, sh->peer_k_full, 0);
         for (int t = 0; t < tile_count && alive; ++t) {
-            alive = wait_both(sh->q_full, sh->peer_q_full, t);
-            if (!alive) {
-                break;
-            }
+            for (int a = 0; a < 2 && alive; ++a) {
+                alive = wait_both(sh->q_full[a], sh->peer_q_full[a], t);
+                if (!alive) {
+                    break;
+                }
+                if (a == 0) {
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                mma_pair_ss_split(tmem_base + TMEM_S, k_lo + LATENT_CHUNKS * (KEY_SLOT >> 4) + 2 * k, HI, rope_lo + 2 * k, HI, IDESC_SCORE, k != 0 ? 1U : 0U,
-                                  leader);
+                    for (int k = 0; k < 4; ++k) {
+                        mma_pair_ss_split(tmem_base + TMEM_S, k_lo + LATENT_CHUNKS * (KEY_SLOT >> 4) + 2 * k, HI, rope_lo + 2 * k, HI, IDESC_SCORE,
+                                          k != 0 ? 1U : 0U, leader);
+                    }
+                }
+                issue_scores(tmem_base + TMEM_S, smem_base + Q_OFFSET, a, false);
+                both(&sh->q_refill_free[a]);
             }
-            issue_scores(tmem_base + TMEM_S, smem_base + Q_OFFSET, false, &sh->q_refill_free);
-            both(&sh->s_full);
-            alive = wait_both(sh->do_full, sh->peer_do_full, t);
-            if (!alive) {
-                break;
+            for (int a = 0; a < 2 && alive; ++a) {
+                alive = wait_both(sh->do_full[a], sh->peer_do_full[a], t);
+                if (!alive) {
+                    break;
+                }
+                issue_scores(tmem_base + TMEM_DP, smem_base + DO_OFFSET, a, a == 0);
+                both(&sh->do_refill_free[a]);
             }
-            issue_scores(tmem_base + TMEM_DP, smem_base + DO_OFFSET, true, &sh->do_refill_free);
-            both(&sh->dp_full);
-            alive = __all_sync(0xffffffffU, wait(sh->p_full, t)) && wait_both(sh->q_refilled, sh->peer_q_refilled, t);
-            if (!alive) {
-                break;
-            }
-            issue_gradients(ds_lo, smem_base + Q_OFFSET, t == 0);
+            alive = alive && __all_sync(0xffffffffU, wait(sh->p_full, t));
+            for (int a = 0; a < 2 && alive; ++a) {
+                alive = wait_both(sh->q_refilled[a], sh->peer_q_refilled[a], t);
+                if (!alive) {
+                    break;
+                }
+                issue_gradients(ds_lo, smem_base + Q_OFFSET, a, t == 0);
+                if (a == 0) {
 #pragma unroll
-            for (int kk = 0; kk < 6; ++kk) {
-                mma_pair_ss_split(tmem_base + TMEM_DROPE, ds_lo + (kk >> 2) * (KEY_SLOT >> 4) + 2 * (kk & 3), HI,
-                                  rope_all_lo + (kk / 3) * (ROW_SLOT >> 4) + (kk % 3) * (2048 >> 4), HI, IDESC_ROPE, (t | kk) != 0 ? 1U : 0U, leader);
+                    for (int kk = 0; kk < 6; ++kk) {
+                        mma_pair_ss_split(tmem_base + TMEM_DROPE, ds_lo + (kk >> 2) * (KEY_SLOT >> 4) + 2 * (kk & 3), HI,
+                                          rope_all_lo + (kk / 3) * (ROW_SLOT >> 4) + (kk % 3) * (2048 >> 4), HI, IDESC_ROPE, (t | kk) != 0 ? 1U : 0U, leader);
+                    }
+                }
+                both(&sh->q_free[a]);
             }
-            both(&sh->q_free);
-            alive = wait_both(sh->do_refilled, sh->peer_do_refilled, t);
-            if (!alive) {
-                break;
+            for (int a = 0; a < 2 && alive; ++a) {
+                alive = wait_both(sh->do_refilled[a], sh->peer_do_refilled[a], t);
+                if (!alive) {
+                    break;
+                }
+                issue_gradients(p_lo, smem_base + DO_OFFSET, a, false);
+                both(&sh->do_free[a]);
             }
-            issue_gradients(p_lo, smem_base + DO_OFFSET, false);
-            both(&sh->do_free);
         }
     } else {
         // =================== softmax: thread = (key, 24 of the 96 rows) ======
@@ -579,7 +494,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ks::KEY_THREADS, 1) 
         const uint32_t p_full_bar = map_to_cta(smem_u32(&sh->p_full), 0);
         bool alive = true;
         for (int t = 0; t < tile_count; ++t) {
-            alive = __all_sync(0xffffffffU, wait(sh->rows_ready[t & 1], t >> 1) && wait(sh->s_full, t));
+            alive = __all_sync(0xffffffffU, wait(sh->rows_ready[t & 1], t >> 1) && wait(sh->q_refill_free[1], t));
             if (!alive) {
                 break;
             }
@@ -614,7 +529,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ks::KEY_THREADS, 1) 
             }
             // P^T and dS^T of the previous tile have been read; this thread's three 16-byte units, swizzled by the key
             if (t > 0) {
-                alive = __all_sync(0xffffffffU, wait(sh->do_free, t - 1));
+                alive = __all_sync(0xffffffffU, wait(sh->do_free[1], t - 1));
                 if (!alive) {
                     break;
                 }
@@ -629,7 +544,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ks::KEY_THREADS, 1) 
                 *unit_address(P_OFFSET, unit) =
                     make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
             }
-            alive = __all_sync(0xffffffffU, wait(sh->dp_full, t));
+            alive = __all_sync(0xffffffffU, wait(sh->do_refill_free[1], t));
             if (!alive) {
                 break;
             }
@@ -659,7 +574,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ks::KEY_THREADS, 1) 
                 mbar_arrive(smem_u32(&sh->rows_done[t & 1]));
             }
         }
-        alive = __all_sync(0xffffffffU, alive && wait(sh->do_free, tile_count - 1));
+        alive = __all_sync(0xffffffffU, alive && wait(sh->do_free[1], tile_count - 1));
         if (alive) {
             tc_fence_after_sync();
             // Every MMA has finished, so the operands' memory is idle: a warp lays out 32 keys x 128 bytes at a time in a 4 KB
@@ -760,274 +675,371 @@ __global__ void __launch_bounds__(144) absorbed_backward_reduce_kernel(const __g
 }
 
 // ---------------------------------------------------------------------------
-// Query side.  Tensor memory: dQ^T as five 64-column blocks at 0..319 (block m holds output
-// columns 128m..128m+127 on the lanes and the 64 rows on the columns; block 4 is the rotary part
-// on lanes 0..63), S^T 320..383, dP^T 384..447.  Shared memory: the 64 rows' query_latent (8
-// chunks), query_rope (1) and dO (8) as 8 KB K-major chunks, a 16 KB dS^T tile (the MN-major B
-// operand of dQ^T += K^T dS^T), a ring of two 32 KB units (pairs of 16 KB key chunks), constants.
-// Per key tile: 5 units (chunk pairs 0-1 .. 6-7, then the rotary chunk alone) for S^T and dP^T,
-// the softmax, and the same 5 units again as the MN-major A operand of the gradient product.
-// The rotary unit's second half is whatever the slot held before: its products land on lanes
-// 64..127 of block 4, which nothing reads.
+// Query side: the key side with the operands exchanged.  A cluster of two CTAs takes 128 (token, head) rows; CTA r owns rows
+// 64r..64r+63, which stay in shared memory as A operands (query 72 KB, dO 64 KB), and every 96-key tile up to the diagonal
+// streams by, CTA r supplying 48 of its keys:
+//
+//   S = Q K^T, dP = dO latent^T     (N = 96), both from the same eight latent chunks of the own keys;
+//   dquery_latent += dS latent      (N = 256 twice), dquery_rope += dS K_rope (N = 128, there twice).
+//
+// The slots of column half a (chunks 4a..4a+3) go round on their own: loaded, read by both score products, two of the four
+// refilled with the other CTA's keys, read by the gradient product, loaded again for the next tile; so the loads of one half
+// run under the MMAs of the other.
+//
+// What bounds it: the chain of a tile, as on the key side.  64 rows of one CTA with 128-key tiles, which this replaces, ran
+// at the N = 64 rate and streamed every key tile twice (288 KB for 64 x 128 pairs, L2 latency over two 32 KB slots; here
+// 84 KB for 64 x 96): 680 us at B=4 T=2048 H=16 against
+// 520 us now.
+//
+// Tensor memory and warps as on the key side; a softmax thread owns 24 keys of one row, so LSE, delta and token are its own.
 // ---------------------------------------------------------------------------
 namespace qs {
-constexpr int RING_SLOTS = 2;
-constexpr int SLOT_BYTES = 2 * KEY_CHUNK;
-constexpr int Q_BYTES = CHUNKS * ROW_CHUNK;
-constexpr int DO_BYTES = LATENT_CHUNKS * ROW_CHUNK;
-constexpr int DS_BYTES = KEYS * 128;
-constexpr int SMEM_BYTES = Q_BYTES + DO_BYTES + DS_BYTES + RING_SLOTS * SLOT_BYTES + MISC_BYTES + 1024;
-constexpr int UNITS_PER_TILE = 10;
-constexpr uint32_t TMEM_DQT = 0;
-constexpr uint32_t TMEM_X0 = 320;
-constexpr uint32_t TMEM_X1 = 384;
+constexpr int TILE_ROWS = 128;                      // rows of a cluster
+constexpr int CTA_ROWS = 64;
+constexpr int TILE_KEYS = 96;
+constexpr int HALF_KEYS = 48;                       // keys a CTA supplies
+constexpr int SHARE_KEYS = 24;                      // keys of a softmax thread
+constexpr int ROW_SLOT = CTA_ROWS * 128;            // 8 KB: [64 rows x 64 bf16]
+constexpr int KEY_SLOT = HALF_KEYS * 128;           // 6 KB: [48 keys x 64 bf16]
+constexpr int Q_BYTES = CHUNKS * ROW_SLOT;
+constexpr int DO_OFFSET = Q_BYTES;
+constexpr int DO_BYTES = LATENT_CHUNKS * ROW_SLOT;
+constexpr int DS_OFFSET = DO_OFFSET + DO_BYTES;     // dS: [64 rows x 96 keys] as two 64-key chunks
+constexpr int K_OFFSET = DS_OFFSET + 2 * ROW_SLOT;
+constexpr int ROPE_OFFSET = K_OFFSET + LATENT_CHUNKS * KEY_SLOT;        // own keys, for the scores
+constexpr int ROPE_ALL_OFFSET = ROPE_OFFSET + KEY_SLOT;                 // all 96 keys, for dquery_rope
+constexpr int MISC_OFFSET = ROPE_ALL_OFFSET + 2 * KEY_SLOT;
+constexpr int SMEM_BYTES = MISC_OFFSET + 1024;
+constexpr int SLAB_BYTES = 32 * 128;
+constexpr uint32_t TMEM_DQ = 0;
+constexpr uint32_t TMEM_DROPE = 256;
+constexpr uint32_t TMEM_S = 320;
+constexpr uint32_t TMEM_DP = 368;
 static_assert(SMEM_BYTES <= 232448, "query-side shared memory");
+static_assert(8 * 3 * SLAB_BYTES <= MISC_OFFSET, "result slabs lie in the operands' memory");
 
 struct Shared {
-    uint64_t resident_full;
-    uint64_t unit_full[RING_SLOTS];
-    uint64_t unit_empty[RING_SLOTS];
-    uint64_t rows_ready;
-    uint64_t s_ready;
-    uint64_t ds_ready;          // 256 softmax threads: dS^T is in shared memory
-    uint64_t final_full;
+    // completed by TMA transactions of this CTA; the arrays by column half
+    uint64_t rows_full;
+    uint64_t k_full[2];             // own keys (the rotary chunk with half 0)
+    uint64_t refilled[2];           // the other CTA's keys (the rotary columns of all keys with half 0)
+    // leader only: the same events of the other CTA, forwarded by its relay (one arrival)
+    uint64_t peer_rows_full;
+    uint64_t peer_k_full[2];
+    uint64_t peer_refilled[2];
+    // completed by tcgen05.commit of the leader
+    uint64_t refill_free[2];        // both score products have read the half; half 1: dP is complete
+    uint64_t s_full;
+    uint64_t k_free[2];             // the gradient products have read the half; half 1: dS and the accumulators are quiescent
+    // leader only: one arrival per softmax warp of either CTA, dS is stored
+    uint64_t ds_full;
     uint32_t tmem_base;
     int abort_flag;
-    RowConstants rows;
 };
-static_assert(sizeof(Shared) <= MISC_BYTES, "query-side barrier block too large");
+static_assert(sizeof(Shared) <= SMEM_BYTES - MISC_OFFSET, "query-side barrier block too large");
 }  // namespace qs
 
-__global__ void __launch_bounds__(THREADS, 1) absorbed_backward_query_kernel(const __grid_constant__ AbsorbedBackwardParams p) {
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) absorbed_backward_query_kernel(const __grid_constant__ AbsorbedBackwardParams p) {
     using namespace qs;
     extern __shared__ uint8_t smem_raw[];
-    if (*reinterpret_cast<volatile int*>(&absorbed_backward_status) == STATUS_WAIT_TIMEOUT) {
-        grid_dependency_wait();
-        return;
-    }
     const int warp = threadIdx.x / 32;
     const int lane = threadIdx.x % 32;
+    const uint32_t rank = cluster_cta_rank();
     const int b = blockIdx.z;
     const int rows_per_sequence = p.sequence * p.heads;
-    const int row0 = static_cast<int>(gridDim.x - 1 - blockIdx.x) * ROWS;       // late rows see the most keys: longest first
-    const int last_row = min(row0 + ROWS, rows_per_sequence) - 1;
-    const int first_token = row0 / p.heads;
-    const int tile_count = (last_row / p.heads) / KEYS + 1;
+    const int row0 = static_cast<int>((gridDim.x >> 1) - 1 - (blockIdx.x >> 1)) * TILE_ROWS;       // late rows see the most keys: longest first
+    const int own_row0 = row0 + static_cast<int>(rank) * CTA_ROWS;
+    const int last_token = (min(row0 + TILE_ROWS, rows_per_sequence) - 1) / p.heads;
+    const int tile_count = last_token / TILE_KEYS + 1;
 
-    const uint32_t smem_base = (smem_u32(smem_raw) + 1023U) & ~1023U;
-    uint8_t* smem_aligned = smem_raw + (smem_base - smem_u32(smem_raw));
-    const uint32_t q_smem = smem_base;
-    const uint32_t do_smem = q_smem + Q_BYTES;
-    const uint32_t ds_smem = do_smem + DO_BYTES;
-    uint8_t* ds_ptr = smem_aligned + Q_BYTES + DO_BYTES;
-    const uint32_t ring = ds_smem + DS_BYTES;
-    Shared* sh = reinterpret_cast<Shared*>(smem_aligned + Q_BYTES + DO_BYTES + DS_BYTES + RING_SLOTS * SLOT_BYTES);
+    const uint32_t smem_base = smem_u32(smem_raw);
+    Shared* sh = reinterpret_cast<Shared*>(smem_raw + MISC_OFFSET);
     volatile int* abort_flag = &sh->abort_flag;
+    if ((smem_base & 1023U) != 0U) {            // a property of the kernel image: the same in both CTAs
+        grid_dependency_wait();
+        if (threadIdx.x == 0) {
+            atomicExch(&absorbed_backward_status, STATUS_SMEM_MISALIGNED);
+        }
+        return;
+    }
 
     if (threadIdx.x == 0) {
-        mbar_init(smem_u32(&sh->resident_full), 1);
-        for (int i = 0; i < RING_SLOTS; ++i) {
-            mbar_init(smem_u32(&sh->unit_full[i]), 1);
-            mbar_init(smem_u32(&sh->unit_empty[i]), 1);
+        for (uint64_t* bar = &sh->rows_full; bar < &sh->ds_full; ++bar) {
+            mbar_init(smem_u32(bar), 1);
         }
-        mbar_init(smem_u32(&sh->rows_ready), 1);
-        mbar_init(smem_u32(&sh->s_ready), 1);
-        mbar_init(smem_u32(&sh->ds_ready), 256);
-        mbar_init(smem_u32(&sh->final_full), 1);
+        mbar_init(smem_u32(&sh->ds_full), 16);
         sh->abort_flag = 0;
         mbar_init_fence();
     }
     if (warp == MMA_WARP) {
-        tmem_alloc(smem_u32(&sh->tmem_base), TMEM_COLUMNS);
-        tmem_relinquish();
+        tmem_alloc_pair(smem_u32(&sh->tmem_base), TMEM_COLUMNS);
+        tmem_relinquish_pair();
     }
     if (warp == LOAD_WARP && lane == 0) {
-        tma_prefetch_descriptor(&p.q_lat);
-        tma_prefetch_descriptor(&p.q_rope);
-        tma_prefetch_descriptor(&p.d_out);
-        tma_prefetch_descriptor(&p.k_lat);
-        tma_prefetch_descriptor(&p.k_rope);
+        tma_prefetch_descriptor(&p.own_q8);
+        tma_prefetch_descriptor(&p.own_rope);
+        tma_prefetch_descriptor(&p.own_do8);
+        tma_prefetch_descriptor(&p.stream_k4);
+        tma_prefetch_descriptor(&p.stream_k2);
+        tma_prefetch_descriptor(&p.stream_rope);
     }
     tc_fence_before_sync();
     __syncthreads();
+    cluster_sync_all();
     tc_fence_after_sync();
     grid_dependency_wait();
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&sh->tmem_base);
+    auto wait = [&](uint64_t& bar, int phase) { return mbar_wait(smem_u32(&bar), phase & 1, abort_flag, &absorbed_backward_status); };
 
     if (warp == LOAD_WARP) {
         // =================== TMA producer ===================================
-        fill_row_constants(p, sh->rows, b, row0, lane);
-        __syncwarp();
         if (lane == 0) {
-            mbar_arrive(smem_u32(&sh->rows_ready));
-            const uint32_t bar = smem_u32(&sh->resident_full);
+            const int own = static_cast<int>(rank) * HALF_KEYS, other = HALF_KEYS - own;
+            const int own_chunk = 2 * static_cast<int>(rank), other_slot = 2 - own_chunk;
+            uint32_t bar = smem_u32(&sh->rows_full);
             mbar_arrive_expect_tx(bar, Q_BYTES + DO_BYTES);
-            const int y = b * rows_per_sequence + row0;
-            for (int c = 0; c < LATENT_CHUNKS; ++c) {
-                tma_load_2d(q_smem + c * ROW_CHUNK, &p.q_lat, bar, c * 64, y);
-                tma_load_2d(do_smem + c * ROW_CHUNK, &p.d_out, bar, c * 64, y);
-            }
-            tma_load_2d(q_smem + LATENT_CHUNKS * ROW_CHUNK, &p.q_rope, bar, 0, y);
+            tma_load_4d(smem_base, &p.own_q8, bar, 0, own_row0, 0, b);
+            tma_load_4d(smem_base + LATENT_CHUNKS * ROW_SLOT, &p.own_rope, bar, 0, own_row0, 0, b);
+            tma_load_4d(smem_base + DO_OFFSET, &p.own_do8, bar, 0, own_row0, 0, b);
             bool alive = true;
-            int unit = 0;
             for (int j = 0; j < tile_count && alive; ++j) {
-                const int ky = b * p.sequence + j * KEYS;
-                for (int u = 0; u < UNITS_PER_TILE && alive; ++u, ++unit) {
-                    const int slot = unit % RING_SLOTS;
-                    if (unit >= RING_SLOTS) {
-                        alive = mbar_wait(smem_u32(&sh->unit_empty[slot]), (unit / RING_SLOTS - 1) & 1, abort_flag, &absorbed_backward_status);
-                        if (!alive) {
-                            break;
+                const int key0 = j * TILE_KEYS;
+                for (int a = 0; a < 2 && alive; ++a) {
+                    alive = j == 0 || wait(sh->k_free[a], j - 1);
+                    if (alive) {
+                        bar = smem_u32(&sh->k_full[a]);
+                        mbar_arrive_expect_tx(bar, (a == 0 ? 5 : 4) * KEY_SLOT);
+                        if (a == 0) {
+                            tma_load_4d(smem_base + ROPE_OFFSET, &p.stream_rope, bar, 0, key0 + own, 0, b);
+                        }
+                        tma_load_4d(smem_base + K_OFFSET + 4 * a * KEY_SLOT, &p.stream_k4, bar, 0, key0 + own, 4 * a, b);
+                    }
+                }
+                for (int a = 0; a < 2 && alive; ++a) {
+                    alive = wait(sh->refill_free[a], j);
+                    if (alive) {
+                        bar = smem_u32(&sh->refilled[a]);
+                        mbar_arrive_expect_tx(bar, (a == 0 ? 4 : 2) * KEY_SLOT);
+                        tma_load_4d(smem_base + K_OFFSET + (4 * a + other_slot) * KEY_SLOT, &p.stream_k2, bar, 0, key0 + other, 4 * a + own_chunk, b);
+                        if (a == 0) {
+                            tma_load_4d(smem_base + ROPE_ALL_OFFSET, &p.stream_rope, bar, 0, key0, 0, b);
+                            tma_load_4d(smem_base + ROPE_ALL_OFFSET + KEY_SLOT, &p.stream_rope, bar, 0, key0 + HALF_KEYS, 0, b);
                         }
                     }
-                    const uint32_t full = smem_u32(&sh->unit_full[slot]);
-                    const uint32_t dst = ring + slot * SLOT_BYTES;
-                    const int pair = u % 5;
-                    if (pair == 4) {
-                        mbar_arrive_expect_tx(full, KEY_CHUNK);
-                        tma_load_2d(dst, &p.k_rope, full, 0, ky);
-                    } else {
-                        mbar_arrive_expect_tx(full, 2 * KEY_CHUNK);
-                        tma_load_2d(dst, &p.k_lat, full, pair * 128, ky);
-                        tma_load_2d(dst + KEY_CHUNK, &p.k_lat, full, pair * 128 + 64, ky);
+                }
+            }
+        }
+    } else if (warp == MMA_WARP && rank != 0) {
+        // =================== relay: this CTA's "loaded" events -> the leader, in the order in which they are loaded =========
+        if (lane == 0) {
+            bool alive = wait(sh->rows_full, 0);
+            if (alive) {
+                mbar_arrive_remote(map_to_cta(smem_u32(&sh->peer_rows_full), 0));
+            }
+            for (int j = 0; j < tile_count && alive; ++j) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    alive = alive && wait(i < 2 ? sh->k_full[i & 1] : sh->refilled[i & 1], j);
+                    if (alive) {
+                        mbar_arrive_remote(map_to_cta(smem_u32(i < 2 ? &sh->peer_k_full[i & 1] : &sh->peer_refilled[i & 1]), 0));
                     }
                 }
             }
         }
     } else if (warp == MMA_WARP) {
-        // =================== MMA issuer (whole warp, elected lane executes) ==
+        // =================== MMA issuer (leader CTA; whole warp, elected lane executes) ==
         const uint32_t leader = elect_one();
-        constexpr uint32_t IDESC_SCORE = make_idesc_bf16(KEYS, ROWS, false, false);
-        constexpr uint32_t IDESC_DQT = make_idesc_bf16(128, ROWS, true, true);        // A = key chunks MN-major, B = dS^T MN-major
-        bool alive = __all_sync(0xffffffffU, mbar_wait(smem_u32(&sh->resident_full), 0, abort_flag, &absorbed_backward_status));
-        int unit = 0;
-        auto wait_unit = [&]() -> uint32_t {
-            const int slot = unit % RING_SLOTS;
-            alive = __all_sync(0xffffffffU, mbar_wait(smem_u32(&sh->unit_full[slot]), (unit / RING_SLOTS) & 1, abort_flag, &absorbed_backward_status));
+        constexpr uint32_t IDESC_SCORE = make_idesc_bf16(TILE_ROWS, TILE_KEYS, false, false);
+        constexpr uint32_t IDESC_GRAD = make_idesc_bf16(TILE_ROWS, 256, false, true);
+        constexpr uint32_t IDESC_ROPE = make_idesc_bf16(TILE_ROWS, 128, false, true);
+        constexpr uint32_t HI = smem_desc_hi(1024);
+        const uint32_t q_lo = smem_desc_lo(smem_base, 16);
+        const uint32_t do_lo = smem_desc_lo(smem_base + DO_OFFSET, 16);
+        const uint32_t ds_lo = smem_desc_lo(smem_base + DS_OFFSET, 16);
+        const uint32_t k_lo = smem_desc_lo(smem_base + K_OFFSET, 16);
+        const uint32_t rope_lo = smem_desc_lo(smem_base + ROPE_OFFSET, 16);
+        const uint32_t column_lo = smem_desc_lo(smem_base + K_OFFSET, KEY_SLOT);
+        const uint32_t rope_all_lo = smem_desc_lo(smem_base + ROPE_ALL_OFFSET, KEY_SLOT);
+        auto both = [&](uint64_t* bar) {        // one commit for this CTA's barrier, one for the other CTA's
+            commit_pair(smem_u32(bar), leader);
+            commit_pair(map_to_cta(smem_u32(bar), 1), leader);
+        };
+        auto issue_scores = [&](uint32_t acc, uint32_t a_lo, int half, bool fresh) {
+#pragma unroll
+            for (int n = 0; n < 4; ++n) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    mma_pair_ss_split(acc, a_lo + (4 * half + n) * (ROW_SLOT >> 4) + 2 * k, HI, k_lo + (4 * half + n) * (KEY_SLOT >> 4) + 2 * k, HI, IDESC_SCORE,
+                                      (fresh && n == 0 && k == 0) ? 0U : 1U, leader);
+                }
+            }
+        };
+        auto wait_both = [&](uint64_t& mine, uint64_t& others, int phase) {
+            const bool alive = __all_sync(0xffffffffU, wait(mine, phase) && wait(others, phase));
             tc_fence_after_sync();
-            return ring + slot * SLOT_BYTES;
+            return alive;
         };
-        auto release_unit = [&]() {
-            mma_commit_elect(smem_u32(&sh->unit_empty[unit % RING_SLOTS]), leader);
-            ++unit;
-        };
+        bool alive = wait_both(sh->rows_full, sh->peer_rows_full, 0);
         for (int j = 0; j < tile_count && alive; ++j) {
-            // ---- S^T = K Q^T, dP^T = latent dO^T ----
-            for (int u = 0; u < 5 && alive; ++u) {
-                const uint32_t src = wait_unit();
-                if (!alive) {
-                    break;
-                }
-                const int chunks_here = u == 4 ? 1 : 2;
-                for (int cc = 0; cc < chunks_here; ++cc) {
-                    const int chunk = 2 * u + cc;
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        mma_ss_elect(tmem_base + TMEM_X0, make_kmajor_desc(src + cc * KEY_CHUNK + k * 32), make_kmajor_desc(q_smem + chunk * ROW_CHUNK + k * 32),
-                                     IDESC_SCORE, (chunk | k) != 0 ? 1U : 0U, leader);
-                    }
-                    if (chunk < LATENT_CHUNKS) {
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            mma_ss_elect(tmem_base + TMEM_X1, make_kmajor_desc(src + cc * KEY_CHUNK + k * 32),
-                                         make_kmajor_desc(do_smem + chunk * ROW_CHUNK + k * 32), IDESC_SCORE, (chunk | k) != 0 ? 1U : 0U, leader);
-                        }
-                    }
-                }
-                release_unit();
-            }
+            alive = wait_both(sh->k_full[0], sh->peer_k_full[0], j);
             if (!alive) {
                 break;
             }
-            // this commit also covers the gradient products of the previous tile, the last readers of the dS^T tile
-            mma_commit_elect(smem_u32(&sh->s_ready), leader);
-            alive = __all_sync(0xffffffffU, mbar_wait(smem_u32(&sh->ds_ready), j & 1, abort_flag, &absorbed_backward_status));
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                mma_pair_ss_split(tmem_base + TMEM_S, q_lo + LATENT_CHUNKS * (ROW_SLOT >> 4) + 2 * k, HI, rope_lo + 2 * k, HI, IDESC_SCORE, k != 0 ? 1U : 0U,
+                                  leader);
+            }
+            issue_scores(tmem_base + TMEM_S, q_lo, 0, false);
+            issue_scores(tmem_base + TMEM_DP, do_lo, 0, true);
+            both(&sh->refill_free[0]);
+            alive = wait_both(sh->k_full[1], sh->peer_k_full[1], j);
             if (!alive) {
                 break;
             }
-            tc_fence_after_sync();
-            // ---- dQ^T block m += (key chunks 2m, 2m+1)^T dS^T ----
-            for (int m = 0; m < 5 && alive; ++m) {
-                const uint32_t src = wait_unit();
+            issue_scores(tmem_base + TMEM_S, q_lo, 1, false);
+            both(&sh->s_full);
+            issue_scores(tmem_base + TMEM_DP, do_lo, 1, false);
+            both(&sh->refill_free[1]);
+            alive = __all_sync(0xffffffffU, wait(sh->ds_full, j));
+            for (int a = 0; a < 2 && alive; ++a) {
+                alive = wait_both(sh->refilled[a], sh->peer_refilled[a], j);
                 if (!alive) {
                     break;
                 }
+                // keys 48g.. of column half a are in slots 4a + 2g, + 1
 #pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    mma_ss_elect(tmem_base + TMEM_DQT + m * ROWS, make_smem_desc(src + k * 2048, KEY_CHUNK, 1024), make_smem_desc(ds_smem + k * 2048, 16, 1024),
-                                 IDESC_DQT, (j | k) != 0 ? 1U : 0U, leader);
+                for (int kk = 0; kk < 6; ++kk) {
+                    mma_pair_ss_split(tmem_base + TMEM_DQ + a * 128, ds_lo + (kk >> 2) * (ROW_SLOT >> 4) + 2 * (kk & 3), HI,
+                                      column_lo + (4 * a + 2 * (kk / 3)) * (KEY_SLOT >> 4) + (kk % 3) * (2048 >> 4), HI, IDESC_GRAD, (j | kk) != 0 ? 1U : 0U,
+                                      leader);
                 }
-                release_unit();
+                if (a == 0) {
+#pragma unroll
+                    for (int kk = 0; kk < 6; ++kk) {
+                        mma_pair_ss_split(tmem_base + TMEM_DROPE, ds_lo + (kk >> 2) * (ROW_SLOT >> 4) + 2 * (kk & 3), HI,
+                                          rope_all_lo + (kk / 3) * (KEY_SLOT >> 4) + (kk % 3) * (2048 >> 4), HI, IDESC_ROPE, (j | kk) != 0 ? 1U : 0U, leader);
+                    }
+                }
+                both(&sh->k_free[a]);
             }
-        }
-        if (alive) {
-            mma_commit_elect(smem_u32(&sh->final_full), leader);
         }
     } else {
-        // =================== softmax: thread = (key, 32 of the 64 rows) ======
-        const int group = warp / 4;
-        const int r = threadIdx.x % KEYS;
-        const uint32_t lane_base = static_cast<uint32_t>((warp % 4) * 32) << 16;
-        const uint32_t st_tmem = tmem_base + lane_base + TMEM_X0 + group * 32;
-        const uint32_t dpt_tmem = tmem_base + lane_base + TMEM_X1 + group * 32;
-        const bool ragged = row0 + ROWS > rows_per_sequence;
-        bool alive = __all_sync(0xffffffffU, mbar_wait(smem_u32(&sh->rows_ready), 0, abort_flag, &absorbed_backward_status));
-        for (int j = 0; j < tile_count && alive; ++j) {
-            alive = __all_sync(0xffffffffU, mbar_wait(smem_u32(&sh->s_ready), j & 1, abort_flag, &absorbed_backward_status));
+        // =================== softmax: thread = (row, 24 of the 96 keys) ======
+        const int tmem_lane = (warp % 4) * 32 + lane;
+        const int row_in_cta = tmem_lane & 63;
+        const int key_half = tmem_lane >> 6;
+        const int share = warp / 4;
+        const int n0 = key_half * HALF_KEYS + share * SHARE_KEYS;           // first key of this thread
+        const uint32_t lane_base = tmem_base + (static_cast<uint32_t>((warp % 4) * 32) << 16);
+        const uint32_t ds_full_bar = map_to_cta(smem_u32(&sh->ds_full), 0);
+        const int row = own_row0 + row_in_cta;
+        float lse2 = 0.0F, delta = 0.0F;
+        int token = -1;                                                     // rows past the end see no key
+        if (row < rows_per_sequence) {
+            token = row / p.heads;
+            lse2 = p.lse[(static_cast<size_t>(b) * p.heads + (row - token * p.heads)) * p.sequence + token] * LOG2E;
+            delta = stored_delta(p, static_cast<size_t>(b) * rows_per_sequence + row);
+        }
+        bool alive = true;
+        for (int j = 0; j < tile_count; ++j) {
+            alive = __all_sync(0xffffffffU, wait(sh->s_full, j));
             if (!alive) {
                 break;
             }
             tc_fence_after_sync();
-            const int key_pos = j * KEYS + r;
-            const bool masked = ragged || j * KEYS + KEYS - 1 > first_token;
-            uint32_t p_packed[16], ds_packed[16];
-            score_tile_share(p, st_tmem, dpt_tmem, sh->rows, group, key_pos, masked, p_packed, ds_packed);
-            // row r of the MN-major tile: 64 rows = eight 16-byte units, swizzled by the key index
-            uint8_t* row = ds_ptr + r * 128;
+            const int visible = token + 1 - (j * TILE_KEYS + n0);          // keys n < visible count
+            uint32_t x[SHARE_KEYS];
+            float prob[SHARE_KEYS];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int unit16 = group * 4 + i;
-                *reinterpret_cast<uint4*>(row + ((unit16 ^ (r & 7)) * 16)) =
-                    make_uint4(ds_packed[4 * i], ds_packed[4 * i + 1], ds_packed[4 * i + 2], ds_packed[4 * i + 3]);
+            for (int n = 0; n < SHARE_KEYS; n += 8) {
+                tmem_ld_x8(lane_base + TMEM_S + share * SHARE_KEYS + n, x + n);
+            }
+            tmem_wait_ld();
+#pragma unroll
+            for (int n = 0; n < SHARE_KEYS; ++n) {
+                prob[n] = exp2_approx(fmaf(__uint_as_float(x[n]), p.scale_log2, -lse2));
+            }
+            if (visible < SHARE_KEYS) {
+#pragma unroll
+                for (int n = 0; n < SHARE_KEYS; ++n) {
+                    prob[n] = n < visible ? prob[n] : 0.0F;
+                }
+            }
+            // dP is complete, and dS of the previous tile has been read
+            alive = __all_sync(0xffffffffU, wait(sh->refill_free[1], j) && (j == 0 || wait(sh->k_free[1], j - 1)));
+            if (!alive) {
+                break;
+            }
+            tc_fence_after_sync();
+            __syncwarp();
+#pragma unroll
+            for (int n = 0; n < SHARE_KEYS; n += 8) {
+                tmem_ld_x8(lane_base + TMEM_DP + share * SHARE_KEYS + n, x + n);
+            }
+            tmem_wait_ld();
+#pragma unroll
+            for (int unit = 0; unit < SHARE_KEYS / 8; ++unit) {
+                const float* v = prob + 8 * unit;
+                const uint32_t* y = x + 8 * unit;
+                uint32_t packed[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    packed[e] = pack_bf16x2(v[2 * e] * (__uint_as_float(y[2 * e]) - delta) * p.scale, v[2 * e + 1] * (__uint_as_float(y[2 * e + 1]) - delta) * p.scale);
+                }
+                const int u = n0 / 8 + unit;        // 16-byte unit of the row, swizzled by the row
+                *reinterpret_cast<uint4*>(smem_raw + DS_OFFSET + (u >> 3) * ROW_SLOT + row_in_cta * 128 + (((u & 7) ^ (row_in_cta & 7)) * 16)) =
+                    make_uint4(packed[0], packed[1], packed[2], packed[3]);
             }
             fence_proxy_async_smem();
             tc_fence_before_sync();
-            mbar_arrive(smem_u32(&sh->ds_ready));
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive_remote(ds_full_bar);
+            }
         }
-        if (alive) {
-            alive = __all_sync(0xffffffffU, mbar_wait(smem_u32(&sh->final_full), 0, abort_flag, &absorbed_backward_status));
-        }
+        alive = __all_sync(0xffffffffU, alive && wait(sh->k_free[1], tile_count - 1));
         if (alive) {
             tc_fence_after_sync();
-            // thread = output column (lane r of block m), values = rows 32*group .. 32*group+31
-            const size_t first_global_row = static_cast<size_t>(b) * rows_per_sequence + row0 + group * 32;
-            const int rows_here = min(32, rows_per_sequence - (row0 + group * 32));
+            // Every MMA has finished, so the operands' memory is idle: 32 rows x 128 bytes at a time go through 4 KB slabs
+            // (swizzled), from where TMA stores write whole lines; rows past the end of the sequence are clipped.
+            const uint32_t slabs = static_cast<uint32_t>(warp) * 3 * SLAB_BYTES;
+            uint8_t* slab_row = smem_raw + slabs + lane * 128;
+            const int store_row = own_row0 + (warp & 1) * 32;
+            const int column = share * 256 + key_half * 128;
+            const int parts = warp < 2 ? 6 : 4;                 // warps 0 and 1 also store the rotary columns (lanes 64-127 hold the same sums)
 #pragma unroll
-            for (int m = 0; m < 5; ++m) {
-                uint32_t values[32];
-                tmem_ld_x32(tmem_base + lane_base + TMEM_DQT + m * ROWS + group * 32, values);
-                tmem_wait_ld();
-                if (m < 4) {
-                    __nv_bfloat16* dst = p.dq_lat + first_global_row * RANK + m * 128 + r;
-#pragma unroll
-                    for (int e = 0; e < 32; ++e) {
-                        if (e < rows_here) {
-                            dst[static_cast<size_t>(e) * RANK] = __float2bfloat16(__uint_as_float(values[e]));
-                        }
-                    }
-                } else if (r < ROPE) {
-                    __nv_bfloat16* dst = p.dq_rope + first_global_row * ROPE + r;
-#pragma unroll
-                    for (int e = 0; e < 32; ++e) {
-                        if (e < rows_here) {
-                            dst[static_cast<size_t>(e) * ROPE] = __float2bfloat16(__uint_as_float(values[e]));
-                        }
-                    }
+            for (int c = 0; c < 6; ++c) {
+                if (c >= parts) {
+                    break;
                 }
+                uint32_t v[32];
+                tmem_ld_x32(lane_base + (c < 4 ? TMEM_DQ + share * 128 + c * 32 : TMEM_DROPE + (c - 4) * 32), v);
+                tmem_wait_ld();
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const uint32_t* y = v + 8 * u;
+                    *reinterpret_cast<uint4*>(slab_row + (c / 2) * SLAB_BYTES + ((((c & 1) * 4 + u) ^ (lane & 7)) * 16)) =
+                        make_uint4(pack_bf16x2(__uint_as_float(y[0]), __uint_as_float(y[1])), pack_bf16x2(__uint_as_float(y[2]), __uint_as_float(y[3])),
+                                   pack_bf16x2(__uint_as_float(y[4]), __uint_as_float(y[5])), pack_bf16x2(__uint_as_float(y[6]), __uint_as_float(y[7])));
+                }
+            }
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0 && store_row < rows_per_sequence) {
+                for (int c = 0; c < 2; ++c) {
+                    tma_store_3d(&p.dq_out, smem_base + slabs + c * SLAB_BYTES, column + c * 64, store_row, b);
+                }
+                if (parts == 6) {
+                    tma_store_3d(&p.dq_rope_out, smem_base + slabs + 2 * SLAB_BYTES, 0, store_row, b);
+                }
+                tma_store_commit();
+                tma_store_wait_read();
             }
         }
     }
 
+    // ---- teardown -----------------------------------------------------------
     __syncwarp();
     tc_fence_before_sync();
     __syncthreads();
@@ -1036,9 +1048,10 @@ __global__ void __launch_bounds__(THREADS, 1) absorbed_backward_query_kernel(con
             __nanosleep(1000);
         }
     }
+    cluster_sync_all();                 // neither CTA frees tensor memory or exits while the other may still signal it
     if (warp == MMA_WARP) {
         tc_fence_after_sync();
-        tmem_dealloc(tmem_base, TMEM_COLUMNS);
+        tmem_dealloc_pair(tmem_base, TMEM_COLUMNS);
     }
 }
 
@@ -1121,11 +1134,6 @@ void mla_compressed_attention_backward_cuda(__nv_bfloat16* dquery_latent, __nv_b
     AbsorbedBackwardParams params{};
     const std::uint64_t q_rows = static_cast<std::uint64_t>(rows_per_sequence) * batch_size;
     const std::uint64_t k_rows = static_cast<std::uint64_t>(sequence_length) * batch_size;
-    params.q_lat = make_bf16_tile_map(query_latent, q_rows, RANK, RANK, ROWS);
-    params.q_rope = make_bf16_tile_map(query_rope, q_rows, ROPE, ROPE, ROWS);
-    params.d_out = make_bf16_tile_map(output_gradient, q_rows, RANK, RANK, ROWS);
-    params.k_lat = make_bf16_tile_map(kv_latent, k_rows, RANK, RANK, KEYS);
-    params.k_rope = make_bf16_tile_map(key_rope, k_rows, ROPE, ROPE, KEYS);
     params.dq_lat = dquery_latent;
     params.dq_rope = dquery_rope;
     params.dlatent = dkv_latent;
@@ -1162,9 +1170,9 @@ void mla_compressed_attention_backward_cuda(__nv_bfloat16* dquery_latent, __nv_b
     params.key_direct = part_count == key_tiles ? 1 : 0;
     params.key_lat8 = make_bf16_batched_chunked_map(kv_latent, batch_size, sequence_length, LATENT_CHUNKS, ks::CTA_KEYS, LATENT_CHUNKS);
     params.key_rope1 = make_bf16_batched_chunked_map(key_rope, batch_size, sequence_length, 1, ks::CTA_KEYS, 1);
-    params.row_q8 = make_bf16_batched_chunked_map(query_latent, batch_size, rows_per_sequence, LATENT_CHUNKS, ks::HALF_ROWS, LATENT_CHUNKS);
+    params.row_q4 = make_bf16_batched_chunked_map(query_latent, batch_size, rows_per_sequence, LATENT_CHUNKS, ks::HALF_ROWS, 4);
     params.row_q2 = make_bf16_batched_chunked_map(query_latent, batch_size, rows_per_sequence, LATENT_CHUNKS, ks::HALF_ROWS, 2);
-    params.row_do8 = make_bf16_batched_chunked_map(output_gradient, batch_size, rows_per_sequence, LATENT_CHUNKS, ks::HALF_ROWS, LATENT_CHUNKS);
+    params.row_do4 = make_bf16_batched_chunked_map(output_gradient, batch_size, rows_per_sequence, LATENT_CHUNKS, ks::HALF_ROWS, 4);
     params.row_do2 = make_bf16_batched_chunked_map(output_gradient, batch_size, rows_per_sequence, LATENT_CHUNKS, ks::HALF_ROWS, 2);
     params.row_rope = make_bf16_batched_chunked_map(query_rope, batch_size, rows_per_sequence, 1, ks::HALF_ROWS, 1);
     params.dlatent_out = make_bf16_batched_rows_map(dkv_latent, batch_size, sequence_length, RANK, 32);
@@ -1175,7 +1183,15 @@ void mla_compressed_attention_backward_cuda(__nv_bfloat16* dquery_latent, __nv_b
     if (params.key_direct == 0) {
         launch_chained(absorbed_backward_reduce_kernel, dim3(sequence_length, batch_size), dim3(144), 0, stream, params);
     }
-    const dim3 query_grid(static_cast<unsigned>((rows_per_sequence + ROWS - 1) / ROWS), 1, batch_size);
+    params.own_q8 = make_bf16_batched_chunked_map(query_latent, batch_size, rows_per_sequence, LATENT_CHUNKS, qs::CTA_ROWS, LATENT_CHUNKS);
+    params.own_rope = make_bf16_batched_chunked_map(query_rope, batch_size, rows_per_sequence, 1, qs::CTA_ROWS, 1);
+    params.own_do8 = make_bf16_batched_chunked_map(output_gradient, batch_size, rows_per_sequence, LATENT_CHUNKS, qs::CTA_ROWS, LATENT_CHUNKS);
+    params.stream_k4 = make_bf16_batched_chunked_map(kv_latent, batch_size, sequence_length, LATENT_CHUNKS, qs::HALF_KEYS, 4);
+    params.stream_k2 = make_bf16_batched_chunked_map(kv_latent, batch_size, sequence_length, LATENT_CHUNKS, qs::HALF_KEYS, 2);
+    params.stream_rope = make_bf16_batched_chunked_map(key_rope, batch_size, sequence_length, 1, qs::HALF_KEYS, 1);
+    params.dq_out = make_bf16_batched_rows_map(dquery_latent, batch_size, rows_per_sequence, RANK, 32);
+    params.dq_rope_out = make_bf16_batched_rows_map(dquery_rope, batch_size, rows_per_sequence, ROPE, 32);
+    const dim3 query_grid(static_cast<unsigned>(2 * ((rows_per_sequence + qs::TILE_ROWS - 1) / qs::TILE_ROWS)), 1, batch_size);
     launch_chained(absorbed_backward_query_kernel, query_grid, dim3(THREADS), qs::SMEM_BYTES, stream, params);
 }
 

@@ -147,6 +147,24 @@ def test_backward_tile_edges(gpu, b, t, h):
         torch.testing.assert_close(x.cpu().double(), ref.double(), atol=1e-2, rtol=1e-2)
 
 
+@pytest.mark.parametrize("t,h", [(50, 3), (130, 5)])
+def test_backward_keeps_batch_entries_apart(gpu, t, h):
+    """Tiles reach past the end of an entry (neither t nor t * h is a multiple of 48): what lies there, even NaN, must not matter."""
+    from dscuda_b200 import mla
+    generator = torch.Generator().manual_seed(t)
+    shapes = ((2, t, h, 512), (2, t, h, 64), (2, t, 512), (2, t, 64), (2, t, h, 512))
+    tensors = [(torch.randn(s, generator=generator) * .25).bfloat16().to(gpu) for s in shapes]
+    out, lse = mla.mla_forward(*tensors[:4], 576 ** -.5)
+    clean = mla.mla_backward(tensors[4], out, lse, *tensors[:4], 576 ** -.5)
+    for x in (*tensors, out, lse):
+        x[1] = float("nan")
+    poisoned = mla.mla_backward(tensors[4], out, lse, *tensors[:4], 576 ** -.5)
+    torch.cuda.synchronize()
+    assert mla.device_status() == 0
+    for x, y in zip(clean, poisoned):
+        assert torch.equal(x[0], y[0])
+
+
 def test_decode_empty_and_overlong_lengths(gpu):
     """Length 0: NaN output and -inf LSE, as the softmax of an empty row gives in the reference
     (reference/python/mla.py:36-38), whatever an earlier call left in the workspace.  A length above
