@@ -127,7 +127,8 @@ constexpr float PARTIAL_FINAL = -1.0F;
 
 struct Schedule {
     int chunk;          // 128-key tiles per cluster
-    int total;          // tiles of all units
+    int pad;            // tiles' worth of time that a change of unit costs, counted behind every unit
+    int total;          // tiles of all units, with their pads
     int first_unit;     // first unit that overlaps this cluster's range
     int first_offset;   // global tile index at which that unit starts
 };
@@ -253,7 +254,7 @@ __device__ __forceinline__ bool next_segment(const DecodeParams& p, const Schedu
         const int unit = w.unit;
         const int offset = w.offset;
         w.unit += 1;
-        w.offset += tiles;
+        w.offset += tiles > 0 ? tiles + s.pad : 0;
         if (end > begin) {
             seg.b = unit / head_tiles;
             seg.row_tile = unit % head_tiles;
@@ -272,16 +273,24 @@ __device__ __forceinline__ int decode_tiles(const DecodeParams& p, int b) {
     return (sequence_length<false>(p, b) + TILE_KEYS - 1) / TILE_KEYS;
 }
 
+// Finishing one unit and starting the next (results out, Q in, the pipeline empty) takes a cluster about as long as two
+// tiles, so every unit counts two tiles more than it has, and a range of many short sequences holds fewer tiles.  Without
+// the pad the slowest cluster of 32 sequences of 2-32 tiles had 7 tiles in three segments beside clusters with 7 in one:
+// 53.1 -> 47.6 us with it; 8 sequences of up to 8192 tokens 27.0 -> 22.8.  Where one tile per cluster is enough there is
+// nothing to balance, and a pad would make ranges of two tiles.
+constexpr int UNIT_PAD = 2;
+
 // The cut of the list of tiles and where this cluster's range starts (splits > 1), by one warp.  A lane takes every 32nd
 // sequence, so the lengths are loaded 32 at a time: one thread walking the list paid an L2 round trip per sequence (6-8 us
 // of every decode call at 74 sequences).
 __device__ __forceinline__ Schedule cut_schedule(const DecodeParams& p, int cluster, int clusters, int lane) {
     const int head_tiles = (p.heads + PAIR_HEADS - 1) / PAIR_HEADS;
+    constexpr int COUNT_SHIFT = 44;             // sequences with tiles are counted above the tiles (fewer than 2^24 * 2^16)
     long long total = 0;
     int longest = 0;
     for (int b = lane; b < p.batch; b += 32) {
         const int tiles = decode_tiles(p, b);
-        total += tiles;
+        total += tiles > 0 ? (1LL << COUNT_SHIFT) + tiles : 0;
         longest = max(longest, tiles);
     }
 #pragma unroll
@@ -289,11 +298,15 @@ __device__ __forceinline__ Schedule cut_schedule(const DecodeParams& p, int clus
         total += __shfl_xor_sync(0xffffffffU, total, offset);
         longest = max(longest, __shfl_xor_sync(0xffffffffU, longest, offset));
     }
-    total *= head_tiles;
+    const long long sequences = total >> COUNT_SHIFT;
+    total &= (1LL << COUNT_SHIFT) - 1;
+    const int pad = total * head_tiles > clusters ? UNIT_PAD : 0;
+    total = (total + sequences * pad) * head_tiles;
     long long chunk = (total + clusters - 1) / clusters;
     chunk = max(chunk, static_cast<long long>((longest + p.splits - 2) / (p.splits - 1)));
     chunk = max(chunk, 1LL);
     Schedule schedule;
+    schedule.pad = pad;
     schedule.chunk = static_cast<int>(min(chunk, 0x7fffffffLL));
     schedule.total = static_cast<int>(min(total, 0x7fffffffLL));
     schedule.first_unit = p.batch * head_tiles;
@@ -303,7 +316,8 @@ __device__ __forceinline__ Schedule cut_schedule(const DecodeParams& p, int clus
     long long start = 0;                        // global tile index of sequence `base`
     for (int base = 0; base < p.batch; base += 32) {
         const int tiles = base + lane < p.batch ? decode_tiles(p, base + lane) : 0;
-        long long end = static_cast<long long>(tiles) * head_tiles;
+        const int length = tiles > 0 ? tiles + pad : 0;
+        long long end = static_cast<long long>(length) * head_tiles;
 #pragma unroll
         for (int offset = 1; offset < 32; offset <<= 1) {
             const long long before = __shfl_up_sync(0xffffffffU, end, offset);
@@ -312,11 +326,11 @@ __device__ __forceinline__ Schedule cut_schedule(const DecodeParams& p, int clus
         const unsigned past = __ballot_sync(0xffffffffU, start + end > lo);
         if (past != 0U) {
             const int which = __ffs(static_cast<int>(past)) - 1;
-            const int tiles_there = __shfl_sync(0xffffffffU, tiles, which);
-            const long long begin = start + __shfl_sync(0xffffffffU, end, which) - static_cast<long long>(tiles_there) * head_tiles;
-            const int head_tile = static_cast<int>((lo - begin) / tiles_there);
+            const int length_there = __shfl_sync(0xffffffffU, length, which);
+            const long long begin = start + __shfl_sync(0xffffffffU, end, which) - static_cast<long long>(length_there) * head_tiles;
+            const int head_tile = static_cast<int>((lo - begin) / length_there);
             schedule.first_unit = (base + which) * head_tiles + head_tile;
-            schedule.first_offset = static_cast<int>(begin + static_cast<long long>(head_tile) * tiles_there);
+            schedule.first_offset = static_cast<int>(begin + static_cast<long long>(head_tile) * length_there);
             break;
         }
         start += __shfl_sync(0xffffffffU, end, 31);
@@ -381,7 +395,7 @@ __device__ __forceinline__ void absorbed_pair_body(const DecodeParams& p) {
     }
     if (warp == 0) {
         grid_dependency_wait();         // the lengths may come from the kernel in front
-        const Schedule schedule = CAUSAL || p.splits == 1 ? Schedule{1, 0, 0, 0} : cut_schedule(p, cluster, clusters, lane);
+        const Schedule schedule = CAUSAL || p.splits == 1 ? Schedule{1, 0, 0, 0, 0} : cut_schedule(p, cluster, clusters, lane);
         if (lane == 0) {
             sh->schedule = schedule;
         }

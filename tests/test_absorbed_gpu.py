@@ -74,6 +74,22 @@ def test_decode_permuted_pages_and_garbage_tail(gpu, batch, heads, low, high, sp
     assert float((lse.cpu() - ref_lse).abs().max()) <= 1e-3
 
 
+@pytest.mark.parametrize("batch,heads,low,high,splits", [(74, 16, 1, 128, 8), (75, 16, 1, 128, 8), (120, 16, 1, 400, 2), (40, 130, 100, 900, 8), (9, 128, 1, 3000, 3)])
+def test_decode_schedule_of_short_sequences(gpu, batch, heads, low, high, splits):
+    """Ranges around one tile per cluster (74 sequences of one tile), many sequences to a range, a range that starts behind a sequence's last
+    tile, two 128-head tiles to a sequence, few partial slots; every fifth sequence is empty."""
+    from dscuda_b200 import mla
+    query, cache, table, lengths = oracle.decode_inputs(seed=batch + heads, batch=batch, heads=heads, low=low, high=high)
+    ref_out, ref_lse = oracle.paged_decode(query, cache, table, lengths, 192 ** -.5)
+    empty = torch.arange(batch) % 5 == 4
+    out, lse = mla.mla_decode(query.to(gpu), cache.to(gpu), table.to(gpu), torch.where(empty, 0, lengths).int().to(gpu), 192 ** -.5, splits=splits)
+    torch.cuda.synchronize()
+    assert mla.device_status() == 0
+    assert max_err_ratio(out.cpu().float()[~empty], ref_out[~empty]) <= 1e-2
+    assert float((lse.cpu() - ref_lse)[~empty].abs().max()) <= 1e-3
+    assert bool(torch.isnan(out.cpu()[empty]).all()) and bool((lse.cpu()[empty] == float("-inf")).all())
+
+
 def test_decode_rejects_bad_arguments(gpu):
     from dscuda_b200 import mla
     g = load_golden("decode_b2_t23_h3")
