@@ -167,12 +167,12 @@ __global__ void __launch_bounds__(256) absorbed_delta_kernel(__nv_bfloat16* dq_r
 // chain scores -> softmax -> gradients of a tile is overlapped only by the loads of the next one: a column half of an operand
 // is loaded again as soon as its gradient product has read it.  96 rows and not 128 because 128 do not fit.  One CTA per (128 keys, half of dlatent), which this
 // replaces, computed the scores twice, at the N = 64 rate: 1305 us at B=4 T=2048 H=16 against
-// 580 us now, 46 against 11 us at B=2 T=33 H=32 (where a part also had at least 1024 rows).
+// 550 us now, 46 against 11 us at B=2 T=33 H=32 (where a part also had at least 1024 rows).
 //
 // Tensor memory: dlatent 2 x 128 columns (lanes 0-63: columns 256a + 0..127, lanes 64-127: 256a + 128..255 of the same 64
 // keys), dkey_rope 64, S^T 48 (lanes 64-127: rows 48..95), dP^T 48.
-// Warps 0-7: softmax (thread = key x 24 rows) and results; 8: MMA issue in the leader, relay of "loaded" events in the other
-// CTA; 9: TMA loads; 10: the rows' constants.
+// Warps 0-7: softmax (thread = key x 24 rows) and results; 8: MMA issue in the leader; 9: TMA loads (the other CTA's signal the
+// leader's barriers); 10: the rows' constants.
 // ---------------------------------------------------------------------------
 namespace ks {
 constexpr int TILE_ROWS = KEY_SIDE_ROWS;
@@ -208,18 +208,12 @@ struct Rows {
 
 struct Shared {
     Rows rows[2];
-    // completed by TMA transactions of this CTA, one phase per tile
+    // leader only: completed by the TMA transactions of both CTAs, one phase per tile
     uint64_t k_full;
     uint64_t q_full[2];         // own rows of query_latent, by column half; the rotary chunk with half 0
     uint64_t do_full[2];        // own rows of dO
     uint64_t q_refilled[2];     // the other CTA's rows; the rotary columns of all rows with half 0
     uint64_t do_refilled[2];
-    // leader only: the same events of the other CTA, forwarded by its relay (one arrival)
-    uint64_t peer_k_full;
-    uint64_t peer_q_full[2];
-    uint64_t peer_do_full[2];
-    uint64_t peer_q_refilled[2];
-    uint64_t peer_do_refilled[2];
     // completed by tcgen05.commit of the leader
     uint64_t q_refill_free[2];  // S has read the half; half 1: S is complete
     uint64_t do_refill_free[2]; // dP^T likewise
@@ -304,12 +298,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ks::KEY_THREADS, 1) 
     if (warp == LOAD_WARP) {
         // =================== TMA producer ===================================
         if (lane == 0) {
+            // the bytes of both CTAs are counted by the leader's barrier
+            auto expect = [&](uint64_t* leaders, uint32_t bytes) {
+                if (rank == 0) {
+                    mbar_arrive_expect_tx(smem_u32(leaders), 2 * bytes);
+                }
+                return map_to_cta(smem_u32(leaders), 0);
+            };
             const int own = static_cast<int>(rank) * HALF_ROWS, other = HALF_ROWS - own;
             const int own_chunk = 2 * static_cast<int>(rank), other_slot = 2 - own_chunk;
-            uint32_t bar = smem_u32(&sh->k_full);
-            mbar_arrive_expect_tx(bar, K_BYTES);
-            tma_load_4d(smem_base, &p.key_lat8, bar, 0, key_start + static_cast<int>(rank) * CTA_KEYS, 0, b);
-            tma_load_4d(smem_base + LATENT_CHUNKS * KEY_SLOT, &p.key_rope1, bar, 0, key_start + static_cast<int>(rank) * CTA_KEYS, 0, b);
+            uint32_t bar = expect(&sh->k_full, K_BYTES);
+            tma_load_4d_pair(smem_base, &p.key_lat8, bar, 0, key_start + static_cast<int>(rank) * CTA_KEYS, 0, b);
+            tma_load_4d_pair(smem_base + LATENT_CHUNKS * KEY_SLOT, &p.key_rope1, bar, 0, key_start + static_cast<int>(rank) * CTA_KEYS, 0, b);
             bool alive = true;
             for (int t = 0; t < tile_count && alive; ++t) {
                 const int row0 = first_row + t * TILE_ROWS;
@@ -318,25 +318,23 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ks::KEY_THREADS, 1) 
                     const int a = i & 1;
                     alive = t == 0 || wait(i < 2 ? sh->q_free[a] : sh->do_free[a], t - 1);
                     if (alive) {
-                        bar = smem_u32(i < 2 ? &sh->q_full[a] : &sh->do_full[a]);
-                        mbar_arrive_expect_tx(bar, (i == 0 ? 5 : 4) * ROW_SLOT);
+                        bar = expect(i < 2 ? &sh->q_full[a] : &sh->do_full[a], (i == 0 ? 5 : 4) * ROW_SLOT);
                         if (i == 0) {
-                            tma_load_4d(smem_base + ROPE_OFFSET, &p.row_rope, bar, 0, row0 + own, 0, b);
+                            tma_load_4d_pair(smem_base + ROPE_OFFSET, &p.row_rope, bar, 0, row0 + own, 0, b);
                         }
-                        tma_load_4d(smem_base + (i < 2 ? Q_OFFSET : DO_OFFSET) + 4 * a * ROW_SLOT, i < 2 ? &p.row_q4 : &p.row_do4, bar, 0, row0 + own, 4 * a, b);
+                        tma_load_4d_pair(smem_base + (i < 2 ? Q_OFFSET : DO_OFFSET) + 4 * a * ROW_SLOT, i < 2 ? &p.row_q4 : &p.row_do4, bar, 0, row0 + own, 4 * a, b);
                     }
                 }
                 for (int i = 0; i < 4 && alive; ++i) {
                     const int a = i & 1;
                     alive = wait(i < 2 ? sh->q_refill_free[a] : sh->do_refill_free[a], t);
                     if (alive) {
-                        bar = smem_u32(i < 2 ? &sh->q_refilled[a] : &sh->do_refilled[a]);
-                        mbar_arrive_expect_tx(bar, (i == 0 ? 4 : 2) * ROW_SLOT);
-                        tma_load_4d(smem_base + (i < 2 ? Q_OFFSET : DO_OFFSET) + (4 * a + other_slot) * ROW_SLOT, i < 2 ? &p.row_q2 : &p.row_do2, bar, 0, row0 + other,
+                        bar = expect(i < 2 ? &sh->q_refilled[a] : &sh->do_refilled[a], (i == 0 ? 4 : 2) * ROW_SLOT);
+                        tma_load_4d_pair(smem_base + (i < 2 ? Q_OFFSET : DO_OFFSET) + (4 * a + other_slot) * ROW_SLOT, i < 2 ? &p.row_q2 : &p.row_do2, bar, 0, row0 + other,
                                     4 * a + own_chunk, b);
                         if (i == 0) {
-                            tma_load_4d(smem_base + ROPE_ALL_OFFSET, &p.row_rope, bar, 0, row0, 0, b);
-                            tma_load_4d(smem_base + ROPE_ALL_OFFSET + ROW_SLOT, &p.row_rope, bar, 0, row0 + HALF_ROWS, 0, b);
+                            tma_load_4d_pair(smem_base + ROPE_ALL_OFFSET, &p.row_rope, bar, 0, row0, 0, b);
+                            tma_load_4d_pair(smem_base + ROPE_ALL_OFFSET + ROW_SLOT, &p.row_rope, bar, 0, row0 + HALF_ROWS, 0, b);
                         }
                     }
                 }
@@ -369,27 +367,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ks::KEY_THREADS, 1) 
                 mbar_arrive(smem_u32(&sh->rows_ready[t & 1]));
             }
         }
-    } else if (warp == MMA_WARP && rank != 0) {
-        // =================== relay: this CTA's "loaded" events -> the leader =========
-        if (lane == 0) {
-            bool alive = wait(sh->k_full, 0);
-            if (alive) {
-                mbar_arrive_remote(map_to_cta(smem_u32(&sh->peer_k_full), 0));
-            }
-            for (int t = 0; t < tile_count && alive; ++t) {
-                // in the order in which they are loaded
-                uint64_t* const mine[4] = {sh->q_full, sh->do_full, sh->q_refilled, sh->do_refilled};
-                uint64_t* const leaders[4] = {sh->peer_q_full, sh->peer_do_full, sh->peer_q_refilled, sh->peer_do_refilled};
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    alive = alive && wait(mine[i / 2][i & 1], t);
-                    if (alive) {
-                        mbar_arrive_remote(map_to_cta(smem_u32(&leaders[i / 2][i & 1]), 0));
-                    }
-                }
-            }
-        }
-    } else if (warp == MMA_WARP) {
+    } else if (warp == MMA_WARP && rank == 0) {
         // =================== MMA issuer (leader CTA; whole warp, elected lane executes) ==
         const uint32_t leader = elect_one();
         constexpr uint32_t IDESC_SCORE = make_idesc_bf16(KEYS, TILE_ROWS, false, false);
@@ -427,15 +405,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ks::KEY_THREADS, 1) 
                                   leader);
             }
         };
-        auto wait_both = [&](uint64_t& mine, uint64_t& others, int phase) {
-            const bool alive = __all_sync(0xffffffffU, wait(mine, phase) && wait(others, phase));
+        auto wait_loaded = [&](uint64_t& bar, int phase) {
+            const bool alive = __all_sync(0xffffffffU, wait(bar, phase));
             tc_fence_after_sync();
             return alive;
         };
-        bool alive = wait_both(sh->k_full, sh->peer_k_full, 0);
+        bool alive = wait_loaded(sh->k_full, 0);
         for (int t = 0; t < tile_count && alive; ++t) {
             for (int a = 0; a < 2 && alive; ++a) {
-                alive = wait_both(sh->q_full[a], sh->peer_q_full[a], t);
+                alive = wait_loaded(sh->q_full[a], t);
                 if (!alive) {
                     break;
                 }
@@ -450,7 +428,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ks::KEY_THREADS, 1) 
                 both(&sh->q_refill_free[a]);
             }
             for (int a = 0; a < 2 && alive; ++a) {
-                alive = wait_both(sh->do_full[a], sh->peer_do_full[a], t);
+                alive = wait_loaded(sh->do_full[a], t);
                 if (!alive) {
                     break;
                 }
@@ -459,7 +437,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ks::KEY_THREADS, 1) 
             }
             alive = alive && __all_sync(0xffffffffU, wait(sh->p_full, t));
             for (int a = 0; a < 2 && alive; ++a) {
-                alive = wait_both(sh->q_refilled[a], sh->peer_q_refilled[a], t);
+                alive = wait_loaded(sh->q_refilled[a], t);
                 if (!alive) {
                     break;
                 }
@@ -474,7 +452,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ks::KEY_THREADS, 1) 
                 both(&sh->q_free[a]);
             }
             for (int a = 0; a < 2 && alive; ++a) {
-                alive = wait_both(sh->do_refilled[a], sh->peer_do_refilled[a], t);
+                alive = wait_loaded(sh->do_refilled[a], t);
                 if (!alive) {
                     break;
                 }
@@ -482,7 +460,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ks::KEY_THREADS, 1) 
                 both(&sh->do_free[a]);
             }
         }
-    } else {
+    } else if (warp < MMA_WARP) {
         // =================== softmax: thread = (key, 24 of the 96 rows) ======
         const int tmem_lane = (warp % 4) * 32 + lane;
         const int key_in_cta = tmem_lane & 63;
@@ -689,7 +667,7 @@ __global__ void __launch_bounds__(144) absorbed_backward_reduce_kernel(const __g
 // What bounds it: the chain of a tile, as on the key side.  64 rows of one CTA with 128-key tiles, which this replaces, ran
 // at the N = 64 rate and streamed every key tile twice (288 KB for 64 x 128 pairs, L2 latency over two 32 KB slots; here
 // 84 KB for 64 x 96): 680 us at B=4 T=2048 H=16 against
-// 520 us now.
+// 497 us now.
 //
 // Tensor memory and warps as on the key side; a softmax thread owns 24 keys of one row, so LSE, delta and token are its own.
 // ---------------------------------------------------------------------------
@@ -719,14 +697,10 @@ static_assert(SMEM_BYTES <= 232448, "query-side shared memory");
 static_assert(8 * 3 * SLAB_BYTES <= MISC_OFFSET, "result slabs lie in the operands' memory");
 
 struct Shared {
-    // completed by TMA transactions of this CTA; the arrays by column half
+    // leader only: completed by the TMA transactions of both CTAs; the arrays by column half
     uint64_t rows_full;
     uint64_t k_full[2];             // own keys (the rotary chunk with half 0)
     uint64_t refilled[2];           // the other CTA's keys (the rotary columns of all keys with half 0)
-    // leader only: the same events of the other CTA, forwarded by its relay (one arrival)
-    uint64_t peer_rows_full;
-    uint64_t peer_k_full[2];
-    uint64_t peer_refilled[2];
     // completed by tcgen05.commit of the leader
     uint64_t refill_free[2];        // both score products have read the half; half 1: dP is complete
     uint64_t s_full;
@@ -794,59 +768,46 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) absorbed
     if (warp == LOAD_WARP) {
         // =================== TMA producer ===================================
         if (lane == 0) {
+            // the bytes of both CTAs are counted by the leader's barrier
+            auto expect = [&](uint64_t* leaders, uint32_t bytes) {
+                if (rank == 0) {
+                    mbar_arrive_expect_tx(smem_u32(leaders), 2 * bytes);
+                }
+                return map_to_cta(smem_u32(leaders), 0);
+            };
             const int own = static_cast<int>(rank) * HALF_KEYS, other = HALF_KEYS - own;
             const int own_chunk = 2 * static_cast<int>(rank), other_slot = 2 - own_chunk;
-            uint32_t bar = smem_u32(&sh->rows_full);
-            mbar_arrive_expect_tx(bar, Q_BYTES + DO_BYTES);
-            tma_load_4d(smem_base, &p.own_q8, bar, 0, own_row0, 0, b);
-            tma_load_4d(smem_base + LATENT_CHUNKS * ROW_SLOT, &p.own_rope, bar, 0, own_row0, 0, b);
-            tma_load_4d(smem_base + DO_OFFSET, &p.own_do8, bar, 0, own_row0, 0, b);
+            uint32_t bar = expect(&sh->rows_full, Q_BYTES + DO_BYTES);
+            tma_load_4d_pair(smem_base, &p.own_q8, bar, 0, own_row0, 0, b);
+            tma_load_4d_pair(smem_base + LATENT_CHUNKS * ROW_SLOT, &p.own_rope, bar, 0, own_row0, 0, b);
+            tma_load_4d_pair(smem_base + DO_OFFSET, &p.own_do8, bar, 0, own_row0, 0, b);
             bool alive = true;
             for (int j = 0; j < tile_count && alive; ++j) {
                 const int key0 = j * TILE_KEYS;
                 for (int a = 0; a < 2 && alive; ++a) {
                     alive = j == 0 || wait(sh->k_free[a], j - 1);
                     if (alive) {
-                        bar = smem_u32(&sh->k_full[a]);
-                        mbar_arrive_expect_tx(bar, (a == 0 ? 5 : 4) * KEY_SLOT);
+                        bar = expect(&sh->k_full[a], (a == 0 ? 5 : 4) * KEY_SLOT);
                         if (a == 0) {
-                            tma_load_4d(smem_base + ROPE_OFFSET, &p.stream_rope, bar, 0, key0 + own, 0, b);
+                            tma_load_4d_pair(smem_base + ROPE_OFFSET, &p.stream_rope, bar, 0, key0 + own, 0, b);
                         }
-                        tma_load_4d(smem_base + K_OFFSET + 4 * a * KEY_SLOT, &p.stream_k4, bar, 0, key0 + own, 4 * a, b);
+                        tma_load_4d_pair(smem_base + K_OFFSET + 4 * a * KEY_SLOT, &p.stream_k4, bar, 0, key0 + own, 4 * a, b);
                     }
                 }
                 for (int a = 0; a < 2 && alive; ++a) {
                     alive = wait(sh->refill_free[a], j);
                     if (alive) {
-                        bar = smem_u32(&sh->refilled[a]);
-                        mbar_arrive_expect_tx(bar, (a == 0 ? 4 : 2) * KEY_SLOT);
-                        tma_load_4d(smem_base + K_OFFSET + (4 * a + other_slot) * KEY_SLOT, &p.stream_k2, bar, 0, key0 + other, 4 * a + own_chunk, b);
+                        bar = expect(&sh->refilled[a], (a == 0 ? 4 : 2) * KEY_SLOT);
+                        tma_load_4d_pair(smem_base + K_OFFSET + (4 * a + other_slot) * KEY_SLOT, &p.stream_k2, bar, 0, key0 + other, 4 * a + own_chunk, b);
                         if (a == 0) {
-                            tma_load_4d(smem_base + ROPE_ALL_OFFSET, &p.stream_rope, bar, 0, key0, 0, b);
-                            tma_load_4d(smem_base + ROPE_ALL_OFFSET + KEY_SLOT, &p.stream_rope, bar, 0, key0 + HALF_KEYS, 0, b);
+                            tma_load_4d_pair(smem_base + ROPE_ALL_OFFSET, &p.stream_rope, bar, 0, key0, 0, b);
+                            tma_load_4d_pair(smem_base + ROPE_ALL_OFFSET + KEY_SLOT, &p.stream_rope, bar, 0, key0 + HALF_KEYS, 0, b);
                         }
                     }
                 }
             }
         }
-    } else if (warp == MMA_WARP && rank != 0) {
-        // =================== relay: this CTA's "loaded" events -> the leader, in the order in which they are loaded =========
-        if (lane == 0) {
-            bool alive = wait(sh->rows_full, 0);
-            if (alive) {
-                mbar_arrive_remote(map_to_cta(smem_u32(&sh->peer_rows_full), 0));
-            }
-            for (int j = 0; j < tile_count && alive; ++j) {
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    alive = alive && wait(i < 2 ? sh->k_full[i & 1] : sh->refilled[i & 1], j);
-                    if (alive) {
-                        mbar_arrive_remote(map_to_cta(smem_u32(i < 2 ? &sh->peer_k_full[i & 1] : &sh->peer_refilled[i & 1]), 0));
-                    }
-                }
-            }
-        }
-    } else if (warp == MMA_WARP) {
+    } else if (warp == MMA_WARP && rank == 0) {
         // =================== MMA issuer (leader CTA; whole warp, elected lane executes) ==
         const uint32_t leader = elect_one();
         constexpr uint32_t IDESC_SCORE = make_idesc_bf16(TILE_ROWS, TILE_KEYS, false, false);
@@ -874,14 +835,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) absorbed
                 }
             }
         };
-        auto wait_both = [&](uint64_t& mine, uint64_t& others, int phase) {
-            const bool alive = __all_sync(0xffffffffU, wait(mine, phase) && wait(others, phase));
+        auto wait_loaded = [&](uint64_t& bar, int phase) {
+            const bool alive = __all_sync(0xffffffffU, wait(bar, phase));
             tc_fence_after_sync();
             return alive;
         };
-        bool alive = wait_both(sh->rows_full, sh->peer_rows_full, 0);
+        bool alive = wait_loaded(sh->rows_full, 0);
         for (int j = 0; j < tile_count && alive; ++j) {
-            alive = wait_both(sh->k_full[0], sh->peer_k_full[0], j);
+            alive = wait_loaded(sh->k_full[0], j);
             if (!alive) {
                 break;
             }
@@ -893,7 +854,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) absorbed
             issue_scores(tmem_base + TMEM_S, q_lo, 0, false);
             issue_scores(tmem_base + TMEM_DP, do_lo, 0, true);
             both(&sh->refill_free[0]);
-            alive = wait_both(sh->k_full[1], sh->peer_k_full[1], j);
+            alive = wait_loaded(sh->k_full[1], j);
             if (!alive) {
                 break;
             }
@@ -903,7 +864,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) absorbed
             both(&sh->refill_free[1]);
             alive = __all_sync(0xffffffffU, wait(sh->ds_full, j));
             for (int a = 0; a < 2 && alive; ++a) {
-                alive = wait_both(sh->refilled[a], sh->peer_refilled[a], j);
+                alive = wait_loaded(sh->refilled[a], j);
                 if (!alive) {
                     break;
                 }
@@ -924,7 +885,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) absorbed
                 both(&sh->k_free[a]);
             }
         }
-    } else {
+    } else if (warp < MMA_WARP) {
         // =================== softmax: thread = (row, 24 of the 96 keys) ======
         const int tmem_lane = (warp % 4) * 32 + lane;
         const int row_in_cta = tmem_lane & 63;
