@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(256) absorbed_delta_kernel(__nv_bfloat16* dq_r
 // chain scores -> softmax -> gradients of a tile is overlapped only by the loads of the next one: a column half of an operand
 // is loaded again as soon as its gradient product has read it.  96 rows and not 128 because 128 do not fit.  One CTA per (128 keys, half of dlatent), which this
 // replaces, computed the scores twice, at the N = 64 rate: 1305 us at B=4 T=2048 H=16 against
-// 550 us now, 46 against 11 us at B=2 T=33 H=32 (where a part also had at least 1024 rows).
+// 532 us now, 46 against 11 us at B=2 T=33 H=32 (where a part also had at least 1024 rows).
 //
 // Tensor memory: dlatent 2 x 128 columns (lanes 0-63: columns 256a + 0..127, lanes 64-127: 256a + 128..255 of the same 64
 // keys), dkey_rope 64, S^T 48 (lanes 64-127: rows 48..95), dP^T 48.
@@ -217,7 +217,7 @@ struct Shared {
     // completed by tcgen05.commit of the leader
     uint64_t q_refill_free[2];  // S has read the half; half 1: S is complete
     uint64_t do_refill_free[2]; // dP^T likewise
-    uint64_t q_free[2];         // dS^T Q has read the half (half 0: and query_rope)
+    uint64_t q_free[2];         // dS^T Q has read the half
     uint64_t do_free[2];        // P^T dO has read the half; half 1: P, dS and the accumulators are quiescent
     // leader only: one arrival per softmax warp of either CTA, P^T and dS^T are stored
     uint64_t p_full;
@@ -442,14 +442,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ks::KEY_THREADS, 1) 
                     break;
                 }
                 issue_gradients(ds_lo, smem_base + Q_OFFSET, a, t == 0);
-                if (a == 0) {
+                both(&sh->q_free[a]);           // before dkey_rope: the next tile's scores wait for this load
+            }
+            if (!alive) {
+                break;
+            }
 #pragma unroll
-                    for (int kk = 0; kk < 6; ++kk) {
-                        mma_pair_ss_split(tmem_base + TMEM_DROPE, ds_lo + (kk >> 2) * (KEY_SLOT >> 4) + 2 * (kk & 3), HI,
-                                          rope_all_lo + (kk / 3) * (ROW_SLOT >> 4) + (kk % 3) * (2048 >> 4), HI, IDESC_ROPE, (t | kk) != 0 ? 1U : 0U, leader);
-                    }
-                }
-                both(&sh->q_free[a]);
+            for (int kk = 0; kk < 6; ++kk) {
+                mma_pair_ss_split(tmem_base + TMEM_DROPE, ds_lo + (kk >> 2) * (KEY_SLOT >> 4) + 2 * (kk & 3), HI,
+                                  rope_all_lo + (kk / 3) * (ROW_SLOT >> 4) + (kk % 3) * (2048 >> 4), HI, IDESC_ROPE, (t | kk) != 0 ? 1U : 0U, leader);
             }
             for (int a = 0; a < 2 && alive; ++a) {
                 alive = wait_loaded(sh->do_refilled[a], t);
@@ -667,7 +668,7 @@ __global__ void __launch_bounds__(144) absorbed_backward_reduce_kernel(const __g
 // What bounds it: the chain of a tile, as on the key side.  64 rows of one CTA with 128-key tiles, which this replaces, ran
 // at the N = 64 rate and streamed every key tile twice (288 KB for 64 x 128 pairs, L2 latency over two 32 KB slots; here
 // 84 KB for 64 x 96): 680 us at B=4 T=2048 H=16 against
-// 497 us now.
+// 483 us now.
 //
 // Tensor memory and warps as on the key side; a softmax thread owns 24 keys of one row, so LSE, delta and token are its own.
 // ---------------------------------------------------------------------------
@@ -875,6 +876,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) absorbed
                                       column_lo + (4 * a + 2 * (kk / 3)) * (KEY_SLOT >> 4) + (kk % 3) * (2048 >> 4), HI, IDESC_GRAD, (j | kk) != 0 ? 1U : 0U,
                                       leader);
                 }
+                both(&sh->k_free[a]);           // before dquery_rope: the next tile's scores wait for this load
                 if (a == 0) {
 #pragma unroll
                     for (int kk = 0; kk < 6; ++kk) {
@@ -882,7 +884,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) absorbed
                                           rope_all_lo + (kk / 3) * (KEY_SLOT >> 4) + (kk % 3) * (2048 >> 4), HI, IDESC_ROPE, (j | kk) != 0 ? 1U : 0U, leader);
                     }
                 }
-                both(&sh->k_free[a]);
             }
         }
     } else if (warp < MMA_WARP) {
