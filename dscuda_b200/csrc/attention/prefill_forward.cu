@@ -16,8 +16,8 @@
 // Warp roles (384 threads): warps 0-3 softmax/epilogue of tile 0, warps 4-7 of
 // tile 1, warp 8 issues every MMA (the whole warp runs the loop, one elected
 // lane executes the instruction), warp 9 issues every TMA load from one thread,
-// warps 10-11 only complete the third warpgroup so that it can hand registers
-// to the softmax warps.  All waits are bounded; a wait that runs out raises the
+// warps 10-11 complete the third warpgroup, so that it can hand registers to the
+// softmax warps, and clear the values behind the end of a packed sequence.  All waits are bounded; a wait that runs out raises the
 // device status word and the CTA tears down normally (tensor memory freed).
 #include "mla.h"
 #include "flash_attention.h"
@@ -39,9 +39,10 @@ constexpr int TILE_N = 128;                 // keys per K/V tile
 constexpr int HEAD_V = 128;                 // value width
 constexpr int CHUNK_BYTES = 16384;          // [128 rows x 64 bf16] or [64 keys x 128 bf16]
 constexpr int V_CHUNKS = TILE_N / 64;       // V tile = 2 chunks of 64 keys
-constexpr int FORWARD_THREADS = 384;     // warps 10 and 11 only complete the third warpgroup for setmaxnreg
+constexpr int FORWARD_THREADS = 384;     // warps 10 and 11 complete the third warpgroup for setmaxnreg
 constexpr int MMA_WARP = 8;
 constexpr int LOAD_WARP = 9;
+constexpr int TAIL_WARP = 10;               // and 11: one for each 64 keys of a V tile
 constexpr int TMEM_COLUMNS = 512;           // S0 | S1 | O0 | O1, 128 columns each
 constexpr int MISC_BYTES = 1024;
 constexpr float RESCALE_THRESHOLD = 8.0F;   // log2 units; below it the old row maximum is kept
@@ -49,6 +50,7 @@ constexpr float RESCALE_THRESHOLD = 8.0F;   // log2 units; below it the old row 
 __device__ int forward_status = 0;
 
 struct ForwardParams {
+    // dense: a batch of S rows each; packed: one entry of all rows
     CUtensorMap q_main;     // [rows, Hq*128], box 128 x 64
     CUtensorMap q_pe;       // [rows, Hq*64],  box 128 x 64 (unused when KQ == 2)
     CUtensorMap k_main;     // [rows, Hkv*128], box 128 x 64
@@ -83,6 +85,7 @@ struct ForwardBarriers {
     uint64_t p_half[2];        // the first 64 keys of P are stored: the first half of P V may start
     uint64_t ring_full[10];
     uint64_t ring_empty[10];
+    uint64_t tail_full[2];     // a last V tile that contains another sequence's rows: its halves have landed
     uint32_t tmem_base;
     int abort_flag;
 };
@@ -140,6 +143,10 @@ __global__ void __launch_bounds__(FORWARD_THREADS, 1) attention_forward_kernel(c
     const int tiles[2] = {q_start / TILE_N + 1, (q_start + TILE_M < length) ? q_start / TILE_N + 2 : 0};
     const int tile_count = tiles[1] > 0 ? tiles[1] : tiles[0];
     const int kv_head = head / p.group;
+    // Rows of a tile behind the end of the sequence: of a batch entry they load as zero, of a packed sequence they are the next one's.
+    const int entry = p.cu_seqlens == nullptr ? static_cast<int>(blockIdx.z) : 0;
+    const int entry_row0 = p.cu_seqlens == nullptr ? 0 : row0;
+    const int tail_keys = p.cu_seqlens != nullptr && row0 + length < p.total ? length - (tile_count - 1) * TILE_N : TILE_N;
 
     // ---- shared memory carve-up -------------------------------------------
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023U) & ~1023U;
@@ -157,6 +164,7 @@ __global__ void __launch_bounds__(FORWARD_THREADS, 1) attention_forward_kernel(c
             mbar_init(smem_u32(&bars->s_full[i]), 1);
             mbar_init(smem_u32(&bars->p_full[i]), TILE_M);
             mbar_init(smem_u32(&bars->p_half[i]), TILE_M);
+            mbar_init(smem_u32(&bars->tail_full[i]), 1);
         }
         for (int i = 0; i < L::RING; ++i) {
             mbar_init(smem_u32(&bars->ring_full[i]), 1);
@@ -194,51 +202,69 @@ __global__ void __launch_bounds__(FORWARD_THREADS, 1) attention_forward_kernel(c
     // cover what warps 0-7 request, or the kernel never starts (launch allocation: 168 each).
     static_assert(8 * (REG_HI - 168) <= 4 * (168 - REG_LO), "register redistribution exceeds the CTA's allocation");
     if (warp >= 8) {
-        reg_dealloc<REG_LO>();      // one instruction for the whole warpgroup; warps 10 and 11 do nothing else
-        if (warp == LOAD_WARP) {
+        reg_dealloc<REG_LO>();      // one instruction for the whole warpgroup
+        if (warp >= TAIL_WARP) {
+            // =================== values behind the end of a packed sequence =====
+            // The softmax masks the scores of such keys, but P V multiplies their values by P = 0.
+            if (tail_keys < TILE_N) {
+                const int half = warp - TAIL_WARP;
+                if (__all_sync(0xffffffffU, mbar_wait(smem_u32(&bars->tail_full[half]), 0, abort_flag, &forward_status))) {
+                    const int slot = ((tile_count - 1) * L::PER_TILE + KQ + half) % L::RING;
+                    uint8_t* chunk = smem_raw + (ring_smem - smem_u32(smem_raw)) + slot * CHUNK_BYTES;
+                    const int first = min(max(tail_keys - half * 64, 0), 64);
+                    clear_rows(chunk, first, 64, lane);
+                    clear_rows(chunk + CHUNK_BYTES / 2, first, 64, lane);
+                    fence_proxy_async_smem();
+                    __syncwarp();
+                    if (lane == 0) {
+                        mbar_arrive(smem_u32(&bars->ring_full[slot]));
+                    }
+                }
+            }
+        } else if (warp == LOAD_WARP) {
             // =================== TMA producer ===================================
             if (lane == 0) {
                 auto load_q = [&](int i) {
                     const uint32_t bar = smem_u32(&bars->q_full[i]);
                     mbar_arrive_expect_tx(bar, KQ * CHUNK_BYTES);
-                    const int y = row0 + q_start + i * TILE_M;
+                    const int y = entry_row0 + q_start + i * TILE_M;
                     for (int c = 0; c < KQ; ++c) {
                         const uint32_t dst = q_smem + (i * KQ + c) * CHUNK_BYTES;
                         if (KQ == 3 && c == 2) {
-                            tma_load_2d(dst, &p.q_pe, bar, head * 64, y);
+                            tma_load_3d(dst, &p.q_pe, bar, head * 64, y, entry);
                         } else {
-                            tma_load_2d(dst, &p.q_main, bar, head * 128 + c * 64, y);
+                            tma_load_3d(dst, &p.q_main, bar, head * 128 + c * 64, y, entry);
                         }
                     }
                 };
                 bool alive = true;
                 int chunk = 0;
-                // Returns the destination of ring chunk `chunk` once it is free, 0 on abort.
-                auto acquire = [&](uint32_t& bar) -> uint32_t {
+                // Returns the destination of ring chunk `chunk` once it is free, 0 on abort.  `bar` names the barrier that counts the
+                // bytes: the chunk's own or `counter`.
+                auto acquire = [&](uint32_t& bar, uint64_t* counter) -> uint32_t {
                     const int slot = chunk % L::RING;
                     const int use = chunk / L::RING;
                     if (use > 0 && !mbar_wait(smem_u32(&bars->ring_empty[slot]), (use - 1) & 1, abort_flag, &forward_status)) {
                         alive = false;
                         return 0;
                     }
-                    bar = smem_u32(&bars->ring_full[slot]);
+                    bar = smem_u32(counter != nullptr ? counter : &bars->ring_full[slot]);
                     mbar_arrive_expect_tx(bar, CHUNK_BYTES);
                     ++chunk;
                     return ring_smem + slot * CHUNK_BYTES;
                 };
-                load_q(0);
-                for (int j = 0; j < tile_count && alive; ++j) {
-                    const int y = row0 + j * TILE_N;
+                auto load_tile = [&](int j, bool tail) {
+                    const int y = entry_row0 + j * TILE_N;
                     for (int c = 0; c < KQ && alive; ++c) {
                         uint32_t bar;
-                        const uint32_t dst = acquire(bar);
+                        const uint32_t dst = acquire(bar, nullptr);
                         if (dst == 0) {
-                            break;
+                            return;
                         }
                         if (KQ == 3 && c == 2) {
-                            tma_load_2d(dst, &p.k_pe, bar, 0, y);
+                            tma_load_3d(dst, &p.k_pe, bar, 0, y, entry);
                         } else {
-                            tma_load_2d(dst, &p.k_main, bar, kv_head * 128 + c * 64, y);
+                            tma_load_3d(dst, &p.k_main, bar, kv_head * 128 + c * 64, y, entry);
                         }
                     }
                     if (j == 0 && tiles[1] > 0) {
@@ -246,13 +272,20 @@ __global__ void __launch_bounds__(FORWARD_THREADS, 1) attention_forward_kernel(c
                     }
                     for (int half = 0; half < V_CHUNKS && alive; ++half) {
                         uint32_t bar;
-                        const uint32_t dst = acquire(bar);
+                        const uint32_t dst = acquire(bar, tail ? &bars->tail_full[half] : nullptr);
                         if (dst == 0) {
-                            break;
+                            return;
                         }
-                        tma_load_2d(dst, &p.v, bar, kv_head * 128, y + half * 64);
-                        tma_load_2d(dst + CHUNK_BYTES / 2, &p.v, bar, kv_head * 128 + 64, y + half * 64);
+                        tma_load_3d(dst, &p.v, bar, kv_head * 128, y + half * 64, entry);
+                        tma_load_3d(dst + CHUNK_BYTES / 2, &p.v, bar, kv_head * 128 + 64, y + half * 64, entry);
                     }
+                };
+                load_q(0);
+                for (int j = 0; j + 1 < tile_count && alive; ++j) {
+                    load_tile(j, false);
+                }
+                if (alive) {
+                    load_tile(tile_count - 1, tail_keys < TILE_N);
                 }
             }
         } else if (warp == MMA_WARP) {
@@ -538,12 +571,14 @@ void launch_prefill_forward(__nv_bfloat16* output, float* logsumexp, const __nv_
                             cudaStream_t stream) {
     check_pointers({output, logsumexp, q_nope, q_pe, k_nope, k_pe, v});
     ForwardParams params{};
-    const std::uint64_t rows = static_cast<std::uint64_t>(total_tokens);
-    params.q_main = make_bf16_tile_map(q_nope, rows, static_cast<std::uint64_t>(heads) * 128, static_cast<std::uint64_t>(heads) * 128, 128);
-    params.q_pe = make_bf16_tile_map(q_pe, rows, static_cast<std::uint64_t>(heads) * 64, static_cast<std::uint64_t>(heads) * 64, 128);
-    params.k_main = make_bf16_tile_map(k_nope, rows, static_cast<std::uint64_t>(heads) * 128, static_cast<std::uint64_t>(heads) * 128, 128);
-    params.k_pe = make_bf16_tile_map(k_pe, rows, 64, 64, 128);
-    params.v = make_bf16_tile_map(v, rows, static_cast<std::uint64_t>(heads) * 128, static_cast<std::uint64_t>(heads) * 128, 64);
+    const std::uint64_t entries = cu_seqlens == nullptr ? batch_size : 1;
+    const std::uint64_t rows = cu_seqlens == nullptr ? max_sequence_length : total_tokens;
+    const std::uint64_t wide = static_cast<std::uint64_t>(heads) * 128;
+    params.q_main = make_bf16_batched_tile_map(q_nope, entries, rows, wide, 128);
+    params.q_pe = make_bf16_batched_tile_map(q_pe, entries, rows, static_cast<std::uint64_t>(heads) * 64, 128);
+    params.k_main = make_bf16_batched_tile_map(k_nope, entries, rows, wide, 128);
+    params.k_pe = make_bf16_batched_tile_map(k_pe, entries, rows, 64, 128);
+    params.v = make_bf16_batched_tile_map(v, entries, rows, wide, 64);
     params.out = output;
     params.lse = logsumexp;
     params.cu_seqlens = cu_seqlens;
@@ -609,9 +644,9 @@ void flash_attention_forward_cuda(__nv_bfloat16* output, float* logsumexp, const
     const std::uint64_t rows = static_cast<std::uint64_t>(batch_size) * sequence_length;
     const std::uint64_t q_cols = static_cast<std::uint64_t>(query_heads) * 128;
     const std::uint64_t kv_cols = static_cast<std::uint64_t>(key_value_heads) * 128;
-    params.q_main = make_bf16_tile_map(query, rows, q_cols, q_cols, 128);
-    params.k_main = make_bf16_tile_map(key, rows, kv_cols, kv_cols, 128);
-    params.v = make_bf16_tile_map(value, rows, kv_cols, kv_cols, 64);
+    params.q_main = make_bf16_batched_tile_map(query, batch_size, sequence_length, q_cols, 128);
+    params.k_main = make_bf16_batched_tile_map(key, batch_size, sequence_length, kv_cols, 128);
+    params.v = make_bf16_batched_tile_map(value, batch_size, sequence_length, kv_cols, 64);
     params.q_pe = params.q_main;
     params.k_pe = params.k_main;
     params.out = output;

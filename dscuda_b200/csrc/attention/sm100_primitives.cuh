@@ -143,6 +143,15 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
+// Rows of a loaded tile that lie behind the end of a packed sequence are the next one's, and 0 * NaN is NaN: where such rows
+// meet zeros of P or dS, one warp clears them between the load and the barrier that the tensor core waits for.
+// A chunk holds rows of 128 bytes (64 bf16, swizzled within the row); rows first..rows-1 are cleared.
+__device__ __forceinline__ void clear_rows(uint8_t* chunk, int first, int rows, int lane) {
+    for (int offset = first * 128 + lane * 16; offset < rows * 128; offset += 32 * 16) {
+        *reinterpret_cast<uint4*>(chunk + offset) = make_uint4(0, 0, 0, 0);
+    }
+}
+
 __device__ __forceinline__ void tc_fence_before_sync() {
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
 }

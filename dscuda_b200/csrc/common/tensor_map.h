@@ -16,6 +16,10 @@ namespace dscuda {
 CUtensorMap make_bf16_tile_map(const void* base, std::uint64_t rows, std::uint64_t cols, std::uint64_t row_stride_elements,
                                std::uint32_t box_rows);
 
+// The same for a batch of `rows` rows each, everything contiguous: box {64, box_rows, 1} at {column, row, entry}.
+// Rows past the entry's last one read as zero, not as the next entry's.
+CUtensorMap make_bf16_batched_tile_map(const void* base, std::uint64_t batch, std::uint64_t rows, std::uint64_t cols, std::uint32_t box_rows);
+
 // The same rows seen as [chunk][row][64 elements]: `chunks` consecutive 64-column chunks of a row are
 // 128 bytes apart, rows `row_stride_elements` apart.  One load of a box {64, box_rows, box_chunks} at
 // coordinates {0, row, chunk} lands in shared memory chunk after chunk, each a [box_rows x 128 byte]

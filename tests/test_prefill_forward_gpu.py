@@ -63,6 +63,51 @@ def test_packed_matches_oracle(gpu, seqlens):
     check_forward(out, lse, ref_out, ref_lse)
 
 
+def poison(tensors, rows):
+    """Copies of tensors with everything outside `rows` (a slice of the first dimension) NaN."""
+    out = []
+    for t in tensors:
+        t = t.clone()
+        t[:rows.start] = float("nan")
+        t[rows.stop:] = float("nan")
+        out.append(t)
+    return out
+
+
+# lengths around the 128-key tiles and their 64-key halves; every sequence but the last ends inside a tile that reaches into the next one
+@pytest.mark.parametrize("seqlens", [[1, 63, 64, 65], [127, 129, 5], [130, 257, 300, 191], [128, 256, 20]])
+def test_packed_sequences_stay_apart(gpu, seqlens):
+    """What lies in the other sequences, even NaN, does not reach a sequence's outputs."""
+    from dscuda_b200 import mla
+    *tensors, _, cu = oracle.prefill_inputs(45, 0, 0, 2, seqlens=seqlens)
+    device, cu_device = [t.to(gpu) for t in tensors], cu.to(gpu)
+    clean, clean_lse = mla.prefill_forward(*device, SCALE, cu_device, max(seqlens))
+    for b, n in enumerate(seqlens):
+        rows = slice(int(cu[b]), int(cu[b]) + n)
+        out, lse = mla.prefill_forward(*poison(device, rows), SCALE, cu_device, max(seqlens))
+        assert torch.equal(out[rows], clean[rows]) and torch.equal(lse[:, rows], clean_lse[:, rows]), f"sequence {b}"
+    assert mla.device_status() == 0
+
+
+@pytest.mark.parametrize("s", [1, 64, 70, 130, 255, 300])
+def test_batch_entries_stay_apart(gpu, s):
+    """The same for the entries of a dense batch, in the non-absorbed, the grouped-query and the absorbed forward."""
+    from dscuda_b200 import mla
+    generator = torch.Generator().manual_seed(s)
+
+    def draw(*tails):
+        return [(torch.randn(3, s, *tail, generator=generator) * .5).bfloat16().to(gpu) for tail in tails]
+
+    calls = [(mla.prefill_forward, draw((2, 128), (2, 64), (2, 128), (1, 64), (2, 128)), SCALE),
+             (mla.flash_forward, draw((4, 128), (2, 128), (2, 128)), 128 ** -0.5),
+             (mla.mla_forward, draw((3, 512), (3, 64), (512,), (64,)), 576 ** -0.5)]
+    for call, tensors, scale in calls:
+        clean, clean_lse = call(*tensors, scale)
+        out, lse = call(*poison(tensors, slice(1, 2)), scale)
+        assert torch.equal(out[1], clean[1]) and torch.equal(lse[1], clean_lse[1]), call.__name__
+    assert mla.device_status() == 0
+
+
 def test_is_deterministic(gpu):
     q_nope, q_pe, k_nope, k_pe, v, _ = oracle.prefill_inputs(77, 1, 384, 2)
     first = run_forward(gpu, (q_nope, q_pe, k_nope, k_pe, v), SCALE)
