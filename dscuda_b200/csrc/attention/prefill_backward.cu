@@ -63,9 +63,10 @@ constexpr float LOG2E = 1.4426950408889634F;
 __device__ int backward_status = 0;
 
 struct BackwardParams {
-    // 128-row boxes (stationary tiles) and 64-row boxes (streamed tiles) of the same tensors
+    // 128-row boxes (stationary tiles) and 64-row boxes (streamed tiles) of the same tensors; dense: a batch of S rows each, packed:
+    // one entry of all rows
     CUtensorMap q_main_big, q_pe_big, k_main_big, k_pe_big, v_big, do_big;
-    CUtensorMap q_main_sub, q_pe_sub, k_main_sub, k_pe_sub, v_sub, do_sub;
+    CUtensorMap q_main_sub, q_pe_sub, k_main_sub, k_pe_sub, do_sub;
     // stores of 32 rows: 64 bf16 columns of the gradients, 32 fp32 columns of a head's dk_pe contributions
     CUtensorMap dq_map, dk_map, dv_map, parts_map;
     __nv_bfloat16* dq;        // [rows, H, 192]
@@ -96,6 +97,7 @@ struct BackwardBarriers {
     uint64_t resident_full;
     uint64_t stage_full[STAGES];
     uint64_t stage_empty[STAGES];
+    uint64_t tail_full;         // a last tile that contains another sequence's rows has landed
     uint64_t mma_a[2];          // tensor core -> softmax group: first score tile ready
     uint64_t mma_b[2];          // tensor core -> softmax group: second score tile ready
     uint64_t soft_a[2];         // softmax group -> tensor core: first bf16 operand stored
@@ -148,6 +150,22 @@ __device__ __forceinline__ bool locate_block(const BackwardParams& p, int rows_p
     return false;
 }
 
+// Where a sequence's rows are in the load maps, and whether another sequence's rows follow there.  Behind the end of a batch entry
+// tiles load as zero; behind a packed sequence they hold the next one's rows, which have to be cleared where the tensor core
+// would multiply them by zeros of P or dS.
+struct LoadPlace {
+    int entry;
+    int row0;
+    bool followed;
+};
+
+__device__ __forceinline__ LoadPlace load_place(const BackwardParams& p, int row0, int length) {
+    if (p.cu_seqlens == nullptr) {
+        return {static_cast<int>(blockIdx.z), 0, false};
+    }
+    return {0, row0, row0 + length < p.total};
+}
+
 // Where the dS^T tiles of `sequence` start inside one head's part of the scratch, how many tiles a head
 // has in all, and the sequence's number of 128-key tiles.
 struct ScratchPlace {
@@ -182,6 +200,7 @@ __device__ __forceinline__ void init_barriers(BackwardBarriers* bars, uint32_t s
         mbar_init(smem_u32(&bars->stage_full[i]), stage_full_arrivals);
         mbar_init(smem_u32(&bars->stage_empty[i]), 1);
     }
+    mbar_init(smem_u32(&bars->tail_full), 1);
     for (int i = 0; i < 2; ++i) {
         mbar_init(smem_u32(&bars->mma_a[i]), 1);
         mbar_init(smem_u32(&bars->mma_b[i]), 1);
@@ -360,6 +379,7 @@ struct Barriers {
     uint64_t k_empty[K_SLOTS];
     uint64_t v_full;
     uint64_t v_empty;
+    uint64_t tail_full[2];      // K and V of a last tile that contains another sequence's keys have landed
     uint64_t s_full;            // tensor core -> softmax: S(j) complete
     uint64_t dp_full;           // tensor core -> softmax: dP(j) complete
     uint64_t s_free;            // 256 softmax threads: S(j) is in registers
@@ -416,6 +436,8 @@ __global__ void __launch_bounds__(THREADS, 1) backward_dq_kernel(const __grid_co
         }
         mbar_init(smem_u32(&bars->v_full), 1);
         mbar_init(smem_u32(&bars->v_empty), 1);
+        mbar_init(smem_u32(&bars->tail_full[0]), 1);
+        mbar_init(smem_u32(&bars->tail_full[1]), 1);
         mbar_init(smem_u32(&bars->s_full), 1);
         mbar_init(smem_u32(&bars->dp_full), 1);
         mbar_init(smem_u32(&bars->s_free), 256);
@@ -435,17 +457,51 @@ __global__ void __launch_bounds__(THREADS, 1) backward_dq_kernel(const __grid_co
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&bars->tmem_base);
 
     if (warp == LOAD_WARP) {
+        // K(last) and V(last) land on barriers of this warp's own where they contain another sequence's keys: dS K multiplies
+        // those by zeros, and dP of such a key would make its dS 0 * dP
+        const LoadPlace place = load_place(p, row0, length);
+        const int last = tile_count - 1;
+        const bool ragged = place.followed && tile_count * KEYS > length;
+        bool alive = true;
+        auto clear_tail = [&](int which, uint32_t offset, int chunks, uint64_t* full) {
+            __syncwarp();               // the other lanes wait here, not in the loop of the barrier, while lane 0 loads
+            if (!__all_sync(0xffffffffU, alive && mbar_wait(smem_u32(&bars->tail_full[which]), 0, abort_flag, &backward_status))) {
+                alive = false;
+                return;
+            }
+            for (int c = 0; c < chunks; ++c) {
+                clear_rows(smem_raw + offset + c * CHUNK, length - last * KEYS, KEYS, lane);
+            }
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(smem_u32(full));
+            }
+        };
+        auto load_v = [&](int j) {
+            // the slot is free once dO has been copied out (first tile) or dP(j-1) has run
+            const bool ready = j == 0 ? mbar_wait(smem_u32(&bars->do_copied), 0, abort_flag, &backward_status)
+                                      : mbar_wait(smem_u32(&bars->v_empty), (j - 1) & 1, abort_flag, &backward_status);
+            if (!ready) {
+                alive = false;
+                return;
+            }
+            const uint32_t full = smem_u32(ragged && j == last ? &bars->tail_full[1] : &bars->v_full);
+            mbar_arrive_expect_tx(full, V_TILE);
+            const int ky = place.row0 + j * KEYS;
+            tma_load_3d(v_smem, &p.v_big, full, head * 128, ky, place.entry);
+            tma_load_3d(v_smem + CHUNK, &p.v_big, full, head * 128 + 64, ky, place.entry);
+        };
         if (lane == 0) {
-            bool alive = true;
             {
                 const uint32_t bar = smem_u32(&bars->resident_full);
                 mbar_arrive_expect_tx(bar, Q_BYTES + V_TILE);
-                const int y = row0 + q_start;
-                tma_load_2d(q_smem, &p.q_main_big, bar, head * 128, y);
-                tma_load_2d(q_smem + CHUNK, &p.q_main_big, bar, head * 128 + 64, y);
-                tma_load_2d(q_smem + 2 * CHUNK, &p.q_pe_big, bar, head * 64, y);
-                tma_load_2d(v_smem, &p.do_big, bar, head * 128, y);
-                tma_load_2d(v_smem + CHUNK, &p.do_big, bar, head * 128 + 64, y);
+                const int y = place.row0 + q_start;
+                tma_load_3d(q_smem, &p.q_main_big, bar, head * 128, y, place.entry);
+                tma_load_3d(q_smem + CHUNK, &p.q_main_big, bar, head * 128 + 64, y, place.entry);
+                tma_load_3d(q_smem + 2 * CHUNK, &p.q_pe_big, bar, head * 64, y, place.entry);
+                tma_load_3d(v_smem, &p.do_big, bar, head * 128, y, place.entry);
+                tma_load_3d(v_smem + CHUNK, &p.do_big, bar, head * 128 + 64, y, place.entry);
             }
             auto load_k = [&](int j) {
                 const int slot = j % K_SLOTS;
@@ -454,27 +510,13 @@ __global__ void __launch_bounds__(THREADS, 1) backward_dq_kernel(const __grid_co
                     alive = false;
                     return;
                 }
-                const uint32_t full = smem_u32(&bars->k_full[slot]);
+                const uint32_t full = smem_u32(ragged && j == last ? &bars->tail_full[0] : &bars->k_full[slot]);
                 mbar_arrive_expect_tx(full, K_TILE);
                 const uint32_t dst = k_ring + slot * K_TILE;
-                const int ky = row0 + j * KEYS;
-                tma_load_2d(dst, &p.k_main_big, full, head * 128, ky);
-                tma_load_2d(dst + CHUNK, &p.k_main_big, full, head * 128 + 64, ky);
-                tma_load_2d(dst + 2 * CHUNK, &p.k_pe_big, full, 0, ky);
-            };
-            auto load_v = [&](int j) {
-                // the slot is free once dO has been copied out (first tile) or dP(j-1) has run
-                const bool ready = j == 0 ? mbar_wait(smem_u32(&bars->do_copied), 0, abort_flag, &backward_status)
-                                          : mbar_wait(smem_u32(&bars->v_empty), (j - 1) & 1, abort_flag, &backward_status);
-                if (!ready) {
-                    alive = false;
-                    return;
-                }
-                const uint32_t full = smem_u32(&bars->v_full);
-                mbar_arrive_expect_tx(full, V_TILE);
-                const int ky = row0 + j * KEYS;
-                tma_load_2d(v_smem, &p.v_big, full, head * 128, ky);
-                tma_load_2d(v_smem + CHUNK, &p.v_big, full, head * 128 + 64, ky);
+                const int ky = place.row0 + j * KEYS;
+                tma_load_3d(dst, &p.k_main_big, full, head * 128, ky, place.entry);
+                tma_load_3d(dst + CHUNK, &p.k_main_big, full, head * 128 + 64, ky, place.entry);
+                tma_load_3d(dst + 2 * CHUNK, &p.k_pe_big, full, 0, ky, place.entry);
             };
             // K(j) becomes loadable after dQ(j-3), V(j-1) right after that (after dP(j-2)).
             for (int j = 0; j < tile_count && alive; ++j) {
@@ -483,9 +525,15 @@ __global__ void __launch_bounds__(THREADS, 1) backward_dq_kernel(const __grid_co
                     load_v(j - 1);
                 }
             }
-            if (alive) {
-                load_v(tile_count - 1);
-            }
+        }
+        if (ragged) {
+            clear_tail(0, Q_BYTES + (last % K_SLOTS) * K_TILE, 3, &bars->k_full[last % K_SLOTS]);
+        }
+        if (lane == 0 && alive) {
+            load_v(last);
+        }
+        if (ragged) {
+            clear_tail(1, Q_BYTES + K_SLOTS * K_TILE, 2, &bars->v_full);
         }
     } else if (warp == MMA_WARP) {
         // Whole warp, uniform control flow; the elected lane executes the tcgen05 instructions.
@@ -728,15 +776,16 @@ __global__ void __launch_bounds__(THREADS, 1) backward_dkdv_kernel(const __grid_
     constexpr uint32_t TMEM_X = 320;
 
     if (warp == LOAD_WARP) {
+        const LoadPlace place = load_place(p, row0, length);
         if (lane == 0) {
             const uint32_t bar = smem_u32(&bars->resident_full);
             mbar_arrive_expect_tx(bar, RESIDENT_BYTES);
-            const int y = row0 + key_start;
-            tma_load_2d(k_smem, &p.k_main_big, bar, head * 128, y);
-            tma_load_2d(k_smem + BIG_CHUNK, &p.k_main_big, bar, head * 128 + 64, y);
-            tma_load_2d(k_smem + 2 * BIG_CHUNK, &p.k_pe_big, bar, 0, y);
-            tma_load_2d(v_smem, &p.v_big, bar, head * 128, y);
-            tma_load_2d(v_smem + BIG_CHUNK, &p.v_big, bar, head * 128 + 64, y);
+            const int y = place.row0 + key_start;
+            tma_load_3d(k_smem, &p.k_main_big, bar, head * 128, y, place.entry);
+            tma_load_3d(k_smem + BIG_CHUNK, &p.k_main_big, bar, head * 128 + 64, y, place.entry);
+            tma_load_3d(k_smem + 2 * BIG_CHUNK, &p.k_pe_big, bar, 0, y, place.entry);
+            tma_load_3d(v_smem, &p.v_big, bar, head * 128, y, place.entry);
+            tma_load_3d(v_smem + BIG_CHUNK, &p.v_big, bar, head * 128 + 64, y, place.entry);
         }
         bool alive = true;
         for (int t = 0; t < tile_count && alive; ++t) {
@@ -750,15 +799,17 @@ __global__ void __launch_bounds__(THREADS, 1) backward_dkdv_kernel(const __grid_
             }
             const int q0 = (first_tile + t) * SUB;
             const uint32_t full = smem_u32(&bars->stage_full[stage]);
+            const bool tail = place.followed && q0 + SUB > length;         // only the last tile: this warp sees it before the tensor core does
             if (lane == 0) {
-                mbar_arrive_expect_tx(full, STAGE_BYTES);
+                const uint32_t bar = tail ? smem_u32(&bars->tail_full) : full;
+                mbar_arrive_expect_tx(bar, STAGE_BYTES);
                 const uint32_t dst = stage_smem + stage * STAGE_BYTES;
-                const int qy = row0 + q0;
-                tma_load_2d(dst, &p.q_main_sub, full, head * 128, qy);
-                tma_load_2d(dst + SUB_CHUNK, &p.q_main_sub, full, head * 128 + 64, qy);
-                tma_load_2d(dst + 2 * SUB_CHUNK, &p.q_pe_sub, full, head * 64, qy);
-                tma_load_2d(dst + 3 * SUB_CHUNK, &p.do_sub, full, head * 128, qy);
-                tma_load_2d(dst + 4 * SUB_CHUNK, &p.do_sub, full, head * 128 + 64, qy);
+                const int qy = place.row0 + q0;
+                tma_load_3d(dst, &p.q_main_sub, bar, head * 128, qy, place.entry);
+                tma_load_3d(dst + SUB_CHUNK, &p.q_main_sub, bar, head * 128 + 64, qy, place.entry);
+                tma_load_3d(dst + 2 * SUB_CHUNK, &p.q_pe_sub, bar, head * 64, qy, place.entry);
+                tma_load_3d(dst + 3 * SUB_CHUNK, &p.do_sub, bar, head * 128, qy, place.entry);
+                tma_load_3d(dst + 4 * SUB_CHUNK, &p.do_sub, bar, head * 128 + 64, qy, place.entry);
             }
 #pragma unroll
             for (int e = 0; e < SUB / 32; ++e) {
@@ -772,9 +823,23 @@ __global__ void __launch_bounds__(THREADS, 1) backward_dkdv_kernel(const __grid_
                 bars->lse2[stage][n] = lse_value;
                 bars->delta[stage][n] = delta_value;
             }
+            if (tail) {
+                // dV += P^T dO and dK += dS^T Q multiply these rows by zeros
+                alive = __all_sync(0xffffffffU, mbar_wait(smem_u32(&bars->tail_full), 0, abort_flag, &backward_status));
+                if (!alive) {
+                    break;
+                }
+                for (int c = 0; c < 5; ++c) {
+                    clear_rows(smem_aligned + RESIDENT_BYTES + stage * STAGE_BYTES + c * SUB_CHUNK, length - q0, SUB, lane);
+                }
+                fence_proxy_async_smem();
+            }
             __syncwarp();
             if (lane == 0) {
                 mbar_arrive(full);
+                if (tail) {
+                    mbar_arrive(full);          // in the place of the transaction
+                }
             }
         }
     } else if (warp == MMA_WARP) {
@@ -948,8 +1013,7 @@ __global__ void __launch_bounds__(THREADS, 1) backward_dkdv_kernel(const __grid_
             if (ds_tiles != nullptr) {
                 // The same 32 bf16 values go to the scratch for the kernel that turns dS into dQ: four 16-byte
                 // units, unit (4 group + e) of this key.  The 32 lanes of a warp write 512 consecutive bytes.
-                // Keys past the end of the sequence are written as zeros, so that whatever lies behind
-                // the last key in the K tensor cannot reach dQ.
+                // Keys past the end of the sequence are written as zeros; dQ multiplies them by rows of zeros.
                 uint4* dst = ds_tiles + static_cast<size_t>(t) * (DS_TILE_BYTES / 16) + (group * 4) * BIG + r;
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
@@ -1076,6 +1140,7 @@ static_assert(STREAM_SMEM_BYTES <= 227 * 1024, "streamed dQ kernel shared memory
 struct StreamBarriers {
     uint64_t full[STREAM_STAGES];
     uint64_t empty[STREAM_STAGES];
+    uint64_t tail_full;         // a last stage that contains another sequence's keys has landed
     uint64_t done;
     uint32_t tmem_base;
     int abort_flag;
@@ -1101,9 +1166,9 @@ __global__ void __launch_bounds__(dqs::STREAM_THREADS, 1) backward_dq_stream_ker
     const int stage_count = (key_end + KSUB - 1) / KSUB;
     const bool second_used = q_start + 128 < length;
     // rows of the scratch view (8-query blocks) before this (head, sequence), and key tiles of the sequence
-    const ScratchPlace place = scratch_place(p, sequence);
-    const int key_tiles = place.key_tiles;
-    const long long ds_row0 = (blockIdx.y * place.head_tiles + place.sequence_first) * 8;
+    const ScratchPlace scratch = scratch_place(p, sequence);
+    const int key_tiles = scratch.key_tiles;
+    const long long ds_row0 = (blockIdx.y * scratch.head_tiles + scratch.sequence_first) * 8;
     const int q_tile0 = q_start / SUB;
 
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023U) & ~1023U;
@@ -1118,6 +1183,7 @@ __global__ void __launch_bounds__(dqs::STREAM_THREADS, 1) backward_dq_stream_ker
             mbar_init(smem_u32(&bars->full[i]), 1);
             mbar_init(smem_u32(&bars->empty[i]), 1);
         }
+        mbar_init(smem_u32(&bars->tail_full), 1);
         mbar_init(smem_u32(&bars->done), 1);
         bars->abort_flag = 0;
         mbar_init_fence();
@@ -1136,6 +1202,7 @@ __global__ void __launch_bounds__(dqs::STREAM_THREADS, 1) backward_dq_stream_ker
     // takes keys below q_start + 128, the second all of them; stages only the second uses
     // load the two chunks of its rows only.
     if (warp == STREAM_LOAD_WARP) {
+        const LoadPlace place = load_place(p, row0, length);
         const uint64_t policy = l2_evict_first_policy();       // dS is read once; the K rows are what should stay in L2
         bool alive = true;
         for (int s = 0; s < stage_count && alive; ++s) {
@@ -1146,10 +1213,11 @@ __global__ void __launch_bounds__(dqs::STREAM_THREADS, 1) backward_dq_stream_ker
                     break;
                 }
             }
+            const int key0 = s * KSUB;
+            const bool tail = place.followed && key0 + KSUB > length;      // only the last stage: this warp sees it before the tensor core does
             if (lane == 0) {
-                const int key0 = s * KSUB;
                 const int first_chunk = key0 < q_start + 128 ? 0 : 2;
-                const uint32_t full = smem_u32(&bars->full[stage]);
+                const uint32_t full = smem_u32(tail ? &bars->tail_full : &bars->full[stage]);
                 const uint32_t dst = smem_base + stage * STREAM_STAGE_BYTES;
                 mbar_arrive_expect_tx(full, (4 - first_chunk) * SUB_CHUNK + K_BYTES);
                 // key tile kt holds its query tiles 2 kt, 2 kt + 1, ... one after the other, 8 rows of the view each
@@ -1158,10 +1226,24 @@ __global__ void __launch_bounds__(dqs::STREAM_THREADS, 1) backward_dq_stream_ker
                 for (int c = first_chunk; c < 4; c += 2) {
                     tma_load_2d_hint(dst + c * SUB_CHUNK, &p.ds_map, full, (key0 % BIG) * 2, static_cast<int>(ds_row0 + (tile + c) * 8), policy);
                 }
-                const int y = row0 + key0;
-                tma_load_2d(dst + DS_BYTES, &p.k_main_sub, full, head * 128, y);
-                tma_load_2d(dst + DS_BYTES + SUB_CHUNK, &p.k_main_sub, full, head * 128 + 64, y);
-                tma_load_2d(dst + DS_BYTES + 2 * SUB_CHUNK, &p.k_pe_sub, full, 0, y);
+                const int y = place.row0 + key0;
+                tma_load_3d(dst + DS_BYTES, &p.k_main_sub, full, head * 128, y, place.entry);
+                tma_load_3d(dst + DS_BYTES + SUB_CHUNK, &p.k_main_sub, full, head * 128 + 64, y, place.entry);
+                tma_load_3d(dst + DS_BYTES + 2 * SUB_CHUNK, &p.k_pe_sub, full, 0, y, place.entry);
+            }
+            if (tail) {                                     // dS K multiplies these keys by zeros
+                alive = __all_sync(0xffffffffU, mbar_wait(smem_u32(&bars->tail_full), 0, abort_flag, &backward_status));
+                if (!alive) {
+                    break;
+                }
+                for (int c = 0; c < 3; ++c) {
+                    clear_rows(smem_aligned + stage * STREAM_STAGE_BYTES + DS_BYTES + c * SUB_CHUNK, length - key0, KSUB, lane);
+                }
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(smem_u32(&bars->full[stage]));
+                }
             }
         }
     } else if (warp == STREAM_MMA_WARP) {
@@ -1366,18 +1448,19 @@ void mla_prefill_backward_cuda(__nv_bfloat16* dq, __nv_bfloat16* dk_nope, __nv_b
     const std::uint64_t rows = static_cast<std::uint64_t>(total_tokens);
     const std::uint64_t wide = static_cast<std::uint64_t>(heads) * 128;
     const std::uint64_t narrow = static_cast<std::uint64_t>(heads) * 64;
-    params.q_main_big = make_bf16_tile_map(q_nope, rows, wide, wide, BIG);
-    params.q_pe_big = make_bf16_tile_map(q_pe, rows, narrow, narrow, BIG);
-    params.k_main_big = make_bf16_tile_map(k_nope, rows, wide, wide, BIG);
-    params.k_pe_big = make_bf16_tile_map(k_pe, rows, 64, 64, BIG);
-    params.v_big = make_bf16_tile_map(v, rows, wide, wide, BIG);
-    params.do_big = make_bf16_tile_map(output_gradient, rows, wide, wide, BIG);
-    params.q_main_sub = make_bf16_tile_map(q_nope, rows, wide, wide, SUB);
-    params.q_pe_sub = make_bf16_tile_map(q_pe, rows, narrow, narrow, SUB);
-    params.k_main_sub = make_bf16_tile_map(k_nope, rows, wide, wide, SUB);
-    params.k_pe_sub = make_bf16_tile_map(k_pe, rows, 64, 64, SUB);
-    params.v_sub = make_bf16_tile_map(v, rows, wide, wide, SUB);
-    params.do_sub = make_bf16_tile_map(output_gradient, rows, wide, wide, SUB);
+    const std::uint64_t entries = cu_seqlens == nullptr ? batch_size : 1;
+    const std::uint64_t entry_rows = cu_seqlens == nullptr ? max_sequence_length : total_tokens;
+    params.q_main_big = make_bf16_batched_tile_map(q_nope, entries, entry_rows, wide, BIG);
+    params.q_pe_big = make_bf16_batched_tile_map(q_pe, entries, entry_rows, narrow, BIG);
+    params.k_main_big = make_bf16_batched_tile_map(k_nope, entries, entry_rows, wide, BIG);
+    params.k_pe_big = make_bf16_batched_tile_map(k_pe, entries, entry_rows, 64, BIG);
+    params.v_big = make_bf16_batched_tile_map(v, entries, entry_rows, wide, BIG);
+    params.do_big = make_bf16_batched_tile_map(output_gradient, entries, entry_rows, wide, BIG);
+    params.q_main_sub = make_bf16_batched_tile_map(q_nope, entries, entry_rows, wide, SUB);
+    params.q_pe_sub = make_bf16_batched_tile_map(q_pe, entries, entry_rows, narrow, SUB);
+    params.k_main_sub = make_bf16_batched_tile_map(k_nope, entries, entry_rows, wide, SUB);
+    params.k_pe_sub = make_bf16_batched_tile_map(k_pe, entries, entry_rows, 64, SUB);
+    params.do_sub = make_bf16_batched_tile_map(output_gradient, entries, entry_rows, wide, SUB);
     params.dq_map = make_bf16_store_map(dq, rows, static_cast<std::uint64_t>(heads) * 192, 64, 32);
     params.dk_map = make_bf16_store_map(dk_nope, rows, wide, 64, 32);
     params.dv_map = make_bf16_store_map(dv, rows, wide, 64, 32);

@@ -72,6 +72,65 @@ def test_packed_matches_oracle(gpu, seqlens):
     check_grads(grads, oracle.prefill_backward(dout, out, lse, *tensors, SCALE, cu))
 
 
+def poison(tensors, rows):
+    """Copies of tensors with everything outside `rows` (a slice of the first dimension) NaN."""
+    out = []
+    for t in tensors:
+        t = t.clone()
+        t[:rows.start] = float("nan")
+        t[rows.stop:] = float("nan")
+        out.append(t)
+    return out
+
+
+# Lengths around the 128-key and 64-row tiles; with limit 0 dQ is recomputed instead of taken from the stored dS.  [700, 400]: the
+# last stage of the streamed dQ comes after its ring of four has gone round.
+@pytest.mark.parametrize("limit", [None, 0])
+@pytest.mark.parametrize("seqlens", [[1, 63, 64, 65], [127, 129, 5], [130, 257, 300, 191], [128, 256, 20], [700, 400]])
+def test_packed_sequences_stay_apart(gpu, seqlens, limit):
+    """What lies in the other sequences, even NaN, does not reach a sequence's gradients."""
+    from dscuda_b200 import mla
+    *tensors, dout, cu = oracle.prefill_inputs(46, 0, 0, 2, dout_std=0.1, seqlens=seqlens)
+    device, cu_device = [t.to(gpu) for t in tensors], cu.to(gpu)
+    out, lse = mla.prefill_forward(*device, SCALE, cu_device, max(seqlens))
+    everything = [dout.to(gpu), out, lse.T.contiguous(), *device]
+    previous = mla.prefill_backward_scratch_limit(limit) if limit is not None else None
+    try:
+        def backward(dout, out, lse_rows, *inputs):
+            return mla.prefill_backward(dout, out, lse_rows.T.contiguous(), *inputs, SCALE, cu_device, max(seqlens))
+
+        clean = backward(*everything)
+        for b, n in enumerate(seqlens):
+            rows = slice(int(cu[b]), int(cu[b]) + n)
+            for name, x, y in zip(NAMES, clean, backward(*poison(everything, rows))):
+                assert torch.equal(x[rows], y[rows]), f"{name} of sequence {b}"
+    finally:
+        if previous is not None:
+            mla.prefill_backward_scratch_limit(previous)
+    assert mla.device_status() == 0
+
+
+@pytest.mark.parametrize("limit", [None, 0])
+@pytest.mark.parametrize("s", [1, 64, 70, 130, 255, 300])
+def test_batch_entries_stay_apart(gpu, s, limit):
+    """The same for the entries of a dense batch."""
+    from dscuda_b200 import mla
+    *tensors, dout = oracle.prefill_inputs(300 + s, 3, s, 2, dout_std=0.1)
+    device = [t.to(gpu) for t in tensors]
+    out, lse = mla.prefill_forward(*device, SCALE)
+    everything = [dout.to(gpu), out, lse, *device]
+    previous = mla.prefill_backward_scratch_limit(limit) if limit is not None else None
+    try:
+        clean = mla.prefill_backward(*everything, SCALE)
+        poisoned = mla.prefill_backward(*poison(everything, slice(1, 2)), SCALE)
+    finally:
+        if previous is not None:
+            mla.prefill_backward_scratch_limit(previous)
+    for name, x, y in zip(NAMES, clean, poisoned):
+        assert torch.equal(x[1], y[1]), name
+    assert mla.device_status() == 0
+
+
 def test_gradients_are_overwritten_not_accumulated(gpu):
     """Two calls on the same buffers give bit-identical results, dk_pe (a sum over heads in a fixed order) included."""
     from dscuda_b200 import mla
