@@ -25,6 +25,8 @@ namespace {
 using at::Tensor;
 
 constexpr int64_t LATENT = 512;                // width of the latent part of a cache row
+constexpr int64_t VALUE = 128;                 // columns of k_nope and v
+constexpr int64_t CACHE_WIDTH = 576;           // of a whole row
 constexpr int64_t FP8_ROW_BYTES = 656;
 
 // A Python error that is not one of c10's (HANDLE_TH_ERRORS would turn std::exception into RuntimeError).
@@ -76,15 +78,39 @@ const Tensor* optional_tensor(PyObject* object) {
     return object == Py_None ? nullptr : &tensor(object);
 }
 
-// An output the caller may bring: taken as it is.
-const Tensor* optional_output(PyObject* object) {
-    if (object == Py_None) {
-        return nullptr;
+// Memory the caller brings for a result or as scratch is written through its pointer, so it has to be where the inputs are and
+// large enough (it may be larger).
+void expect_device(const Tensor& t, const Tensor& like, const char* what) {
+    if (t.device() != like.device()) {
+        fail(PyExc_ValueError, std::string(what) + " is on another device than the inputs");
     }
-    if (!THPVariable_Check(object)) {
-        fail(PyExc_TypeError, std::string("expected a torch tensor, got ") + Py_TYPE(object)->tp_name);
+}
+
+// An output the caller may bring, of `elements` values of `type`; null for None.
+const Tensor* optional_output(PyObject* object, const Tensor& like, at::ScalarType type, int64_t elements, const char* what) {
+    const Tensor* t = optional_tensor(object);
+    if (t != nullptr) {
+        expect_device(*t, like, what);
+        if (t->scalar_type() != type) {
+            fail(PyExc_ValueError, std::string(what) + " has the wrong dtype");
+        }
+        if (t->numel() < elements) {
+            fail(PyExc_ValueError, std::string(what) + " has " + std::to_string(t->numel()) + " elements, " + std::to_string(elements) + " are written");
+        }
     }
-    return &THPVariable_Unpack(object);
+    return t;
+}
+
+// Scratch the caller may bring, of at least `bytes` bytes and any dtype; null for None.
+const Tensor* optional_workspace(PyObject* object, const Tensor& like, size_t bytes) {
+    const Tensor* t = optional_tensor(object);
+    if (t != nullptr) {
+        expect_device(*t, like, "the workspace");
+        if (t->nbytes() < bytes) {
+            fail(PyExc_ValueError, "the workspace has " + std::to_string(t->nbytes()) + " bytes, " + std::to_string(bytes) + " are needed");
+        }
+    }
+    return t;
 }
 
 void* pointer(const Tensor& t) {
@@ -240,14 +266,18 @@ DSCUDA_FUNCTION(mla_decode) {
         const Tensor &query = tensor(args[0], 4), &cache = tensor(args[1]), &table = tensor(args[2]), &lengths = tensor(args[3]);
         const float scale = number(args[4]);
         const int splits = static_cast<int>(integer(args[5]));
-        const Tensor* workspace_given = optional_tensor(args[6]);
-        const Tensor *output_given = optional_output(args[7]), *lse_given = optional_output(args[8]);
         const int pages_checked = PyObject_IsTrue(args[9]);
         if (pages_checked < 0) {
             throw python_error();
         }
         const int b = extent(query, 0), h = extent(query, 2), rope = static_cast<int>(query.size(3) - LATENT), page_size = extent(cache, 1);
         const int pages = extent(table, 1), blocks = extent(cache, 0);
+        const int64_t rows = static_cast<int64_t>(b) * h;
+        // sizes that are not positive are refused below
+        const size_t partials_bytes = splits > 0 ? dscuda_mla_workspace_elements(b, h, splits, static_cast<int>(LATENT)) * sizeof(float) : 0;
+        const Tensor* workspace_given = optional_workspace(args[6], query, partials_bytes);
+        const Tensor *output_given = optional_output(args[7], query, at::kBFloat16, rows * LATENT, "the output"),
+                     *lse_given = optional_output(args[8], query, at::kFloat, rows, "the LSE");
         Tensor workspace =
             workspace_given != nullptr
                 ? *workspace_given
@@ -305,14 +335,21 @@ DSCUDA_FUNCTION(cache_dequantize_fp8) {
     return guarded([&] {
         expect_arguments(count, 4);
         const Tensor& fp8 = tensor(args[0]);
-        const Tensor* given = optional_tensor(args[1]);
         const long long first = integer(args[2]);
         if (fp8.dim() != 3) {
             fail(PyExc_ValueError, "the FP8 cache is a uint8 tensor [blocks, page, 656]");
         }
         const int64_t blocks = fp8.size(0), page = fp8.size(1);
-        Tensor cache = given != nullptr ? *given : new_tensor({blocks, page, 1, 576}, fp8, at::kBFloat16);
         const long long rows = args[3] == Py_None ? blocks * page - first : integer(args[3]);
+        int64_t elements = 0;
+        if (first >= 0 && rows > 0) {                       // what is not is refused below
+            if (first > blocks * page || rows > blocks * page - first || fp8.nbytes() < static_cast<size_t>(first + rows) * FP8_ROW_BYTES) {
+                fail(PyExc_ValueError, "the rows do not lie inside the FP8 cache");
+            }
+            elements = (first + rows) * CACHE_WIDTH;
+        }
+        const Tensor* given = optional_output(args[1], fp8, at::kBFloat16, elements, "the cache");
+        Tensor cache = given != nullptr ? *given : new_tensor({blocks, page, 1, CACHE_WIDTH}, fp8, at::kBFloat16);
         void* stream = current_stream();
         checked(dscuda_mla_last_error, [&] { return dscuda_mla_cache_dequantize_fp8(pointer(cache), pointer(fp8), first, rows, stream); });
         return wrap(cache);
@@ -417,8 +454,10 @@ DSCUDA_FUNCTION(prefill_forward) {
         const Tensor &q_nope = tensor(args[0]), &q_pe = tensor(args[1]), &k_nope = tensor(args[2]), &k_pe = tensor(args[3]), &v = tensor(args[4]);
         const float scale = number(args[5]);
         const Tensor* cu = optional_tensor(args[6]);
-        const Tensor *output_given = optional_output(args[8]), *lse_given = optional_output(args[9]);
         const PrefillShape n = prefill_shape(q_nope, cu, args[7]);
+        const int64_t rows = static_cast<int64_t>(n.total) * n.heads;
+        const Tensor *output_given = optional_output(args[8], v, at::kBFloat16, rows * VALUE, "the output"),
+                     *lse_given = optional_output(args[9], v, at::kFloat, rows, "the LSE");
         Tensor output = output_given != nullptr ? *output_given : new_like(v);
         Tensor lse = lse_given != nullptr ? *lse_given
                      : cu == nullptr      ? new_tensor({n.batch, n.heads, n.longest}, v, at::kFloat)
@@ -443,9 +482,6 @@ DSCUDA_FUNCTION(prefill_backward) {
         const float scale = number(args[8]);
         const Tensor *cu = optional_tensor(args[9]), *workspace_given = optional_tensor(args[11]);
         const PrefillShape n = prefill_shape(q_nope, cu, args[10]);
-        Tensor workspace = workspace_given != nullptr
-                               ? *workspace_given
-                               : new_tensor({static_cast<int64_t>(dscuda_mla_prefill_backward_workspace_bytes(n.batch, n.longest, n.total, n.heads))}, v, at::kByte);
         Tensor grads[4];
         if (args[12] == Py_None) {
             at::DimVector sizes(q_nope.sizes().begin(), q_nope.sizes().end() - 1);
@@ -463,14 +499,20 @@ DSCUDA_FUNCTION(prefill_backward) {
             if (PySequence_Fast_GET_SIZE(items) != 4) {
                 fail(PyExc_ValueError, "grads is a sequence of four tensors");
             }
+            const int64_t total = n.total, rows = total * n.heads;
+            const int64_t elements[4] = {rows * 192, rows * VALUE, total * 64, rows * VALUE};
+            const char* names[4] = {"dq", "dk_nope", "dk_pe", "dv"};
             for (int i = 0; i < 4; ++i) {
-                PyObject* item = PySequence_Fast_GET_ITEM(items, i);
-                if (!THPVariable_Check(item)) {
+                const Tensor* grad = optional_output(PySequence_Fast_GET_ITEM(items, i), v, at::kBFloat16, elements[i], names[i]);
+                if (grad == nullptr) {
                     fail(PyExc_TypeError, "grads is a sequence of four tensors");
                 }
-                grads[i] = THPVariable_Unpack(item);
+                grads[i] = *grad;
             }
         }
+        Tensor workspace = workspace_given != nullptr
+                               ? *workspace_given
+                               : new_tensor({static_cast<int64_t>(dscuda_mla_prefill_backward_workspace_bytes(n.batch, n.longest, n.total, n.heads))}, v, at::kByte);
         const int nope = extent(q_nope, -1), rope = extent(q_pe, -1), value = extent(v, -1);
         void* stream = current_stream();
         checked(dscuda_mla_last_error, [&] {
