@@ -1378,6 +1378,9 @@ std::size_t ds_tiles_per_head(int batch_size, int max_sequence_length, int total
 }
 
 int ds_group_heads(int batch_size, int max_sequence_length, int total_tokens, int heads) {
+    if (batch_size <= 0 || max_sequence_length <= 0 || total_tokens <= 0 || heads <= 0) {
+        return 0;           // no tiles; the size queries get here with shapes that no backward accepts
+    }
     const std::size_t per_head = ds_tiles_per_head(batch_size, max_sequence_length, total_tokens) * DS_TILE_BYTES;
     const std::size_t fit = ds_scratch_limit.load() / per_head;
     return static_cast<int>(fit < static_cast<std::size_t>(heads) ? fit : static_cast<std::size_t>(heads));

@@ -6,6 +6,8 @@ reaches a launch)."""
 import ctypes
 import pathlib
 import re
+import subprocess
+import sys
 
 import pytest
 
@@ -70,6 +72,18 @@ def test_backward_workspace_follows_the_scratch_limit():
     finally:
         lib.dscuda_mla_prefill_backward_scratch_limit(previous)
     assert lib.dscuda_mla_prefill_backward_scratch_limit(-1) == previous
+
+
+@pytest.mark.parametrize("shape", [(0, 16, 16, 2), (1, 0, 16, 2), (1, 16, 0, 2), (1, 16, 16, 0), (-1, -1, 16, 2)])
+def test_backward_size_queries_survive_empty_shapes(shape):
+    """The queries take any sizes: the division by a head's tiles must not see zero.  In a child, since a trap would end the process."""
+    code = f"""if True:
+        from dscuda_b200 import library
+        lib = library.library("mla")
+        assert 0 <= lib.dscuda_mla_prefill_backward_workspace_bytes(*{shape}) <= 65536
+        assert lib.dscuda_mla_prefill_backward_launches(*{shape}, 0) == 4"""
+    done = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True)
+    assert done.returncode == 0, (done.returncode, done.stderr[-300:])
 
 
 @pytest.mark.parametrize("rank,rope", [(256, 64), (512, 32)])
