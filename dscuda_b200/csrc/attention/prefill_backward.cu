@@ -37,7 +37,9 @@
 #include <algorithm>
 #include <atomic>
 #include <cstddef>
+#include <cstdint>
 #include <stdexcept>
+#include <string>
 
 namespace dscuda {
 namespace {
@@ -1386,6 +1388,13 @@ int ds_group_heads(int batch_size, int max_sequence_length, int total_tokens, in
     return static_cast<int>(fit < static_cast<std::size_t>(heads) ? fit : static_cast<std::size_t>(heads));
 }
 
+// dk_pe sums, then delta [tokens, heads], then the per-head dk_pe contributions [tokens, heads, 64],
+// then dS^T of one group of heads
+std::size_t workspace_bytes_for(int group, int batch_size, int max_sequence_length, int total_tokens, int heads) {
+    return accumulator_bytes(total_tokens) + delta_bytes(total_tokens, heads) + parts_bytes(total_tokens, heads) +
+           static_cast<std::size_t>(group) * ds_tiles_per_head(batch_size, max_sequence_length, total_tokens) * DS_TILE_BYTES;
+}
+
 }  // namespace
 
 namespace internal {
@@ -1418,18 +1427,15 @@ std::size_t mla_prefill_backward_workspace_bytes(int batch_size, int max_sequenc
     if (total_tokens <= 0 || heads <= 0) {
         return 0;
     }
-    // dk_pe sums, then delta [tokens, heads], then the per-head dk_pe contributions [tokens, heads, 64],
-    // then dS^T of one group of heads
-    const std::size_t scratch = static_cast<std::size_t>(ds_group_heads(batch_size, max_sequence_length, total_tokens, heads)) *
-                                ds_tiles_per_head(batch_size, max_sequence_length, total_tokens) * DS_TILE_BYTES;
-    return accumulator_bytes(total_tokens) + delta_bytes(total_tokens, heads) + parts_bytes(total_tokens, heads) + scratch;
+    return workspace_bytes_for(ds_group_heads(batch_size, max_sequence_length, total_tokens, heads), batch_size, max_sequence_length, total_tokens, heads);
 }
 
-void mla_prefill_backward_cuda(__nv_bfloat16* dq, __nv_bfloat16* dk_nope, __nv_bfloat16* dk_pe, __nv_bfloat16* dv,
-                               const __nv_bfloat16* output_gradient, const __nv_bfloat16* output, const float* logsumexp,
-                               const __nv_bfloat16* q_nope, const __nv_bfloat16* q_pe, const __nv_bfloat16* k_nope, const __nv_bfloat16* k_pe,
-                               const __nv_bfloat16* v, const int* cu_seqlens, void* workspace, int batch_size, int max_sequence_length,
-                               int total_tokens, int heads, int nope_size, int rope_size, int value_size, float scale, cudaStream_t stream) {
+void mla_prefill_backward_sized_cuda(__nv_bfloat16* dq, __nv_bfloat16* dk_nope, __nv_bfloat16* dk_pe, __nv_bfloat16* dv,
+                                     const __nv_bfloat16* output_gradient, const __nv_bfloat16* output, const float* logsumexp,
+                                     const __nv_bfloat16* q_nope, const __nv_bfloat16* q_pe, const __nv_bfloat16* k_nope,
+                                     const __nv_bfloat16* k_pe, const __nv_bfloat16* v, const int* cu_seqlens, void* workspace,
+                                     std::size_t workspace_bytes, int batch_size, int max_sequence_length, int total_tokens, int heads,
+                                     int nope_size, int rope_size, int value_size, float scale, cudaStream_t stream) {
     internal::check_prefill_shape(cu_seqlens, batch_size, max_sequence_length, total_tokens, heads, nope_size, rope_size, value_size, scale);
     for (const void* pointer : {static_cast<const void*>(dq), static_cast<const void*>(dk_nope), static_cast<const void*>(dk_pe),
                                 static_cast<const void*>(dv), static_cast<const void*>(output_gradient), static_cast<const void*>(output),
@@ -1442,6 +1448,13 @@ void mla_prefill_backward_cuda(__nv_bfloat16* dq, __nv_bfloat16* dk_nope, __nv_b
         if ((reinterpret_cast<std::uintptr_t>(pointer) & 15U) != 0) {
             throw std::invalid_argument("tensor pointers must be 16-byte aligned");
         }
+    }
+    // the limit is read once: what is checked here is what the launches below use
+    const int group = ds_group_heads(batch_size, max_sequence_length, total_tokens, heads);
+    const std::size_t needed = workspace_bytes_for(group, batch_size, max_sequence_length, total_tokens, heads);
+    if (workspace_bytes < needed) {
+        throw std::invalid_argument("MLA backward needs a workspace of " + std::to_string(needed) + " bytes under the present scratch limit, got " +
+                                    std::to_string(workspace_bytes));
     }
     float* accumulator = static_cast<float*>(workspace);
     float* delta = reinterpret_cast<float*>(static_cast<char*>(workspace) + accumulator_bytes(total_tokens));
@@ -1487,7 +1500,6 @@ void mla_prefill_backward_cuda(__nv_bfloat16* dq, __nv_bfloat16* dk_nope, __nv_b
     const unsigned delta_blocks = static_cast<unsigned>(pairs / 8 + 1 < 148 * 32 ? pairs / 8 + 1 : 148 * 32);
     launch_chained(delta_kernel, dim3(delta_blocks), dim3(256), 0, stream, delta, output_gradient, output, cu_seqlens, batch_size, max_sequence_length, total_tokens, heads);
 
-    const int group = ds_group_heads(batch_size, max_sequence_length, total_tokens, heads);
     if (group > 0) {
         // per group of heads: the key-side kernel (which leaves dS^T in the scratch) and then dQ from it
         params.ds_scratch = reinterpret_cast<__nv_bfloat16*>(static_cast<char*>(workspace) + accumulator_bytes(total_tokens) + delta_bytes(total_tokens, heads) +
@@ -1525,6 +1537,16 @@ void mla_prefill_backward_cuda(__nv_bfloat16* dq, __nv_bfloat16* dk_nope, __nv_b
     const std::size_t sum_blocks = std::min<std::size_t>((static_cast<std::size_t>(total_tokens) + SUM_ROWS - 1) / SUM_ROWS, 148 * 8);
     launch_chained(sum_dk_pe_kernel, dim3(static_cast<unsigned>(sum_blocks)), dim3(SUM_ROWS * 16 * SUM_QUARTERS), 0, stream, dk_pe, accumulator,
                    reinterpret_cast<const float4*>(parts), static_cast<std::size_t>(total_tokens), heads);
+}
+
+void mla_prefill_backward_cuda(__nv_bfloat16* dq, __nv_bfloat16* dk_nope, __nv_bfloat16* dk_pe, __nv_bfloat16* dv,
+                               const __nv_bfloat16* output_gradient, const __nv_bfloat16* output, const float* logsumexp,
+                               const __nv_bfloat16* q_nope, const __nv_bfloat16* q_pe, const __nv_bfloat16* k_nope, const __nv_bfloat16* k_pe,
+                               const __nv_bfloat16* v, const int* cu_seqlens, void* workspace, int batch_size, int max_sequence_length,
+                               int total_tokens, int heads, int nope_size, int rope_size, int value_size, float scale, cudaStream_t stream) {
+    mla_prefill_backward_sized_cuda(dq, dk_nope, dk_pe, dv, output_gradient, output, logsumexp, q_nope, q_pe, k_nope, k_pe, v, cu_seqlens,
+                                    workspace, SIZE_MAX, batch_size, max_sequence_length, total_tokens, heads, nope_size, rope_size,
+                                    value_size, scale, stream);
 }
 
 }  // namespace dscuda

@@ -147,6 +147,18 @@ extern "C" int dscuda_mla_prefill_backward(bf16* dq, bf16* dk_nope, bf16* dk_pe,
     });
 }
 
+extern "C" int dscuda_mla_prefill_backward_sized(bf16* dq, bf16* dk_nope, bf16* dk_pe, bf16* dv, const bf16* dout, const bf16* output,
+                                                 const float* lse, const bf16* q_nope, const bf16* q_pe, const bf16* k_nope,
+                                                 const bf16* k_pe, const bf16* v, const int* cu_seqlens, void* workspace,
+                                                 std::size_t workspace_bytes, int batch, int max_sequence, int total_tokens, int heads,
+                                                 int nope, int rope, int value, float scale, cudaStream_t stream) {
+    return guarded([&] {
+        dscuda::mla_prefill_backward_sized_cuda(dq, dk_nope, dk_pe, dv, dout, output, lse, q_nope, q_pe, k_nope, k_pe, v, cu_seqlens,
+                                                workspace, workspace_bytes, batch, max_sequence, total_tokens, heads, nope, rope, value,
+                                                scale, stream);
+    });
+}
+
 extern "C" int dscuda_mla_up_project(bf16* k_nope, bf16* v, const bf16* kv_latent, const bf16* w_uk, const bf16* w_uv, long long rows, int heads,
                                      cudaStream_t stream) {
     return guarded([&] { dscuda::mla_up_project_cuda(k_nope, v, kv_latent, w_uk, w_uv, rows, heads, stream); });

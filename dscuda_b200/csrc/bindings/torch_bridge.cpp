@@ -480,8 +480,10 @@ DSCUDA_FUNCTION(prefill_backward) {
         const Tensor &dout = tensor(args[0]), &output = tensor(args[1]), &lse = tensor(args[2]), &q_nope = tensor(args[3]), &q_pe = tensor(args[4]),
                      &k_nope = tensor(args[5]), &k_pe = tensor(args[6]), &v = tensor(args[7]);
         const float scale = number(args[8]);
-        const Tensor *cu = optional_tensor(args[9]), *workspace_given = optional_tensor(args[11]);
+        const Tensor* cu = optional_tensor(args[9]);
         const PrefillShape n = prefill_shape(q_nope, cu, args[10]);
+        const size_t workspace_bytes = dscuda_mla_prefill_backward_workspace_bytes(n.batch, n.longest, n.total, n.heads);
+        const Tensor* workspace_given = optional_workspace(args[11], v, workspace_bytes);
         Tensor grads[4];
         if (args[12] == Py_None) {
             at::DimVector sizes(q_nope.sizes().begin(), q_nope.sizes().end() - 1);
@@ -510,16 +512,14 @@ DSCUDA_FUNCTION(prefill_backward) {
                 grads[i] = *grad;
             }
         }
-        Tensor workspace = workspace_given != nullptr
-                               ? *workspace_given
-                               : new_tensor({static_cast<int64_t>(dscuda_mla_prefill_backward_workspace_bytes(n.batch, n.longest, n.total, n.heads))}, v, at::kByte);
+        Tensor workspace = workspace_given != nullptr ? *workspace_given : new_tensor({static_cast<int64_t>(workspace_bytes)}, v, at::kByte);
         const int nope = extent(q_nope, -1), rope = extent(q_pe, -1), value = extent(v, -1);
         void* stream = current_stream();
         checked(dscuda_mla_last_error, [&] {
-            return dscuda_mla_prefill_backward(pointer(grads[0]), pointer(grads[1]), pointer(grads[2]), pointer(grads[3]), pointer(dout), pointer(output),
-                                               static_cast<const float*>(pointer(lse)), pointer(q_nope), pointer(q_pe), pointer(k_nope), pointer(k_pe),
-                                               pointer(v), int_pointer(cu), pointer(workspace), n.batch, n.longest, n.total, n.heads, nope, rope, value,
-                                               scale, stream);
+            return dscuda_mla_prefill_backward_sized(pointer(grads[0]), pointer(grads[1]), pointer(grads[2]), pointer(grads[3]), pointer(dout),
+                                                     pointer(output), static_cast<const float*>(pointer(lse)), pointer(q_nope), pointer(q_pe),
+                                                     pointer(k_nope), pointer(k_pe), pointer(v), int_pointer(cu), pointer(workspace),
+                                                     workspace.nbytes(), n.batch, n.longest, n.total, n.heads, nope, rope, value, scale, stream);
         });
         if (args[12] != Py_None) {
             Py_INCREF(args[12]);

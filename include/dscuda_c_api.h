@@ -136,6 +136,16 @@ int dscuda_mla_prefill_backward(
     int batch, int max_sequence, int total_tokens, int heads,
     int nope, int rope, int value, float scale, void* stream);
 
+/* No counterpart in the reference (mla_prefill_backward_sized_cuda): the same with the size of the workspace,
+ * refused when the scratch limit in force asks for more. */
+int dscuda_mla_prefill_backward_sized(
+    void* dq, void* dk_nope, void* dk_pe, void* dv,
+    const void* dout, const void* output, const float* lse,
+    const void* q_nope, const void* q_pe, const void* k_nope, const void* k_pe, const void* v,
+    const int* cu_seqlens, void* workspace, size_t workspace_bytes,
+    int batch, int max_sequence, int total_tokens, int heads,
+    int nope, int rope, int value, float scale, void* stream);
+
 /* No counterpart in the reference (include/mla.h, mla_up_project_cuda): k_nope [rows,H,128] =
  * kv_latent [rows,512] W_UK^T and v = kv_latent W_UV^T, weights [H*128,512]; k_nope or v may be NULL. */
 int dscuda_mla_up_project(

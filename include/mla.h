@@ -208,7 +208,7 @@ void mla_prefill_forward_cuda(
 // heads as fit in the limit set here (default 20 GiB; the call returns the previous limit, a negative
 // value only reads it).  When not even one head fits, dQ comes from a kernel that recomputes S and dP
 // instead and the workspace is small.  Set the limit before asking for the workspace size and keep it
-// unchanged until the backward call that uses that workspace.
+// unchanged until the backward call that uses that workspace, or hand its size to mla_prefill_backward_sized_cuda.
 std::size_t mla_prefill_backward_scratch_limit(long long bytes);
 
 // Kernels one mla_prefill_backward_cuda call launches for this shape (`packed` is ignored: dense and
@@ -244,6 +244,34 @@ void mla_prefill_backward_cuda(
     const __nv_bfloat16* v,
     const int* cu_seqlens,
     void* workspace,
+    int batch_size,
+    int max_sequence_length,
+    int total_tokens,
+    int heads,
+    int nope_size,
+    int rope_size,
+    int value_size,
+    float scale,
+    cudaStream_t stream = nullptr);
+
+// The same with the size of the workspace: throws std::invalid_argument when the workspace is smaller than the
+// call needs under the scratch limit in force (which another thread may have raised since the workspace was made).
+void mla_prefill_backward_sized_cuda(
+    __nv_bfloat16* dq,
+    __nv_bfloat16* dk_nope,
+    __nv_bfloat16* dk_pe,
+    __nv_bfloat16* dv,
+    const __nv_bfloat16* output_gradient,
+    const __nv_bfloat16* output,
+    const float* logsumexp,
+    const __nv_bfloat16* q_nope,
+    const __nv_bfloat16* q_pe,
+    const __nv_bfloat16* k_nope,
+    const __nv_bfloat16* k_pe,
+    const __nv_bfloat16* v,
+    const int* cu_seqlens,
+    void* workspace,
+    std::size_t workspace_bytes,
     int batch_size,
     int max_sequence_length,
     int total_tokens,

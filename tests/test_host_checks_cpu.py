@@ -80,6 +80,27 @@ def test_refused(call):
         call()
 
 
+def test_backward_workspace_of_a_lower_limit_is_refused():
+    """The scratch limit belongs to the process: a workspace made under a lower one is too small once the limit is raised."""
+    from dscuda_b200.library import library
+    shape = (BATCH, SEQ, BATCH * SEQ, HEADS)
+    previous = mla.prefill_backward_scratch_limit(0)
+    try:
+        low = library("mla").dscuda_mla_prefill_backward_workspace_bytes(*shape)
+        mla.prefill_backward_scratch_limit(1 << 30)
+        high = library("mla").dscuda_mla_prefill_backward_workspace_bytes(*shape)
+        assert high > low
+        for packed in (False, True):
+            with pytest.raises(ValueError, match="workspace"):
+                backward(grads=gradients(), workspace=fake(low, dtype=U8), packed=packed)
+            with pytest.raises(ValueError, match="device"):
+                backward(grads=gradients(), workspace=fake(high, dtype=U8, device="cuda:1"), packed=packed)
+            with pytest.raises(RuntimeError, match="[Dd]river|data pointer|storage"):
+                backward(grads=gradients(), workspace=fake(high, dtype=U8), packed=packed)
+    finally:
+        mla.prefill_backward_scratch_limit(previous)
+
+
 def test_host_memory_is_refused():
     with pytest.raises(RuntimeError, match="no CPU path"):
         decode(output=torch.empty(BATCH, 1, HEADS, 512, dtype=BF16))

@@ -114,6 +114,16 @@ def test_prefill_entry_points_validate_on_the_host():
     assert b"null tensor pointer" in lib.dscuda_mla_last_error()
 
 
+def test_sized_backward_refuses_a_small_workspace():
+    """The native check behind the one of the host layer: the size and the scratch limit are looked at in one place, before the first
+    launch (the pointers are made up and never read)."""
+    lib = library.library("mla")
+    needed = lib.dscuda_mla_prefill_backward_workspace_bytes(1, 16, 16, 2)
+    pointers = [ctypes.c_void_p(4096)] * 12 + [None, ctypes.c_void_p(4096)]
+    assert lib.dscuda_mla_prefill_backward_sized(*pointers, needed - 1, 1, 16, 16, 2, 128, 64, 128, 0.1, None) == 1
+    assert f"{needed} bytes".encode() in lib.dscuda_mla_last_error()
+
+
 def test_flash_entry_point_validates_on_the_host():
     lib = library.library("flash_attention")
     assert lib.dscuda_flash_forward(None, None, None, None, None, 1, 64, 4, 2, 64, 0.1, None) == 1
