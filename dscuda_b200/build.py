@@ -5,8 +5,8 @@
 Outputs `build/libdscuda_mla_bench.so` and
 `build/libdscuda_flash_attention_bench.so` at the repository root, the names the
 reference's harness loads (`benchmarks/common.py:19-20`), and
-`build/_dscuda_torch.so`, the extension `dscuda_b200.mla` calls them through.  nvcc cross-compiles,
-so no GPU is needed to build.
+`build/_dscuda_torch.so`, the extension `dscuda_b200.mla` calls them through, for the torch of the
+interpreter this runs under (left out if it has none).  nvcc cross-compiles, so no GPU is needed to build.
 """
 
 from __future__ import annotations
@@ -20,7 +20,8 @@ import sys
 ROOT = pathlib.Path(__file__).resolve().parents[1]
 BUILD = ROOT / "build"
 # the two product libraries, the Python extension over them, then the test-only probe library (tests/csrc)
-LIBRARIES = ("libdscuda_mla_bench.so", "libdscuda_flash_attention_bench.so", "_dscuda_torch.so", "libdscuda_test_probes.so")
+EXTENSION = "_dscuda_torch.so"
+LIBRARIES = ("libdscuda_mla_bench.so", "libdscuda_flash_attention_bench.so", EXTENSION, "libdscuda_test_probes.so")
 
 
 def _tool(name: str) -> str:
@@ -48,7 +49,9 @@ def build(verbose: bool = False) -> list[pathlib.Path]:
         done = subprocess.run(command, stdout=sink, stderr=subprocess.STDOUT, text=True)
         if done.returncode != 0:
             raise RuntimeError(f"{' '.join(command)} failed:\n{done.stdout or ''}")
-    paths = [BUILD / name for name in LIBRARIES]
+    # configured without a torch (CMakeLists.txt says so), the build leaves the extension out
+    extension_built = "DSCUDA_EXTENSION:INTERNAL=ON" in (work / "CMakeCache.txt").read_text()
+    paths = [BUILD / name for name in LIBRARIES if extension_built or name != EXTENSION]
     for path in paths:
         if not path.exists():
             raise RuntimeError(f"build finished without producing {path}")

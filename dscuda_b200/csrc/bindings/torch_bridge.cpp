@@ -13,6 +13,7 @@
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/utils/object_ptr.h>
+#include <torch/version.h>
 
 #include <Python.h>
 
@@ -561,5 +562,16 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_dscuda_torch", nullptr, -1, metho
 }  // namespace
 
 PyMODINIT_FUNC PyInit__dscuda_torch() {
-    return PyModule_Create(&module);
+    // The extension is compiled against one Python and one torch; library.py compares the latter.
+    static const std::string python = std::to_string(PY_MAJOR_VERSION) + "." + std::to_string(PY_MINOR_VERSION) + ".";
+    if (std::string(Py_GetVersion()).compare(0, python.size(), python) != 0) {
+        PyErr_SetString(PyExc_ImportError, ("built for Python " + python + "x").c_str());
+        return nullptr;
+    }
+    PyObject* result = PyModule_Create(&module);
+    if (result != nullptr && PyModule_AddStringConstant(result, "torch_version", TORCH_VERSION) != 0) {
+        Py_DECREF(result);
+        return nullptr;
+    }
+    return result;
 }

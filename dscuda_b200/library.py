@@ -13,6 +13,8 @@ import importlib.machinery
 import importlib.util
 import os
 import pathlib
+import re
+import sys
 
 ROOT = pathlib.Path(__file__).resolve().parents[1]
 P, I, F = ctypes.c_void_p, ctypes.c_int, ctypes.c_float
@@ -76,15 +78,22 @@ def library(name: str) -> ctypes.CDLL:
 
 @functools.lru_cache(maxsize=None)
 def extension():
-    """The Python extension over both libraries (`csrc/bindings/torch_bridge.cpp`): torch tensors in, C-ABI calls out."""
-    import torch  # noqa: F401 (its shared libraries must be loaded first)
+    """The Python extension over both libraries (`csrc/bindings/torch_bridge.cpp`): torch tensors in, C-ABI calls out.
+    It belongs to one torch and one Python; the libraries themselves need neither."""
+    import torch  # its shared libraries must be loaded first
 
     library("mla"), library("flash_attention")
     name = "_dscuda_torch"
     path = str(_built(build_directory() / f"{name}.so"))
     loader = importlib.machinery.ExtensionFileLoader(name, path)
-    module = importlib.util.module_from_spec(importlib.util.spec_from_file_location(name, path, loader=loader))
-    loader.exec_module(module)
+    again = f"run `python -m dscuda_b200.build` with the interpreter that uses it ({sys.executable})"
+    try:
+        module = importlib.util.module_from_spec(importlib.util.spec_from_file_location(name, path, loader=loader))
+        loader.exec_module(module)
+    except ImportError as error:
+        raise RuntimeError(f"{path} does not load into torch {torch.__version__}: {error}; {again}") from error
+    if re.match(r"\d+\.\d+\.\d+", torch.__version__)[0] != module.torch_version:        # pre-release and build suffixes aside
+        raise RuntimeError(f"{path} was built for torch {module.torch_version}, this is {torch.__version__}; {again}")
     return module
 
 
