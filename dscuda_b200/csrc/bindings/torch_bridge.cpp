@@ -390,10 +390,10 @@ DSCUDA_FUNCTION(up_project) {
         expect_arguments(count, 4);
         const Tensor &latent = tensor(args[0]), &w_uk = tensor(args[1]), &w_uv = tensor(args[2]);
         const int heads = static_cast<int>(integer(args[3]));
+        const long long rows = row_count(latent, latent.size(-1));          // size() refuses a tensor without dimensions
         at::DimVector sizes(latent.sizes().begin(), latent.sizes().end() - 1);
         sizes.push_back(heads);
         sizes.push_back(128);
-        const long long rows = row_count(latent, latent.size(-1));
         Tensor k_nope = new_tensor(sizes, latent, at::kBFloat16), v = new_tensor(sizes, latent, at::kBFloat16);
         void* stream = current_stream();
         checked(dscuda_mla_last_error,

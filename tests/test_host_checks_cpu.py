@@ -12,7 +12,7 @@ F32, BF16, I32, U8 = torch.float32, torch.bfloat16, torch.int32, torch.uint8
 
 def fake(*shape, dtype=BF16, device="cuda:0"):
     with FakeTensorMode():
-        return torch.empty(*shape, dtype=dtype, device=device)
+        return torch.empty(shape, dtype=dtype, device=device)
 
 
 def strided(*shape, dtype=BF16):
@@ -120,3 +120,14 @@ def test_what_fits_is_accepted(call):
     """The call gets past the checks: what ends it is the missing storage or, without a driver, the question for the stream."""
     with pytest.raises(RuntimeError, match="[Dd]river|data pointer|storage"):
         call()
+
+
+@pytest.mark.parametrize("call", [
+    lambda x: mla.up_project(x, fake(128, 512), fake(128, 512), 1),
+    lambda x: mla.absorb_query(x, fake(128, 512)),
+    lambda x: mla.unabsorb_output(x, fake(128, 512)),
+    lambda x: mla.rope_apply(x),
+], ids=["up_project", "absorb_query", "unabsorb_output", "rope"])
+def test_tensor_without_dimensions(call):
+    with pytest.raises(IndexError):
+        call(fake())
