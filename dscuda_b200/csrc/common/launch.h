@@ -28,7 +28,11 @@ void launch_chained(void (*kernel)(Parameters...), dim3 grid, dim3 block, std::s
     config.stream = stream;
     config.attrs = &attribute;
     config.numAttrs = 1;
-    CUDA_CHECK(cudaLaunchKernelEx(&config, kernel, std::forward<Arguments>(arguments)...));
+    const cudaError_t result = cudaLaunchKernelEx(&config, kernel, std::forward<Arguments>(arguments)...);
+    if (result != cudaSuccess) {
+        (void)cudaGetLastError();       // reported here: the caller's next check must not find it again
+    }
+    CUDA_CHECK(result);
 }
 
 }  // namespace dscuda

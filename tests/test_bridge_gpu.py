@@ -1,4 +1,7 @@
 """What the native host layer refuses, and with which exception: nothing of it reaches a kernel."""
+import ctypes
+import pathlib
+
 import pytest
 import torch
 
@@ -47,3 +50,9 @@ def test_longest_sequence_as_any_number(longest):
     packed = mla.prefill_forward(*inputs, 0.1, cu, longest)
     dense = mla.prefill_forward(*(x[None] for x in inputs), 0.1)
     assert torch.equal(packed[0], dense[0][0]) and torch.equal(packed[1], dense[1][0])
+
+
+def test_a_refused_launch_leaves_no_error_behind():
+    """The host refuses the launch (too many threads to a block); the next check of the caller's must not find its error."""
+    lib = ctypes.CDLL(str(pathlib.Path(__file__).resolve().parents[1] / "build" / "libdscuda_test_probes.so"))
+    assert lib.dscuda_test_failed_launch() == 0
