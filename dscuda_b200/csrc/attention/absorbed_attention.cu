@@ -461,7 +461,7 @@ __device__ __forceinline__ void absorbed_pair_body(const DecodeParams& p) {
                 if (half_tile < w.first || half_tile >= w.first + 32) {
                     w.first = half_tile & ~31;
                     const int token = min((w.first + lane) * HALF_KEYS, last_half_start);     // a half past the end rereads the last one; it is masked
-                    int page = __ldg(p.block_table + static_cast<size_t>(seg.b) * p.pages + token / p.page_size);
+                    int page = p.block_table[static_cast<size_t>(seg.b) * p.pages + token / p.page_size];
                     if (p.cache_blocks > 0 && static_cast<unsigned>(page) >= static_cast<unsigned>(p.cache_blocks)) {
                         atomicExch(&decode_status, STATUS_BAD_INDEX);       // a page number outside the cache: read page 0 instead and report it
                         page = 0;

@@ -129,8 +129,8 @@ __global__ void __launch_bounds__(256) absorbed_delta_kernel(__nv_bfloat16* dq_r
         float sum = 0.0F;
 #pragma unroll
         for (int part = 0; part < 2; ++part) {
-            const uint4 a = __ldg(reinterpret_cast<const uint4*>(dout + row * RANK) + part * 32 + lane);
-            const uint4 b = __ldg(reinterpret_cast<const uint4*>(out + row * RANK) + part * 32 + lane);
+            const uint4 a = reinterpret_cast<const uint4*>(dout + row * RANK)[part * 32 + lane];
+            const uint4 b = reinterpret_cast<const uint4*>(out + row * RANK)[part * 32 + lane];
             const __nv_bfloat162* a2 = reinterpret_cast<const __nv_bfloat162*>(&a);
             const __nv_bfloat162* b2 = reinterpret_cast<const __nv_bfloat162*>(&b);
 #pragma unroll

@@ -64,11 +64,11 @@ __global__ void __launch_bounds__(APPEND_THREADS) cache_append_kernel(uint4* cac
         uint4* dst = cache + (static_cast<long long>(physical_page) * page_size + position % page_size) * ROW_UNITS;
         const uint4* src_latent = latent + item * LATENT_UNITS;
         const uint4* src_rope = rope + item * ROPE_UNITS;
-        const uint4 first = __ldg(src_latent + lane);
-        const uint4 second = __ldg(src_latent + 32 + lane);
+        const uint4 first = src_latent[lane];
+        const uint4 second = src_latent[32 + lane];
         uint4 third = make_uint4(0, 0, 0, 0);
         if (lane < ROPE_UNITS) {
-            third = __ldg(src_rope + lane);
+            third = src_rope[lane];
         }
         dst[lane] = first;
         dst[32 + lane] = second;
@@ -126,7 +126,8 @@ __global__ void __launch_bounds__(APPEND_THREADS) cache_append_fp8_kernel(uint8_
         }
         uint8_t* dst = cache + (static_cast<long long>(physical_page) * page_size + position % page_size) * FP8_ROW_BYTES;
         // 16 latent columns per lane: two 16-byte units of bf16
-        const uint4 raw[2] = {__ldg(latent + item * LATENT_UNITS + 2 * lane), __ldg(latent + item * LATENT_UNITS + 2 * lane + 1)};
+        const uint4 rotary = lane < ROPE_UNITS ? rope[item * ROPE_UNITS + lane] : make_uint4(0, 0, 0, 0);
+        const uint4 raw[2] = {latent[item * LATENT_UNITS + 2 * lane], latent[item * LATENT_UNITS + 2 * lane + 1]};
         float values[16];
         const __nv_bfloat162* pairs = reinterpret_cast<const __nv_bfloat162*>(raw);
         float amax = 0.0F;
@@ -154,7 +155,7 @@ __global__ void __launch_bounds__(APPEND_THREADS) cache_append_fp8_kernel(uint8_
             reinterpret_cast<float*>(dst + FP8_SCALES_OFFSET)[lane >> 3] = scale;
         }
         if (lane < ROPE_UNITS) {
-            reinterpret_cast<uint4*>(dst + FP8_ROPE_OFFSET)[lane] = __ldg(rope + item * ROPE_UNITS + lane);
+            reinterpret_cast<uint4*>(dst + FP8_ROPE_OFFSET)[lane] = rotary;
         }
     }
 }
@@ -176,10 +177,10 @@ __global__ void __launch_bounds__(APPEND_THREADS) cache_dequantize_fp8_kernel(ui
             const uint8_t* src = fp8_cache + min(first + i, rows - 1) * FP8_ROW_BYTES;
 #pragma unroll
             for (int half = 0; half < 2; ++half) {
-                codes[i][half] = __ldg(reinterpret_cast<const uint2*>(src) + half * 32 + lane);
-                scales[i][half] = __ldg(reinterpret_cast<const float*>(src + FP8_SCALES_OFFSET) + half * 2 + (lane >> 4));
+                codes[i][half] = reinterpret_cast<const uint2*>(src)[half * 32 + lane];
+                scales[i][half] = reinterpret_cast<const float*>(src + FP8_SCALES_OFFSET)[half * 2 + (lane >> 4)];
             }
-            rope[i] = lane < ROPE_UNITS ? __ldg(reinterpret_cast<const uint4*>(src + FP8_ROPE_OFFSET) + lane) : make_uint4(0, 0, 0, 0);
+            rope[i] = lane < ROPE_UNITS ? reinterpret_cast<const uint4*>(src + FP8_ROPE_OFFSET)[lane] : make_uint4(0, 0, 0, 0);
         }
 #pragma unroll
         for (int i = 0; i < PASS; ++i) {

@@ -264,8 +264,8 @@ __global__ void __launch_bounds__(256) delta_kernel(float* delta, const __nv_bfl
         const size_t pair = base + half;
         float sum = 0.0F;
         if (pair < pairs) {
-            const uint4 a = __ldg(reinterpret_cast<const uint4*>(dout + pair * 128) + part);
-            const uint4 b = __ldg(reinterpret_cast<const uint4*>(out + pair * 128) + part);
+            const uint4 a = reinterpret_cast<const uint4*>(dout + pair * 128)[part];
+            const uint4 b = reinterpret_cast<const uint4*>(out + pair * 128)[part];
             const __nv_bfloat162* a2 = reinterpret_cast<const __nv_bfloat162*>(&a);
             const __nv_bfloat162* b2 = reinterpret_cast<const __nv_bfloat162*>(&b);
 #pragma unroll
@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(SUM_ROWS * 16 * SUM_QUARTERS) sum_dk_pe_kernel
             const float4* src = parts + (index / 16) * static_cast<size_t>(heads) * 16 + index % 16;
 #pragma unroll 8
             for (int h = head_begin; h < head_end; ++h) {
-                const float4 x = __ldg(src + static_cast<size_t>(h) * 16);
+                const float4 x = src[static_cast<size_t>(h) * 16];
                 total.x += x.x;
                 total.y += x.y;
                 total.z += x.z;

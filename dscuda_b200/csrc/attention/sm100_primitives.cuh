@@ -37,8 +37,8 @@ __device__ __forceinline__ uint32_t lane_id() {
 }
 
 // ---------------------------------------------------------------------------
-// Dependent launches (../common/launch.h).  The wait comes before the first access to global memory; at least one
-// block of every grid has to reach it, or the grid could end before the one in front of it.
+// Dependent launches (../common/launch.h).  The wait comes before the first access to memory that another kernel writes; at
+// least one block of every grid has to reach it, or the grid could end before the one in front of it.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void grid_dependency_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -10,12 +10,14 @@
 
 namespace dscuda {
 
-// Programmatic dependent launch: the grid's blocks may start while the last blocks of the preceding grid drain, so its
-// launch latency, barrier set-up and tensor-memory allocation overlap that tail.  Every kernel launched this way calls
-// sm100::grid_dependency_wait() before it touches global memory; that returns when the preceding grid has ended and its
-// writes are visible.  No kernel lets its dependents go early (griddepcontrol.launch_dependents): blocks of the next grid
-// that sit beside a running decode slowed it (8 ragged sequences, 128 heads: 35.3 us without, 41-44 us with), and nothing
-// else gained.
+// Programmatic dependent launch: the blocks of a grid may start when every block of the preceding grid has exited, so its
+// launch latency, barrier set-up and tensor-memory allocation overlap the end of that grid (the flush of its writes).
+// Every kernel launched this way calls sm100::grid_dependency_wait() before it touches memory that another kernel writes; that
+// returns when the preceding grid has ended and its writes are visible.  The one thing read earlier is the kernel family's own
+// status word.  Loads are plain, not ld.global.nc: that form wants memory that nothing writes while the kernel lives, and its
+// life begins before the grid in front has ended.  No kernel lets its dependents go early
+// (griddepcontrol.launch_dependents): blocks of the next grid that sit beside a running decode slowed it (8 ragged sequences,
+// 128 heads: 35.3 us without, 41-44 us with), and nothing else gained.
 template <class... Parameters, class... Arguments>
 void launch_chained(void (*kernel)(Parameters...), dim3 grid, dim3 block, std::size_t shared_bytes, cudaStream_t stream, Arguments&&... arguments) {
     cudaLaunchAttribute attribute{};
