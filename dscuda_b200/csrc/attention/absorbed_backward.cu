@@ -225,6 +225,7 @@ struct Shared {
     uint64_t rows_done[2];      // eight softmax warps have read them
     uint32_t tmem_base;
     int abort_flag;
+    int latched;                // an earlier launch ran into a time limit
 };
 static_assert(sizeof(Shared) <= SMEM_BYTES - MISC_OFFSET, "key-side barrier block too large");
 }  // namespace ks
@@ -232,7 +233,6 @@ static_assert(sizeof(Shared) <= SMEM_BYTES - MISC_OFFSET, "key-side barrier bloc
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ks::KEY_THREADS, 1) absorbed_backward_key_kernel(const __grid_constant__ AbsorbedBackwardParams p) {
     using namespace ks;
     extern __shared__ uint8_t smem_raw[];
-    // No early exit on a status left by an earlier launch: both CTAs have to take the same path to the cluster barriers.
     const int warp = threadIdx.x / 32;
     const int lane = threadIdx.x % 32;
     const uint32_t rank = cluster_cta_rank();
@@ -286,6 +286,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ks::KEY_THREADS, 1) 
         tma_prefetch_descriptor(&p.row_do4);
         tma_prefetch_descriptor(&p.row_do2);
         tma_prefetch_descriptor(&p.row_rope);
+        sh->latched = *reinterpret_cast<volatile int*>(&absorbed_backward_status) == STATUS_WAIT_TIMEOUT;
     }
     tc_fence_before_sync();
     __syncthreads();
@@ -295,7 +296,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ks::KEY_THREADS, 1) 
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&sh->tmem_base);
     auto wait = [&](uint64_t& bar, int phase) { return mbar_wait(smem_u32(&bar), phase & 1, abort_flag, &absorbed_backward_status); };
 
-    if (warp == LOAD_WARP) {
+    if (pair_flag(&sh->latched, rank)) {
+        // both CTAs leave through the teardown
+    } else if (warp == LOAD_WARP) {
         // =================== TMA producer ===================================
         if (lane == 0) {
             // the bytes of both CTAs are counted by the leader's barrier
@@ -710,6 +713,7 @@ struct Shared {
     uint64_t ds_full;
     uint32_t tmem_base;
     int abort_flag;
+    int latched;                // an earlier launch ran into a time limit
 };
 static_assert(sizeof(Shared) <= SMEM_BYTES - MISC_OFFSET, "query-side barrier block too large");
 }  // namespace qs
@@ -757,6 +761,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) absorbed
         tma_prefetch_descriptor(&p.stream_k4);
         tma_prefetch_descriptor(&p.stream_k2);
         tma_prefetch_descriptor(&p.stream_rope);
+        sh->latched = *reinterpret_cast<volatile int*>(&absorbed_backward_status) == STATUS_WAIT_TIMEOUT;
     }
     tc_fence_before_sync();
     __syncthreads();
@@ -766,7 +771,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) absorbed
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&sh->tmem_base);
     auto wait = [&](uint64_t& bar, int phase) { return mbar_wait(smem_u32(&bar), phase & 1, abort_flag, &absorbed_backward_status); };
 
-    if (warp == LOAD_WARP) {
+    if (pair_flag(&sh->latched, rank)) {
+        // both CTAs leave through the teardown
+    } else if (warp == LOAD_WARP) {
         // =================== TMA producer ===================================
         if (lane == 0) {
             // the bytes of both CTAs are counted by the leader's barrier

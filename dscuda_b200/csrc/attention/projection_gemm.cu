@@ -320,6 +320,7 @@ struct PairShared {
     uint64_t acc_empty[2];                  // leader: one arrival per epilogue warp of either CTA
     uint32_t tmem_base;
     int abort_flag;
+    int latched;                            // an earlier launch ran into a time limit
 };
 static_assert(sizeof(PairShared) <= MISC_BYTES, "barrier block too large");
 }  // namespace pk
@@ -366,6 +367,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) projecti
         tma_prefetch_descriptor(&p.a);
         tma_prefetch_descriptor(&p.b[0]);
         tma_prefetch_descriptor(&p.c[0]);
+        sh->latched = *reinterpret_cast<volatile int*>(&projection_status) == STATUS_WAIT_TIMEOUT;
     }
     tc_fence_before_sync();
     __syncthreads();
@@ -383,7 +385,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) projecti
     // a column of tiles (batch entry, n) shares its B tile
     auto column_of = [&](long long tile) { return static_cast<int>(tile / tiles_m); };
 
-    if (warp == LOAD_WARP) {
+    if (pair_flag(&sh->latched, rank)) {
+        // both CTAs leave through the teardown
+    } else if (warp == LOAD_WARP) {
         if (lane == 0) {
             bool alive = true;
             long long chunk = 0;

@@ -14,9 +14,10 @@ namespace dscuda {
 namespace sm100 {
 
 // ---------------------------------------------------------------------------
-// Device status word.  A wait that runs out sets it; every kernel in the same
-// translation unit checks it on entry and leaves at once when it is set, so a
-// broken pipeline costs one time limit, not one per CTA.
+// Device status word.  A wait that runs out sets it; the kernels with such waits in
+// the same translation unit check it on entry and leave at once when it is set, so a
+// broken pipeline costs one time limit, not one per CTA.  Kernels on CTA pairs decide
+// together (pair_flag); the absorbed forward and the decode do not look and run again.
 // ---------------------------------------------------------------------------
 enum DeviceStatus : int {
     STATUS_OK = 0,
@@ -500,6 +501,14 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t rank
     uint32_t result;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(result) : "r"(smem_addr), "r"(rank));
     return result;
+}
+
+// Whether `flag` is set in this CTA's shared memory or at the same place in the other's.  After a cluster barrier that follows the
+// writes, and before one that both CTAs pass at their end.
+__device__ __forceinline__ bool pair_flag(const int* flag, uint32_t rank) {
+    int other;
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(other) : "r"(map_to_cta(smem_u32(flag), rank ^ 1U)) : "memory");
+    return *reinterpret_cast<const volatile int*>(flag) != 0 || other != 0;
 }
 
 // One arrival on a barrier of the other CTA.  Default semantics (release at CTA scope), like every

@@ -53,3 +53,49 @@ def test_wait_runs_out_cleanly_and_the_context_stays_usable(gpu):
     assert float((out.float().cpu() - ref_out).abs().max()) <= 1e-2 * float(ref_out.abs().max())
     assert float((lse.cpu() - ref_lse).abs().max()) <= 1e-3
     assert mla.device_status() == 0
+
+
+def test_pair_kernels_leave_at_once_while_the_status_is_set(gpu):
+    """The kernels on CTA pairs, in a copy of their sources whose status word can be set: a launch that finds a time limit of an earlier one
+    writes nothing (both CTAs of a pair go to the teardown together), and after a reset the same launch gives the product's results."""
+    from dscuda_b200 import mla
+    lib = probe_library()
+    generator = torch.Generator().manual_seed(3)
+
+    def draw(*shape):
+        return (torch.randn(*shape, generator=generator) * .25).bfloat16().to(gpu)
+
+    rows, heads = 3001, 7                   # reaches the pair kernel
+    latent, w_uk, w_uv = draw(rows, 512), draw(heads * 128, 512), draw(heads * 128, 512)
+    projected = [torch.full((rows, heads, 128), 7.0, device=gpu, dtype=torch.bfloat16) for _ in range(2)]
+
+    def project():
+        pointers = [ctypes.c_void_p(t.data_ptr()) for t in (*projected, latent, w_uk, w_uv)]
+        assert lib.dscuda_test_up_project(*pointers, ctypes.c_longlong(rows), heads, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+
+    b, t, h = 1, 130, 5
+    inputs = [draw(b, t, h, 512), draw(b, t, h, 64), draw(b, t, 512), draw(b, t, 64)]
+    dout = draw(b, t, h, 512)
+    out, lse = mla.mla_forward(*inputs, 576 ** -.5)
+    # dquery, dlatent and dkey_rope; the first bytes of dquery_rope hold delta, which a kernel without waits writes
+    grads = [torch.full_like(x, 7.0) for x in inputs]
+
+    def backward():
+        pointers = (ctypes.c_void_p * 11)(*(x.data_ptr() for x in (*grads, dout, out, lse, *inputs)))
+        assert lib.dscuda_test_absorbed_backward(pointers, b, t, h, ctypes.c_float(576 ** -.5), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+
+    for set_status, call, results, product in (
+            (lib.dscuda_test_set_projection_status, project, projected, lambda: mla.up_project(latent, w_uk, w_uv, heads)),
+            (lib.dscuda_test_set_absorbed_backward_status, backward, grads, lambda: mla.mla_backward(dout, out, lse, *inputs, 576 ** -.5))):
+        torch.cuda.synchronize()
+        assert set_status(1) == 0
+        call()
+        torch.cuda.synchronize()
+        untouched = results[0]              # the partial sums and dquery itself share a buffer
+        assert bool((untouched == 7.0).all())
+        assert set_status(0) == 0
+        call()
+        torch.cuda.synchronize()
+        for got, expected in zip(results, product()):
+            assert torch.equal(got, expected)
+    assert mla.device_status() == 0
