@@ -15,7 +15,7 @@
 // half).  With many rows the kernel is bound by HBM: every element is read once
 // and written once.  With few rows a warp takes only a group of a row's heads
 // (GROUPED) and computes the row's angles again: one warp per row left a decode
-// step of 32 rows and 128 heads to 32 warps, 6.9 us against 4.5 us now.
+// step of 32 rows and 128 heads to 32 warps, 6.8 us against 2.4 us now (back to back).
 #include "mla.h"
 #include "cuda_common.h"
 #include "sm100_primitives.cuh"
@@ -123,8 +123,11 @@ void mla_rope_apply_cuda(__nv_bfloat16* q_pe, __nv_bfloat16* k_pe, const int* po
             throw std::invalid_argument("tensor pointers must be 16-byte aligned");
         }
     }
-    constexpr long long WARPS = 148LL * 8 * (ROPE_THREADS / 32);      // 8 CTAs to each of 148 SMs
-    // groups of at least 8 heads (one pass of the kernel's loop) for as long as every item has a warp of its own
+    // Groups of at least 8 heads (one pass of the kernel's loop), for as long as two CTAs to an SM hold all the items: every group
+    // computes the row's angles again, in double precision, which costs more than it gives once the SMs have work.  128 heads,
+    // us with one warp per row / groups for 2 / 4 / 8 CTAs to an SM: 32 rows 6.8 2.4 2.3 2.3, 512 rows 7.0 4.2 4.4 5.8,
+    // 2048 rows 8.6 8.6 8.9 10.4; 16 heads: 100 rows 2.43 2.36 2.36 2.36, 2048 rows 2.95 2.95 3.65 3.66.
+    constexpr long long WARPS = 148LL * 2 * (ROPE_THREADS / 32);
     const int passes = q_pe != nullptr ? (heads + 7) / 8 : 1;
     const int groups = static_cast<int>(std::max(1LL, std::min<long long>(passes, WARPS / rows)));
     const int group_heads = (passes + groups - 1) / groups * 8;

@@ -52,6 +52,20 @@ def test_explicit_positions_and_single_tensors(gpu):
         mla.rope_apply(q_pe.to(gpu))            # packed layout without positions
 
 
+# Few rows: a row's heads are split over warps in groups of whole eights, the last group a part of one (9: 8 + 1), more groups than two
+# (33, 127); 600 rows of 33 heads take fewer, larger groups (16, 16, 1).
+@pytest.mark.parametrize("rows,heads", [(1, 9), (5, 33), (37, 127), (600, 33), (1, 8)])
+def test_head_groups(gpu, rows, heads):
+    from dscuda_b200 import mla
+    positions = torch.randint(0, 32768, (rows,), generator=torch.Generator().manual_seed(rows), dtype=torch.int32)
+    q_pe, k_pe = draw(6, rows, heads, 64), draw(7, rows, 1, 64)
+    q, k = q_pe.to(gpu), k_pe.to(gpu)
+    mla.rope_apply(q, k, positions.to(gpu))
+    torch.cuda.synchronize()
+    check(q.cpu(), reference(q_pe, positions))
+    check(k.cpu(), reference(k_pe, positions))
+
+
 def test_rotated_inputs_feed_the_attention_kernel(gpu):
     """prefill_inputs() rotates on the host; rotating raw draws on the device gives the same attention output."""
     from dscuda_b200 import mla
