@@ -90,6 +90,30 @@ def test_decode_schedule_of_short_sequences(gpu, batch, heads, low, high, splits
     assert bool(torch.isnan(out.cpu()[empty]).all()) and bool((lse.cpu()[empty] == float("-inf")).all())
 
 
+# One sequence over 74 clusters: 74 tiles in ranges of two are 37 partials; 63 tiles fill 63 of 64 slots, 64 tiles two whole groups of 32
+# headers and the end mark in a third, 74 tiles three groups.
+@pytest.mark.parametrize("direction", [1, -1])
+@pytest.mark.parametrize("tiles,splits", [(74, 64), (63, 64), (64, 65), (74, 80)])
+def test_decode_merges_more_partials_than_a_warp_holds(gpu, tiles, splits, direction):
+    """The partials' maxima rise or fall along the sequence, so that the running maximum over groups of 32 slots changes, or not."""
+    from dscuda_b200 import mla
+    tokens, heads = tiles * 128 - 5, 16
+    generator = torch.Generator().manual_seed(tiles + splits)
+    rows = torch.randn(1, tokens, 576, generator=generator)
+    rows[0, :, 0] = direction * torch.linspace(-8, 8, tokens)           # times 30 / sqrt(192): scores move by 35 from end to end
+    query = torch.randn(1, 1, heads, 576, generator=generator)
+    query[..., 0] = 30.0
+    query, rows = query.bfloat16(), rows.bfloat16()
+    cache, table = oracle.pack_cache(rows, 64)
+    lengths = torch.tensor([tokens], dtype=torch.int32)
+    ref_out, ref_lse = oracle.paged_decode(query, cache, table, lengths, 192 ** -.5)
+    out, lse = mla.mla_decode(query.to(gpu), cache.to(gpu), table.to(gpu), lengths.to(gpu), 192 ** -.5, splits=splits)
+    torch.cuda.synchronize()
+    assert mla.device_status() == 0
+    assert max_err_ratio(out.cpu().float(), ref_out) <= 1e-2
+    assert float((lse.cpu() - ref_lse).abs().max()) <= 1e-3
+
+
 def test_decode_rejects_bad_arguments(gpu):
     from dscuda_b200 import mla
     g = load_golden("decode_b2_t23_h3")

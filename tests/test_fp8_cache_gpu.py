@@ -48,6 +48,28 @@ def test_append_and_dequantize_are_bit_exact(gpu, batch, tokens, page):
     assert bool((error <= bound).all())
 
 
+# two rows to a pass: one row alone, odd counts, a start inside a page, more rows than the grid's first pass (18944)
+@pytest.mark.parametrize("first,rows", [(0, 1), (5, 1), (0, 3), (63, 66), (127, 129), (1, 19199)])
+def test_dequantize_part_of_the_cache(gpu, first, rows):
+    """Rows of the range as the format says, every other row as it was."""
+    from dscuda_b200 import mla
+    g = torch.Generator().manual_seed(rows)
+    pages = (first + rows) // 64 + 1
+    kv = torch.randn(1, pages * 64, 576, generator=g).bfloat16()
+    codes, scales, rope = oracle.quantize_fp8_rows(kv)
+    expected = oracle.dequantize_fp8_rows(codes, scales, rope)[0]
+    table = torch.arange(pages, dtype=torch.int32)[None]
+    fp8 = torch.zeros(pages, 64, 656, dtype=torch.uint8, device=gpu)
+    mla.cache_append_fp8(fp8, kv[..., :512].contiguous().to(gpu), kv[..., 512:].contiguous().to(gpu), table.to(gpu))
+    cache = torch.full((pages, 64, 1, 576), 7.0, device=gpu, dtype=torch.bfloat16)
+    assert mla.cache_dequantize_fp8(fp8, cache, first, rows) is cache
+    torch.cuda.synchronize()
+    assert mla.device_status() == 0
+    got = cache.cpu().view(-1, 576)
+    assert torch.equal(got[first:first + rows], expected[first:first + rows])
+    assert bool((got[:first] == 7.0).all()) and bool((got[first + rows:] == 7.0).all())
+
+
 def test_decode_over_the_fp8_cache(gpu):
     from dscuda_b200 import mla
     g = torch.Generator().manual_seed(21)

@@ -82,3 +82,58 @@ def test_decode_append_and_rope_replay(gpu):
         page = int(table[b, int(positions[b]) // 64])
         row = cache[page, int(positions[b]) % 64, 0]
         assert torch.equal(row[:512], new_latent[b, 0]) and torch.equal(row[512:], new_rope[b, 0])
+
+
+def test_replay_with_a_joined_second_stream(gpu):
+    """The query's side of a decode step on one stream, the cache's on another, joined in front of the decode: inside a capture the
+    programmatic edge of a dependent launch then meets an ordinary one."""
+    from dscuda_b200 import mla
+    batch, heads = 3, 16
+    _, cache, table, lengths = (t.to(gpu) for t in oracle.decode_inputs(seed=6, batch=batch, heads=heads, low=100, high=900))
+    generator = torch.Generator(device=gpu).manual_seed(8)
+
+    def draw(*shape, std=1.0):
+        return (torch.randn(*shape, device=gpu, generator=generator) * std).bfloat16()
+
+    q_nope, q_pe, latent, k_pe = draw(batch, 1, heads, 128), draw(batch, 1, heads, 64), draw(batch, 1, 512), draw(batch, 1, 64)
+    w_uk, w_uv = draw(heads * 128, 512, std=0.04), draw(heads * 128, 512, std=0.04)
+    positions = (lengths - 1).contiguous()
+    workspace = mla.decode_workspace(batch, heads, 8, 512, gpu)
+    query = torch.zeros(batch, 1, heads, 576, device=gpu, dtype=torch.bfloat16)
+    out, lse = torch.empty(batch, 1, heads, 512, device=gpu, dtype=torch.bfloat16), torch.empty(batch, heads, 1, device=gpu)
+    result = torch.empty(batch, 1, heads, 128, device=gpu, dtype=torch.bfloat16)
+    side = torch.cuda.Stream()
+
+    def step():
+        main = torch.cuda.current_stream()
+        side.wait_stream(main)
+        with torch.cuda.stream(side):
+            mla.rope_apply(None, k_pe.view(batch, 1, 64), positions)
+            mla.cache_append(cache, latent, k_pe, table, positions)
+        mla.rope_apply(q_pe, None, positions)
+        query[..., :512].copy_(mla.absorb_query(q_nope, w_uk))
+        query[..., 512:].copy_(q_pe)
+        main.wait_stream(side)
+        mla.mla_decode(query, cache, table, lengths, SCALE, 8, workspace, out, lse)
+        result.copy_(mla.unabsorb_output(out, w_uv))
+
+    graph = capture(step)
+    inputs = (q_nope, q_pe, latent, k_pe)
+    fresh = [torch.randn(x.shape, device=gpu, generator=generator).bfloat16() for x in inputs]
+
+    def run(launch):
+        for buffer, value in zip(inputs, fresh):
+            buffer.copy_(value)
+        for buffer in (query, out, lse, result):
+            buffer.zero_()
+        launch()
+        torch.cuda.synchronize()
+        return [x.clone() for x in (query, cache, out, lse, result)]
+
+    replayed, direct = run(graph.replay), run(step)
+    assert mla.device_status() == 0
+    for a, b in zip(replayed, direct):
+        assert torch.equal(a, b)
+    ref_out, ref_lse = oracle.paged_decode(direct[0].cpu(), cache.cpu(), table.cpu(), lengths.cpu(), SCALE)
+    assert float((out.float().cpu() - ref_out).abs().max()) <= 1e-2 * float(ref_out.abs().max())
+    assert float((lse.cpu() - ref_lse).abs().max()) <= 1e-3
