@@ -225,7 +225,6 @@ struct Shared {
     uint64_t rows_done[2];      // eight softmax warps have read them
     uint32_t tmem_base;
     int abort_flag;
-    int latched;                // an earlier launch ran into a time limit
 };
 static_assert(sizeof(Shared) <= SMEM_BYTES - MISC_OFFSET, "key-side barrier block too large");
 }  // namespace ks
@@ -286,7 +285,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ks::KEY_THREADS, 1) 
         tma_prefetch_descriptor(&p.row_do4);
         tma_prefetch_descriptor(&p.row_do2);
         tma_prefetch_descriptor(&p.row_rope);
-        sh->latched = *reinterpret_cast<volatile int*>(&absorbed_backward_status) == STATUS_WAIT_TIMEOUT;
     }
     tc_fence_before_sync();
     __syncthreads();
@@ -296,9 +294,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ks::KEY_THREADS, 1) 
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&sh->tmem_base);
     auto wait = [&](uint64_t& bar, int phase) { return mbar_wait(smem_u32(&bar), phase & 1, abort_flag, &absorbed_backward_status); };
 
-    if (pair_flag(&sh->latched, rank)) {
-        // both CTAs leave through the teardown
-    } else if (warp == LOAD_WARP) {
+    if (warp == LOAD_WARP) {
         // =================== TMA producer ===================================
         if (lane == 0) {
             // the bytes of both CTAs are counted by the leader's barrier
@@ -474,8 +470,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ks::KEY_THREADS, 1) 
         const uint32_t lane_base = tmem_base + (static_cast<uint32_t>((warp % 4) * 32) << 16);
         const int key_pos = key_start + static_cast<int>(rank) * CTA_KEYS + key_in_cta;
         const uint32_t p_full_bar = map_to_cta(smem_u32(&sh->p_full), 0);
-        bool alive = true;
-        for (int t = 0; t < tile_count; ++t) {
+        bool alive = !gave_up_before(&absorbed_backward_status, abort_flag);
+        for (int t = 0; t < tile_count && alive; ++t) {
             alive = __all_sync(0xffffffffU, wait(sh->rows_ready[t & 1], t >> 1) && wait(sh->q_refill_free[1], t));
             if (!alive) {
                 break;
@@ -713,7 +709,6 @@ struct Shared {
     uint64_t ds_full;
     uint32_t tmem_base;
     int abort_flag;
-    int latched;                // an earlier launch ran into a time limit
 };
 static_assert(sizeof(Shared) <= SMEM_BYTES - MISC_OFFSET, "query-side barrier block too large");
 }  // namespace qs
@@ -761,7 +756,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) absorbed
         tma_prefetch_descriptor(&p.stream_k4);
         tma_prefetch_descriptor(&p.stream_k2);
         tma_prefetch_descriptor(&p.stream_rope);
-        sh->latched = *reinterpret_cast<volatile int*>(&absorbed_backward_status) == STATUS_WAIT_TIMEOUT;
     }
     tc_fence_before_sync();
     __syncthreads();
@@ -771,9 +765,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) absorbed
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&sh->tmem_base);
     auto wait = [&](uint64_t& bar, int phase) { return mbar_wait(smem_u32(&bar), phase & 1, abort_flag, &absorbed_backward_status); };
 
-    if (pair_flag(&sh->latched, rank)) {
-        // both CTAs leave through the teardown
-    } else if (warp == LOAD_WARP) {
+    if (warp == LOAD_WARP) {
         // =================== TMA producer ===================================
         if (lane == 0) {
             // the bytes of both CTAs are counted by the leader's barrier
@@ -910,8 +902,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) absorbed
             lse2 = p.lse[(static_cast<size_t>(b) * p.heads + (row - token * p.heads)) * p.sequence + token] * LOG2E;
             delta = stored_delta(p, static_cast<size_t>(b) * rows_per_sequence + row);
         }
-        bool alive = true;
-        for (int j = 0; j < tile_count; ++j) {
+        bool alive = !gave_up_before(&absorbed_backward_status, abort_flag);
+        for (int j = 0; j < tile_count && alive; ++j) {
             alive = __all_sync(0xffffffffU, wait(sh->s_full, j));
             if (!alive) {
                 break;

@@ -320,7 +320,6 @@ struct PairShared {
     uint64_t acc_empty[2];                  // leader: one arrival per epilogue warp of either CTA
     uint32_t tmem_base;
     int abort_flag;
-    int latched;                            // an earlier launch ran into a time limit
 };
 static_assert(sizeof(PairShared) <= MISC_BYTES, "barrier block too large");
 }  // namespace pk
@@ -367,7 +366,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) projecti
         tma_prefetch_descriptor(&p.a);
         tma_prefetch_descriptor(&p.b[0]);
         tma_prefetch_descriptor(&p.c[0]);
-        sh->latched = *reinterpret_cast<volatile int*>(&projection_status) == STATUS_WAIT_TIMEOUT;
     }
     tc_fence_before_sync();
     __syncthreads();
@@ -385,9 +383,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) projecti
     // a column of tiles (batch entry, n) shares its B tile
     auto column_of = [&](long long tile) { return static_cast<int>(tile / tiles_m); };
 
-    if (pair_flag(&sh->latched, rank)) {
-        // both CTAs leave through the teardown
-    } else if (warp == LOAD_WARP) {
+    if (warp == LOAD_WARP) {
         if (lane == 0) {
             bool alive = true;
             long long chunk = 0;
@@ -516,7 +512,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) projecti
     } else {
         // =================== epilogue: warp = 32 rows of this CTA's half of the tile, thread = row ==================
         const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
-        bool alive = true;
+        bool alive = !gave_up_before(&projection_status, abort_flag);
         int local_tile = 0;
         for (long long tile = tile_begin; tile < tile_end && alive; ++tile, ++local_tile) {
             const int column = column_of(tile);

@@ -16,8 +16,10 @@ namespace sm100 {
 // ---------------------------------------------------------------------------
 // Device status word.  A wait that runs out sets it; the kernels with such waits in
 // the same translation unit check it on entry and leave at once when it is set, so a
-// broken pipeline costs one time limit, not one per CTA.  Kernels on CTA pairs decide
-// together (pair_flag); the absorbed forward and the decode do not look and run again.
+// broken pipeline costs one time limit, not one per CTA.  In kernels on CTA pairs the
+// softmax or epilogue warps of each CTA look while they have nothing to do yet, and tell
+// their CTA to give up (gave_up_before); nothing is written then.  The absorbed forward
+// and the decode do not look and run again.
 // ---------------------------------------------------------------------------
 enum DeviceStatus : int {
     STATUS_OK = 0,
@@ -123,6 +125,16 @@ __device__ __forceinline__ bool mbar_wait_limit(uint32_t bar, uint32_t parity, v
 
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status_word) {
     return mbar_wait_limit(bar, parity, abort_flag, status_word, WAIT_LIMIT_CYCLES);
+}
+
+// Whether an earlier launch ran into a time limit; if so, this CTA is told to give up as well.  By whole warps, in front of their
+// first wait.
+__device__ __forceinline__ bool gave_up_before(const int* status_word, volatile int* abort_flag) {
+    if (*reinterpret_cast<const volatile int*>(status_word) != STATUS_WAIT_TIMEOUT) {
+        return false;
+    }
+    *abort_flag = 1;
+    return true;
 }
 
 // Register re-distribution between warpgroups (all four warps of a warpgroup
@@ -501,14 +513,6 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t rank
     uint32_t result;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(result) : "r"(smem_addr), "r"(rank));
     return result;
-}
-
-// Whether `flag` is set in this CTA's shared memory or at the same place in the other's.  After a cluster barrier that follows the
-// writes, and before one that both CTAs pass at their end.
-__device__ __forceinline__ bool pair_flag(const int* flag, uint32_t rank) {
-    int other;
-    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(other) : "r"(map_to_cta(smem_u32(flag), rank ^ 1U)) : "memory");
-    return *reinterpret_cast<const volatile int*>(flag) != 0 || other != 0;
 }
 
 // One arrival on a barrier of the other CTA.  Default semantics (release at CTA scope), like every

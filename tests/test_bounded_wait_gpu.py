@@ -57,7 +57,7 @@ def test_wait_runs_out_cleanly_and_the_context_stays_usable(gpu):
 
 def test_pair_kernels_leave_at_once_while_the_status_is_set(gpu):
     """The kernels on CTA pairs, in a copy of their sources whose status word can be set: a launch that finds a time limit of an earlier one
-    writes nothing (both CTAs of a pair go to the teardown together), and after a reset the same launch gives the product's results."""
+    writes nothing, and after a reset the same launch gives the product's results."""
     from dscuda_b200 import mla
     lib = probe_library()
     generator = torch.Generator().manual_seed(3)
