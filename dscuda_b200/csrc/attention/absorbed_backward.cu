@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(256) absorbed_delta_kernel(__nv_bfloat16* dq_r
 // The eight 64-column chunks of a CTA's own 48 rows sit in slots 0..7.  Chunks {2r, 2r+1, 4+2r, 4+2r+1} are in place as
 // columns of the gradient products; the other four slots are refilled with the other CTA's rows of those columns as soon as
 // the score MMAs have read them (the same scheme as in absorbed_attention.cu), and the rotary columns of all 96 rows are
-// loaded once more into a place of their own.  So the scores are computed once per (key, row) pair and a CTA reads 168 KB
+// loaded once more into a place of their own.  So the scores are computed once per (key, row) pair and a CTA reads 162 KB
 // from L2 for 64 x 96 pairs.
 //
 // What bounds it: shared memory.  The resident keys (72 KB), P and dS (32 KB) and one tile of rows (114 KB) fill it, so the
@@ -666,7 +666,7 @@ __global__ void __launch_bounds__(144) absorbed_backward_reduce_kernel(const __g
 //
 // What bounds it: the chain of a tile, as on the key side.  64 rows of one CTA with 128-key tiles, which this replaces, ran
 // at the N = 64 rate and streamed every key tile twice (288 KB for 64 x 128 pairs, L2 latency over two 32 KB slots; here
-// 84 KB for 64 x 96): 680 us at B=4 T=2048 H=16 against
+// 90 KB for 64 x 96): 680 us at B=4 T=2048 H=16 against
 // 483 us now.
 //
 // Tensor memory and warps as on the key side; a softmax thread owns 24 keys of one row, so LSE, delta and token are its own.

@@ -35,10 +35,6 @@ __device__ __forceinline__ uint32_t smem_u32(const void* pointer) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(pointer));
 }
 
-__device__ __forceinline__ uint32_t lane_id() {
-    return threadIdx.x & 31U;
-}
-
 // ---------------------------------------------------------------------------
 // Dependent launches (../common/launch.h).  The wait comes before the first access to memory that another kernel writes; at
 // least one block of every grid has to reach it, or the grid could end before the one in front of it.
@@ -243,12 +239,6 @@ __device__ __forceinline__ uint64_t l2_evict_first_policy() {
     uint64_t policy;
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
     return policy;
-}
-
-__device__ __forceinline__ void tma_store_2d_hint(const void* tensor_map, uint32_t smem_src, int x, int y, uint64_t policy) {
-    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group.L2::cache_hint [%0, {%2, %3}], [%1], %4;" ::"l"(tensor_map), "r"(smem_src), "r"(x),
-                 "r"(y), "l"(policy)
-                 : "memory");
 }
 
 __device__ __forceinline__ void tma_store_commit() {
@@ -461,38 +451,6 @@ __host__ __device__ constexpr uint32_t smem_desc_hi(uint32_t stride_bytes) {
 
 __device__ __forceinline__ uint32_t smem_desc_lo(uint32_t smem_addr, uint32_t leading_bytes) {
     return ((smem_addr & 0x3FFFFU) >> 4) | (((leading_bytes >> 4) & 0x3FFFU) << 16);
-}
-
-// Elected-lane forms of the split-descriptor MMAs (see elect_one()).
-__device__ __forceinline__ void mma_ss_split_elect(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi,
-                                                   uint32_t idesc, uint32_t accumulate, uint32_t leader) {
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p, q;\n\t"
-        ".reg .b64 da, db;\n\t"
-        "setp.ne.b32 p, %6, 0;\n\t"
-        "setp.ne.b32 q, %7, 0;\n\t"
-        "mov.b64 da, {%1, %2};\n\t"
-        "mov.b64 db, {%3, %4};\n\t"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t"
-        "}\n"
-        ::"r"(d_tmem), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(leader)
-        : "memory");
-}
-
-__device__ __forceinline__ void mma_ts_split_elect(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t b_hi, uint32_t idesc,
-                                                   uint32_t accumulate, uint32_t leader) {
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p, q;\n\t"
-        ".reg .b64 db;\n\t"
-        "setp.ne.b32 p, %5, 0;\n\t"
-        "setp.ne.b32 q, %6, 0;\n\t"
-        "mov.b64 db, {%2, %3};\n\t"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t"
-        "}\n"
-        ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(leader)
-        : "memory");
 }
 
 // ---------------------------------------------------------------------------

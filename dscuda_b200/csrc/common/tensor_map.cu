@@ -156,18 +156,15 @@ CUtensorMap make_bf16_batched_rows_map(void* base, std::uint64_t batch, std::uin
     return map;
 }
 
-CUtensorMap make_bf16_store_map(void* base, std::uint64_t rows, std::uint64_t cols, std::uint32_t box_cols, std::uint32_t box_rows) {
-    if (box_cols != 32 && box_cols != 64) {
-        throw std::invalid_argument("store tiles are 32 or 64 columns wide");
-    }
+CUtensorMap make_bf16_store_map(void* base, std::uint64_t rows, std::uint64_t cols, std::uint32_t box_rows) {
     CUtensorMap map;
     const cuuint64_t dims[2] = {cols, rows};
     const cuuint64_t strides[1] = {cols * 2};
-    const cuuint32_t box[2] = {box_cols, box_rows};
+    const cuuint32_t box[2] = {64, box_rows};
     const cuuint32_t element_strides[2] = {1, 1};
     const CUresult result = encode_entry_point()(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides, box, element_strides,
-                                                 CU_TENSOR_MAP_INTERLEAVE_NONE, box_cols == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
-                                                 CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                                                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                                                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (result != CUDA_SUCCESS) {
         throw std::runtime_error("cuTensorMapEncodeTiled (store) failed with code " + std::to_string(static_cast<int>(result)));
     }

@@ -36,12 +36,12 @@ CUtensorMap make_bf16_batched_chunked_map(const void* base, std::uint64_t batch,
 // a box {box_words, box_rows} at {word, row} lands in shared memory row after row, box_words * 8 bytes each.
 CUtensorMap make_u64_rows_map(const void* base, std::uint64_t rows, std::uint32_t row_words, std::uint32_t box_words, std::uint32_t box_rows);
 
-// Store views; 128-byte swizzle in shared memory unless stated.  Rows of `cols` bf16, `rows` to a batch entry, everything contiguous; box
+// Store views; 128-byte swizzle in shared memory.  Rows of `cols` bf16, `rows` to a batch entry, everything contiguous; box
 // {64, box_rows, 1} at {column, row, entry}: rows past the entry's last one are clipped, not written into the next entry.
 CUtensorMap make_bf16_batched_rows_map(void* base, std::uint64_t batch, std::uint64_t rows, std::uint32_t cols, std::uint32_t box_rows);
 
-// Rows of `cols` bf16, contiguous; box {box_cols, box_rows}, box_cols 32 (64-byte swizzle) or 64 (128-byte swizzle).
-CUtensorMap make_bf16_store_map(void* base, std::uint64_t rows, std::uint64_t cols, std::uint32_t box_cols, std::uint32_t box_rows);
+// Rows of `cols` bf16, contiguous; box {64, box_rows}.
+CUtensorMap make_bf16_store_map(void* base, std::uint64_t rows, std::uint64_t cols, std::uint32_t box_rows);
 
 // fp32 records [batch][rows][slots][cols], contiguous; box {32, 1, box_rows, 1} at {column, slot, row, entry}.
 CUtensorMap make_f32_records_map(void* base, std::uint64_t batch, std::uint64_t rows, std::uint64_t slots, std::uint32_t cols, std::uint32_t box_rows);
