@@ -89,7 +89,7 @@ def main(argv=None) -> int:
     parser.add_argument("family", choices=("mla",))
     parser.add_argument("suite", nargs="?", default="quick", choices=("quick", "full"))
     parser.add_argument("mode", nargs="?", default="profile", choices=("profile", "extract", "print"))
-    parser.add_argument("--out-dir", type=pathlib.Path, default=ROOT / "gpurun_out", help="raw ncu output (reports, CSV, logs)")
+    parser.add_argument("--out-dir", type=pathlib.Path, default=BUILD / "profile", help="raw ncu output (reports, CSV, logs)")
     parser.add_argument("--profiles-dir", type=pathlib.Path, default=ROOT / "profiles", help="markdown summaries and traffic.json")
     parser.add_argument("--only", help="comma-separated case names")
     args = parser.parse_args(argv)

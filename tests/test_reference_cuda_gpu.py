@@ -98,8 +98,8 @@ def test_decode_equals_the_reference_kernels(gpu, reference, b, t, h):
 
 def test_speed_beside_the_reference_kernels(gpu, reference):
     """Both libraries timed with CUDA events on the reference's benchmark shapes (`benchmarks/mla.py:34-45`: its largest
-    prefill shape, decode shapes of its `h100` suite).  The figures go to gpurun_out/reference_cuda_timing.json where
-    that directory exists; the assertion only says that nothing here is slower than the code it replaces."""
+    prefill shape, decode shapes of its `h100` suite).  The figures go to build/reference_cuda_timing.json;
+    the assertion only says that nothing here is slower than the code it replaces."""
     import json
     from dscuda_b200 import mla
     g = torch.Generator(device=gpu).manual_seed(11)
@@ -162,9 +162,7 @@ def test_speed_beside_the_reference_kernels(gpu, reference):
     report = {name: {"this_us": mine, "reference_us": theirs, "speedup": theirs / mine} for name, (mine, theirs) in rows.items()}
     for name, row in report.items():
         print(f"{name}: this {row['this_us']:.1f} us, reference kernels {row['reference_us']:.1f} us, x{row['speedup']:.1f}")
-    log = ROOT / "gpurun_out"
-    if log.is_dir():
-        (log / "reference_cuda_timing.json").write_text(json.dumps(report, indent=1))
+    (ROOT / "build" / "reference_cuda_timing.json").write_text(json.dumps(report, indent=1))
     assert all(row["speedup"] >= 1.0 for row in report.values()), report
 
 

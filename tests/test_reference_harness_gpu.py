@@ -48,8 +48,6 @@ def test_reference_harness_passes_against_these_libraries(gpu, tmp_path, family,
     for name in ("mla", "flash_attention"):
         shutil.copyfile(ROOT / "build" / f"libdscuda_{name}_bench.so", tmp_path / "build" / f"libdscuda_{name}_bench.so")
     done = subprocess.run([sys.executable, "benchmarks/run.py", family, "--test"], cwd=tmp_path, capture_output=True, text=True, timeout=600)
-    log = ROOT / "gpurun_out"
-    if log.is_dir():
-        (log / f"reference_harness_{family}.log").write_text(done.stdout + done.stderr)
+    (ROOT / "build" / f"reference_harness_{family}.log").write_text(done.stdout + done.stderr)
     assert done.returncode == 0, done.stdout[-2000:] + done.stderr[-4000:]
     assert f"{family}: {checks} correctness checks passed" in done.stdout
