@@ -203,7 +203,25 @@ __global__ void __launch_bounds__(FORWARD_THREADS, 1) attention_forward_kernel(c
     static_assert(8 * (REG_HI - 168) <= 4 * (168 - REG_LO), "register redistribution exceeds the CTA's allocation");
     if (warp >= 8) {
         reg_dealloc<REG_LO>();      // one instruction for the whole warpgroup
-        if (warp == LOAD_WARP) {
+        if (warp >= TAIL_WARP) {
+            // =================== values behind the end of a packed sequence =====
+            // The softmax masks the scores of such keys, but P V multiplies their values by P = 0.
+            if (tail_keys < TILE_N) {
+                const int half = warp - TAIL_WARP;
+                if (__all_sync(0xffffffffU, mbar_wait(smem_u32(&bars->tail_full[half]), 0, abort_flag, &forward_status))) {
+                    const int slot = ((tile_count - 1) * L::PER_TILE + KQ + half) % L::RING;
+                    uint8_t* chunk = smem_raw + (ring_smem - smem_u32(smem_raw)) + slot * CHUNK_BYTES;
+                    const int first = min(max(tail_keys - half * 64, 0), 64);
+                    clear_rows(chunk, first, 64, lane);
+                    clear_rows(chunk + CHUNK_BYTES / 2, first, 64, lane);
+                    fence_proxy_async_smem();
+                    __syncwarp();
+                    if (lane == 0) {
+                        mbar_arrive(smem_u32(&bars->ring_full[slot]));
+                    }
+                }
+            }
+        } else if (warp == LOAD_WARP) {
             // =================== TMA producer ===================================
             if (lane == 0) {
                 auto load_q = [&](int i) {
@@ -236,7 +254,8 @@ __global__ void __launch_bounds__(FORWARD_THREADS, 1) attention_forward_kernel(c
                     return ring_smem + slot * CHUNK_BYTES;
                 };
                 // The shape of this thread's code, by measurement: 128 columns 4 x 2048 x 64 / 8 heads 343 us as a plain loop, 352 with the
-                // last tile apart and the loops unrolled; 192 columns 1 x 256 x 16 heads 9.7 us that way, 10.1 as a plain loop.
+                // last tile apart and the loops unrolled; 192 columns 1 x 256 x 16 heads 9.7 us that way, 10.1 as a plain loop.  (With the
+                // branch of the clearing warps behind the other two, 192 columns 4 x 4096 x 128 heads took 2 % longer.)
                 constexpr int LOAD_UNROLL = KQ == 2 ? 1 : KQ;
                 auto load_tile = [&](int j, bool tail) {
                     const int y = entry_row0 + j * TILE_N;
@@ -380,22 +399,6 @@ __global__ void __launch_bounds__(FORWARD_THREADS, 1) attention_forward_kernel(c
                             mma_commit_elect(smem_u32(&bars->s_full[i]), leader);   // O_i is final
                         }
                     }
-                }
-            }
-        } else if (tail_keys < TILE_N) {
-            // =================== values behind the end of a packed sequence =====
-            // The softmax masks the scores of such keys, but P V multiplies their values by P = 0.
-            const int half = warp - TAIL_WARP;
-            if (__all_sync(0xffffffffU, mbar_wait(smem_u32(&bars->tail_full[half]), 0, abort_flag, &forward_status))) {
-                const int slot = ((tile_count - 1) * L::PER_TILE + KQ + half) % L::RING;
-                uint8_t* chunk = smem_raw + (ring_smem - smem_u32(smem_raw)) + slot * CHUNK_BYTES;
-                const int first = min(max(tail_keys - half * 64, 0), 64);
-                clear_rows(chunk, first, 64, lane);
-                clear_rows(chunk + CHUNK_BYTES / 2, first, 64, lane);
-                fence_proxy_async_smem();
-                __syncwarp();
-                if (lane == 0) {
-                    mbar_arrive(smem_u32(&bars->ring_full[slot]));
                 }
             }
         }
