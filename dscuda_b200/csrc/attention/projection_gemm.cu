@@ -8,7 +8,7 @@
 //     and W_UV applied to the latent output,
 //       out [rows, h, 128] = o_latent [rows, h, 512] W_UV[h]^T.
 //
-// All four are one operation: a batched bf16 GEMM  C_b [M, N] = A_b [M, K] op(B_b)  with fp32 accumulation
+// All four are one kernel: a batched bf16 GEMM  C_b [M, N] = A_b [M, K] op(B_b)  with fp32 accumulation
 // in tensor memory, where a batch entry (a head) is a column offset into A and C and a row offset into
 // B, and op(B) is either B^T (B stored [N, K], K-major) or B itself (B stored [K, N], N contiguous: the
 // MN-major operand form, no transpose pass).  The reference has none of these (its inputs are drawn
@@ -20,7 +20,7 @@
 //   cta_group::2 MMAs.  K is at most 512, so the weights of a column tile (the B operand) stay in shared memory
 //   for as long as the cluster walks down the rows, half of them in each CTA, and only A streams: 32 bytes per
 //   clock and SM where single-CTA 128 x 128 tiles asked L2 for 128, three times what it gives.
-//   projection_gemm_kernel (a decode step, short prompts, W_UV at any size, W_UK into very many queries): persistent CTAs with one 128 x 128
+//   projection_gemm_kernel (a decode step, short prompts, and W_UV at any size): persistent CTAs with one 128 x 128
 //   tile at a time; less to set up, and at a few rows per head the weights, read once, are what bounds it.
 //
 // In both the accumulator is double-buffered in tensor memory, so the MMA warp starts the next tile while the epilogue
@@ -618,16 +618,7 @@ void configure_kernel() {
 
 // Up to this many (128 x 128 tile, 64-column chunk of K) steps the single-CTA kernel runs: it takes about 5 us + 0.39 us for
 // each step of an SM (32 KB from L2), the pair kernel about 8 us + 0.25 us for the same work, so they meet at 20 steps per SM.
-// That is for K = 512.  At K = 128 (W_UK into the query) they meet earlier, near 8 steps per SM: 16 heads of 1024 rows 8.4 and 8.6 us,
-// of 1536 rows 11.0 and 10.1, of 2048 rows 12.4 and 11.6 (single-CTA, pair).
 constexpr long long SMALL_STEPS = 20 * 148;
-
-// At K = 128 both kernels are bound by writing C.  The pair kernel's clusters work on a column of tiles each and write pieces of 512
-// bytes, far apart when there are more columns than clusters; once C is too large for L2 that is the slower order (by measurement:
-// pair / single-CTA time, 36 and 40 heads 0.80-0.92 at 1024-16384 rows; 56 heads 0.94, 0.98, 1.02, 1.02 at 3072, 4096, 6000, 8192 rows;
-// 64 heads 0.95, 1.01, 1.03, 1.03 at 2500, 3072, 4096, 8192; 128 heads 0.96, 0.99, 1.05, 1.04, 1.02 at 1536, 2048, 3072, 4096, 8192).
-constexpr long long PAIR_OUTPUT_LIMIT = 240LL * 1000 * 1000;
-
 
 // C_b [m, n] = A_b [m, k] op(B_b) for b in [0, batch): see GemmParams for the batch offsets.  With `b2` the entries of a
 // batch of two are two weights and two outputs of the same A.
@@ -655,9 +646,7 @@ void launch_gemm(__nv_bfloat16* c, const __nv_bfloat16* a, const __nv_bfloat16* 
     const long long small_tiles = ((m + TILE_M - 1) / TILE_M) * (n / TILE_N) * batch;
     // a head's own 128 columns (W_UV) make no 256-wide tile; there the kernel is bound by reading the latent rows anyway
     const bool wide = n % pk::N_TILE == 0 || batch == 1 || b2 != nullptr;
-    const long long column_tiles = static_cast<long long>((n + pk::N_TILE - 1) / pk::N_TILE) * batch;
-    const bool scattered = k <= 2 * TILE_K && 2 * column_tiles > 3 * (sm_count() / 2) && 2 * m * n * batch > PAIR_OUTPUT_LIMIT;
-    const bool small = !wide || scattered || small_tiles * (k / TILE_K) <= SMALL_STEPS;
+    const bool small = !wide || small_tiles * (k / TILE_K) <= SMALL_STEPS;
     GemmParams params{};
     const std::uint64_t rows = static_cast<std::uint64_t>(m);
     auto columns = [](long long value) { return static_cast<std::uint64_t>(value); };

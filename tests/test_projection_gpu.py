@@ -79,20 +79,3 @@ def test_pair_kernel_tile_edges(gpu, rows, heads):
     ref_q = torch.einsum("rhk,hkn->rhn", q_nope.float(), w_uk.float().reshape(heads, 128, 512))
     for got, ref in ((k_nope, ref_k), (v, ref_v), (q_latent, ref_q)):
         assert max_err_ratio(got.float().cpu(), ref) <= 2 ** -7
-
-
-def test_absorbed_query_on_both_sides_of_the_output_limit(gpu):
-    """57 heads, rows around 240 MB of output: the two kernels that meet there add the 128 products of an element in the same order of
-    chunks, so the rows they share are the same bits; a sample of rows against an fp32 matmul."""
-    from dscuda_b200 import mla
-    heads, rows = 57, 4200                          # 245 MB; 3000 rows are 175 MB
-    generator = torch.Generator(device=gpu).manual_seed(57)
-    q_nope = torch.randn(rows, heads, 128, device=gpu, generator=generator).bfloat16()
-    w_uk = (torch.randn(heads * 128, 512, device=gpu, generator=generator) * .05).bfloat16()
-    many = mla.absorb_query(q_nope, w_uk)
-    fewer = mla.absorb_query(q_nope[:3000].contiguous(), w_uk)
-    assert torch.equal(many[:3000], fewer)
-    sample = torch.tensor([0, 127, 128, 2999, 4095, 4096, 4199], device=gpu)
-    ref = torch.einsum("rhk,hkn->rhn", q_nope[sample].cpu().float(), w_uk.cpu().float().reshape(heads, 128, 512))
-    assert max_err_ratio(many[sample].float().cpu(), ref) <= 2 ** -7
-    assert mla.device_status() == 0
