@@ -8,7 +8,7 @@
 //     and W_UV applied to the latent output,
 //       out [rows, h, 128] = o_latent [rows, h, 512] W_UV[h]^T.
 //
-// All four are one kernel: a batched bf16 GEMM  C_b [M, N] = A_b [M, K] op(B_b)  with fp32 accumulation
+// All four are one operation: a batched bf16 GEMM  C_b [M, N] = A_b [M, K] op(B_b)  with fp32 accumulation
 // in tensor memory, where a batch entry (a head) is a column offset into A and C and a row offset into
 // B, and op(B) is either B^T (B stored [N, K], K-major) or B itself (B stored [K, N], N contiguous: the
 // MN-major operand form, no transpose pass).  The reference has none of these (its inputs are drawn
@@ -618,6 +618,10 @@ void configure_kernel() {
 
 // Up to this many (128 x 128 tile, 64-column chunk of K) steps the single-CTA kernel runs: it takes about 5 us + 0.39 us for
 // each step of an SM (32 KB from L2), the pair kernel about 8 us + 0.25 us for the same work, so they meet at 20 steps per SM.
+// That is for K = 512.  At K = 128 (W_UK into the query), where writing C is the bound, they meet earlier, near 8 steps per SM:
+// 16 heads of 1024 rows 8.4 and 8.6 us, of 1536 rows 11.0 and 10.1, of 2048 rows 12.4 and 11.6 (single-CTA, pair).  Beyond L2 the
+// place of C in memory decides between them: 128 heads of 4096 rows 152 and 158 us with nothing else allocated, 172 and 163 in a
+// program that holds 2 GB more; 64 heads of 16384 rows 299 and 305, 350 and 316.
 constexpr long long SMALL_STEPS = 20 * 148;
 
 // C_b [m, n] = A_b [m, k] op(B_b) for b in [0, batch): see GemmParams for the batch offsets.  With `b2` the entries of a
